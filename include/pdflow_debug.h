@@ -113,6 +113,14 @@ int pdflow_set_quad_prefetch(unsigned ctas_ahead);
  * use it in and returns how many differ (0 expected). */
 int pdflow_check_div_rcp(unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches);
 
+/* Check of the disc projection's factor (no counterpart in the reference):
+ * the iteration kernels take min(1, 1 / hypot(a, b)) from the reciprocal root
+ * of the sum of squares instead of calling rhypotf; this compares the two bit
+ * for bit on `pairs` random pairs (around the unit circle, inside and outside
+ * it, over wide exponents, with zero, infinite and NaN operands among them)
+ * and returns how many differ (0 expected). */
+int pdflow_check_disc_factor(unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches);
+
 /* The strip walk's work units (iteration form 10; no counterpart in the
  * reference), as the launcher computes them for `bands` 24-row bands of
  * `cols` columns on `ctas` CTAs at `iters_per_launch` iterations per launch:

@@ -276,6 +276,39 @@ __global__ void k_div_rcp_check(unsigned long long n, unsigned long long seed, u
     if (mine) atomicAdd(bad, mine);
 }
 
+// disc_factor against rhypotf clamped at 1: a third of the pairs near the unit
+// circle, a third in [0, 2)^2, a third over exponents -30 .. 40, and one pair
+// in 64 with a zero, subnormal, huge, infinite or NaN operand.
+__global__ void k_disc_check(unsigned long long n, unsigned long long seed, unsigned long long* bad)
+{
+    const unsigned special[8] = {0u, 0x80000000u, 1u, 0x7f7fffffu, 0x71800000u, 0x7f800000u, 0xff800000u, 0x7fc00000u};
+    unsigned long long mine = 0;
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        const unsigned r1 = mix64(seed + 2 * i), r2 = mix64(seed + 2 * i + 1);
+        float a, b;
+        if (i % 3 == 0) {
+            float c, d;
+            sincosf(float(r1 & 0xffffffu) * 0x1p-24f * 6.2831853f, &d, &c);
+            const float r = 1.f + (float(r2 & 0xffffu) - 32768.f) * 0x1p-24f;
+            a = r * c;
+            b = r * d;
+        } else if (i % 3 == 1) {
+            a = float(r1 & 0xffffffu) * 0x1p-23f;
+            b = -float(r2 & 0xffffffu) * 0x1p-23f;
+        } else {
+            a = rand_mag(r1, -30, 40);
+            b = rand_mag(r2, -30, 40);
+        }
+        if ((mix64(r1 ^ r2) & 63u) == 0) {
+            a = __uint_as_float(special[r1 & 7u]);
+            if (r2 & 64u) b = __uint_as_float(special[r2 & 7u]);
+        }
+        if (__float_as_uint(disc_factor(a, b)) != __float_as_uint(fminf(rhypotf(a, b), 1.f))) ++mine;
+    }
+    if (mine) atomicAdd(bad, mine);
+}
+
 // `passes` copies a -> b, b -> a, a -> b ... in one launch; each thread moves
 // the same elements every pass (no cross-thread hazard), with L2-level loads
 // and stores (ld/st.global.cg) that the compiler cannot fold across passes.
@@ -300,7 +333,8 @@ __global__ void __launch_bounds__(512) k_copy4(float4* a, float4* b, size_t n, u
 
 extern "C" {
 
-int pdflow_check_div_rcp(unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches)
+static int count_mismatches(void (*check)(unsigned long long, unsigned long long, unsigned long long*),
+                            unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches)
 {
     if (!mismatches) return fail(PDFLOW_ERR_ARG, "null output");
     unsigned long long* d = nullptr;
@@ -310,12 +344,22 @@ int pdflow_check_div_rcp(unsigned long long pairs, unsigned long long seed, unsi
     }
     cudaError_t e = cudaMemset(d, 0, sizeof *d);
     if (e == cudaSuccess) {
-        k_div_rcp_check<<<1024, 256>>>(pairs, seed, d);
+        check<<<1024, 256>>>(pairs, seed, d);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(mismatches, d, sizeof *d, cudaMemcpyDeviceToHost);
     cudaFree(d);
-    return e == cudaSuccess ? PDFLOW_OK : fail("division check", e);
+    return e == cudaSuccess ? PDFLOW_OK : fail("arithmetic check", e);
+}
+
+int pdflow_check_div_rcp(unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches)
+{
+    return count_mismatches(k_div_rcp_check, pairs, seed, mismatches);
+}
+
+int pdflow_check_disc_factor(unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches)
+{
+    return count_mismatches(k_disc_check, pairs, seed, mismatches);
 }
 
 int pdflow_strip_units(unsigned bands, unsigned cols, unsigned iters_per_launch, unsigned ctas, unsigned* whole,

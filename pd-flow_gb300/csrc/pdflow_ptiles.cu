@@ -104,27 +104,44 @@ constexpr uint32_t kStreamWaitLimit = 1u << 22;
 
 __device__ __forceinline__ float clamp1(float pd) { return (fabsf(pd) > 1.f) ? ((pd > 1.f) ? 1.f : -1.f) : pd; }
 
-// Projection onto the unit disc (updateDualVariables, pdflow_cudalib.cu:813-887).
-// Branch-free: outside the projection the factor is 1 and x * 1 == x exactly,
-// so the bits are those of the reference's conditional update.
-__device__ __forceinline__ void disc(float& a, float& b)
+// The three TV duals' projections onto the unit disc (updateDualVariables,
+// pdflow_cudalib.cu:813-887) for both pixels of a pair, with disc_factor's
+// expressions in packed FP32x2.  Evaluated for every lane without a test of
+// which lanes are outside: at a handful of instructions a projection, a vote
+// to skip it costs as much (one vote guards all six sums' range instead; a
+// warp with one beyond it takes the scalar form).
+struct Disc2 {
+    float2 s;
+    __device__ __forceinline__ Disc2(float2 a, float2 b)
+    {
+        const float2 hi = make_float2(max_nan(fabsf(a.x), fabsf(b.x)), max_nan(fabsf(a.y), fabsf(b.y)));
+        const float2 lo = make_float2(fminf(fabsf(a.x), fabsf(b.x)), fminf(fabsf(a.y), fabsf(b.y)));
+        s = fm2(hi, hi, mul2(lo, lo));
+    }
+    __device__ __forceinline__ float peak() const { return max_nan(s.x, s.y); }
+    __device__ __forceinline__ void apply(float2& a, float2& b) const
+    {
+        const float2 f = make_float2(rsqrt_min1(s.x), rsqrt_min1(s.y));
+        a = mul2(a, f);
+        b = mul2(b, f);
+    }
+};
+__device__ __forceinline__ void project_duals(float2& puu, float2& puv, float2& pvu, float2& pvv, float2& pwu,
+                                              float2& pwv)
 {
-    const float m = rhypotf(a, b);
-    const float f = (m < 1.f) ? m : 1.f;
-    a = mul(a, f);
-    b = mul(b, f);
-}
-
-// Both pixels of a pair.  Inside the disc of radius sqrt(0.999) rhypotf
-// (maximum error 2 ulp) returns more than 1, the factor is 1 and the values
-// stay as they are: a warp whose 64 pixels are all there skips the
-// reciprocal norms (NaN and infinite inputs fail the test and take them).
-__device__ __forceinline__ void disc2(float2& a, float2& b)
-{
-    const float2 s = fm2(a, a, mul2(b, b));
-    if (__all_sync(0xffffffffu, s.x < 0.999f && s.y < 0.999f)) return;
-    disc(a.x, b.x);
-    disc(a.y, b.y);
+    const Disc2 u(puu, puv), v(pvu, pvv), w(pwu, pwv);
+    if (__all_sync(0xffffffffu, max_nan(max_nan(u.peak(), v.peak()), w.peak()) < kDiscLimit)) {
+        u.apply(puu, puv);
+        v.apply(pvu, pvv);
+        w.apply(pwu, pwv);
+    } else {
+        project_disc(puu.x, puv.x);
+        project_disc(puu.y, puv.y);
+        project_disc(pvu.x, pvv.x);
+        project_disc(pvu.y, pvv.y);
+        project_disc(pwu.x, pwv.x);
+        project_disc(pwu.y, pwv.y);
+    }
 }
 
 // shrink_rcp (pdflow_math.cuh) for both pixels of a pair: the quotients'
@@ -415,9 +432,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
                     pwv = fm2(s4, gw2, pwv);
                     pd.x = clamp1(pd.x);
                     pd.y = clamp1(pd.y);
-                    disc2(puu, puv);
-                    disc2(pvu, pvv);
-                    disc2(pwu, pwv);
+                    project_duals(puu, puv, pvu, pvv, pwu, pwv);
                 }
                 // ---------------- primal step (computeDivergence + updatePrimalVariables) ----------------
                 {

@@ -161,17 +161,6 @@ __device__ __forceinline__ Q shift_up(const Q& a, float below)
 
 __device__ __forceinline__ float clamp1(float pd) { return (fabsf(pd) > 1.f) ? ((pd > 1.f) ? 1.f : -1.f) : pd; }
 
-// Projection onto the unit disc (updateDualVariables, pdflow_cudalib.cu:813-887).
-// Branch-free: outside the projection the factor is 1 and x * 1 == x exactly,
-// so the bits are those of the reference's conditional update.
-__device__ __forceinline__ void disc(float& a, float& b)
-{
-    const float m = rhypotf(a, b);
-    const float f = (m < 1.f) ? m : 1.f;
-    a = mul(a, f);
-    b = mul(b, f);
-}
-
 __global__ void __launch_bounds__(kQThreads, 2) k_iterate_quads(QuadArgs a, const __grid_constant__ QuadMaps tm)
 {
     extern __shared__ __align__(128) float sm[];   // TMA tensor copies land on 128-byte boundaries
@@ -317,18 +306,18 @@ __global__ void __launch_bounds__(kQThreads, 2) k_iterate_quads(QuadArgs a, cons
             pd.lo.y = clamp1(pd.lo.y);
             pd.hi.x = clamp1(pd.hi.x);
             pd.hi.y = clamp1(pd.hi.y);
-            disc(puu.lo.x, puv.lo.x);
-            disc(puu.lo.y, puv.lo.y);
-            disc(puu.hi.x, puv.hi.x);
-            disc(puu.hi.y, puv.hi.y);
-            disc(pvu.lo.x, pvv.lo.x);
-            disc(pvu.lo.y, pvv.lo.y);
-            disc(pvu.hi.x, pvv.hi.x);
-            disc(pvu.hi.y, pvv.hi.y);
-            disc(pwu.lo.x, pwv.lo.x);
-            disc(pwu.lo.y, pwv.lo.y);
-            disc(pwu.hi.x, pwv.hi.x);
-            disc(pwu.hi.y, pwv.hi.y);
+            project_disc(puu.lo.x, puv.lo.x);
+            project_disc(puu.lo.y, puv.lo.y);
+            project_disc(puu.hi.x, puv.hi.x);
+            project_disc(puu.hi.y, puv.hi.y);
+            project_disc(pvu.lo.x, pvv.lo.x);
+            project_disc(pvu.lo.y, pvv.lo.y);
+            project_disc(pvu.hi.x, pvv.hi.x);
+            project_disc(pvu.hi.y, pvv.hi.y);
+            project_disc(pwu.lo.x, pwv.lo.x);
+            project_disc(pwu.lo.y, pwv.lo.y);
+            project_disc(pwu.hi.x, pwv.hi.x);
+            project_disc(pwu.hi.y, pwv.hi.y);
         }
         // ---------------- primal step (computeDivergence + updatePrimalVariables) ----------------
         {
