@@ -205,14 +205,75 @@ __global__ void k_pool_grad(const float* __restrict__ dy, int C, int n, int H, i
     dx[i] += dy[(((size_t)b * Ho + ho) * Wo + wo) * C + c] / (float)cnt;
 }
 
-// dY (bf16) = dA * relu'(A) (A the layer's bf16 output); no mask for the head.
-__global__ void k_relu_grad(const float* __restrict__ da, const __nv_bfloat16* __restrict__ a, size_t count,
-                            __nv_bfloat16* __restrict__ dy)
+// dY (bf16) = dA * relu'(A) (A the layer's bf16 output; no mask for the head),
+// and the column sums of the rounded dY [P][C] (the bias gradient) in the same
+// pass: a thread owns eight channels (one 16-byte piece) of every rows-th row
+// of its block's share, the block adds its threads in a fixed tree and writes
+// one partial sum a channel; k_bias_sum adds the blocks in order.  Bound by
+// memory (dA 4 B, A 2 B, dY 2 B a value).  Separate sums, a block per channel
+// striding through dY two bytes at a time, took 2.78 of the 8.3 ms of a
+// 64-input gradient on a GB300; this pass takes over the dY kernel's 0.14 ms.
+constexpr int kSumThreads = 256;
+constexpr unsigned kSumBlocks = 608;   // four 256-thread blocks on each of 152 SMs
+
+__global__ void __launch_bounds__(kSumThreads) k_relu_grad(const float* __restrict__ da,
+                                                           const __nv_bfloat16* __restrict__ a, size_t P, int C,
+                                                           __nv_bfloat16* __restrict__ dy, float* __restrict__ part)
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const float g = (!a || __bfloat162float(a[i]) > 0.f) ? da[i] : 0.f;
-    dy[i] = __float2bfloat16_rn(g);
+    __shared__ float red[kSumThreads][8 + 1];
+    const int pieces = C / 8, rows = kSumThreads / pieces;   // rows of a block at once (C = 96: 21, four threads idle)
+    const int piece = threadIdx.x % pieces, row = threadIdx.x / pieces;
+    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (row < rows)
+        for (size_t p = (size_t)blockIdx.x * rows + row; p < P; p += (size_t)gridDim.x * rows) {
+            const size_t i = p * C + piece * 8;
+            const float4 g0 = *reinterpret_cast<const float4*>(da + i), g1 = *reinterpret_cast<const float4*>(da + i + 4);
+            float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+            if (a) {
+                const uint4 av = *reinterpret_cast<const uint4*>(a + i);
+                const __nv_bfloat16* ap = reinterpret_cast<const __nv_bfloat16*>(&av);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) g[k] = __bfloat162float(ap[k]) > 0.f ? g[k] : 0.f;
+            }
+            uint4 out;
+            __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(&out);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                q[k] = __float2bfloat16_rn(g[k]);
+                sum[k] += __bfloat162float(q[k]);
+            }
+            *reinterpret_cast<uint4*>(dy + i) = out;
+        }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) red[threadIdx.x][k] = sum[k];
+    __syncthreads();
+    // thread t < C: channel t of the block, its rows added in pairs
+    for (int n = rows; n > 1; n = (n + 1) / 2) {
+        const int half = (n + 1) / 2;
+        if (row + half < n)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) red[threadIdx.x][k] += red[threadIdx.x + half * pieces][k];
+        __syncthreads();
+    }
+    for (int c = threadIdx.x; c < C; c += kSumThreads) part[(size_t)blockIdx.x * C + c] = red[c / 8][c % 8];
+}
+
+// The blocks' partial sums of k_relu_grad, added per channel: 16 warps a
+// channel block of 32 take every 16th partial, then a fixed tree.
+__global__ void __launch_bounds__(512) k_bias_sum(const float* __restrict__ part, int nblocks, int C, int cout,
+                                                  float* __restrict__ out)
+{
+    __shared__ float red[16][33];
+    const int c = blockIdx.x * 32 + threadIdx.x;
+    float s = 0.f;
+    if (c < C)
+        for (int b = threadIdx.y; b < nblocks; b += 16) s += part[(size_t)b * C + c];
+    red[threadIdx.y][threadIdx.x] = s;
+    for (int w = 8; w > 0; w >>= 1) {
+        __syncthreads();
+        if ((int)threadIdx.y < w) red[threadIdx.y][threadIdx.x] += red[threadIdx.y + w][threadIdx.x];
+    }
+    if (threadIdx.y == 0 && c < cout) out[c] = red[0][threadIdx.x];
 }
 
 // out[c][r] = in[r][c] for a rows x cols bf16 matrix (32 x 32 tiles); out's
@@ -235,22 +296,6 @@ __global__ void k_transpose(const __nv_bfloat16* __restrict__ in, size_t rows, s
         if (r < rows_pad && c < cols)
             out[(size_t)c * rows_pad + r] = r < rows ? t[threadIdx.x][k] : __float2bfloat16_rn(0.f);
     }
-}
-
-// Column sums of dY [P][C] (bias gradients); one block per channel, fixed order.
-__global__ void k_colsum(const __nv_bfloat16* __restrict__ dy, size_t P, int C, float* __restrict__ out)
-{
-    const int c = blockIdx.x;
-    float s = 0.f;
-    for (size_t p = threadIdx.x; p < P; p += blockDim.x) s += __bfloat162float(dy[p * C + c]);
-    __shared__ float red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[c] = red[0];
 }
 
 // Masked mean-squared error of the head output [P][16] against labels
@@ -675,15 +720,15 @@ int backward(pdflow_net* n, int nb)
                 k_pool_grad<<<blocks(size_t(nb) * a.H * a.W * a.C), 256, 0, st>>>(b.g, a.C, nb, a.H, a.W, a.g);
                 NET_TRY(cudaGetLastError(), "pool grad launch");
             }
-        // dY = dA * relu'(A)  (head: dY = dOut)
+        // dY = dA * relu'(A)  (head: dY = dOut) and the bias gradient
         const Act& o = n->act[c.out];
-        if (c.relu)
-            k_relu_grad<<<blocks(P * c.cout_pad), 256, 0, st>>>(o.g, o.x, P * c.cout_pad, n->dy);
-        else
-            k_relu_grad<<<blocks(P * 16), 256, 0, st>>>(n->dhead, nullptr, P * 16, n->dy);
+        const unsigned srows = unsigned(kSumThreads / (c.cout_pad / 8));
+        const unsigned nsum = std::min(kSumBlocks, unsigned((P + srows - 1) / srows));
+        k_relu_grad<<<nsum, kSumThreads, 0, st>>>(c.relu ? o.g : n->dhead, c.relu ? o.x : nullptr, P, c.cout_pad,
+                                                  n->dy, n->part);
         NET_TRY(cudaGetLastError(), "relu grad launch");
-        // bias gradient
-        k_colsum<<<c.cout, 256, 0, st>>>(n->dy, P, c.cout_pad, n->grad + c.boff);
+        k_bias_sum<<<unsigned((c.cout_pad + 31) / 32), dim3(32, 16), 0, st>>>(n->part, int(nsum), c.cout_pad, c.cout,
+                                                                             n->grad + c.boff);
         NET_TRY(cudaGetLastError(), "bias grad launch");
         // weight gradient: dW^T [K][cout_pad] = col^T [K][P] * dY^T [cout_pad][P]^T
         {
