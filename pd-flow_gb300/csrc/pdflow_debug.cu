@@ -271,7 +271,7 @@ __global__ void k_div_rcp_check(unsigned long long n, unsigned long long seed, u
         if ((r2 & 1023u) == 0) a = (r2 & 1024u) ? -0.f : 0.f;
         float b = rand_mag(r2 & 0x7fffffffu, -40, 59);
         if ((r1 & 255u) == 3) b = __fadd_rn(__uint_as_float((mix64(r1) & 0x007fffffu) | 0x2e000000u), 1e-10f);
-        if (__float_as_uint(div_rcp(a, b, __frcp_rn(b))) != __float_as_uint(__fdiv_rn(a, b))) ++mine;
+        if (__float_as_uint(div_rcp(-a, b, -__frcp_rn(b))) != __float_as_uint(__fdiv_rn(a, b))) ++mine;
     }
     if (mine) atomicAdd(bad, mine);
 }

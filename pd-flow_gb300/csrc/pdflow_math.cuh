@@ -331,22 +331,23 @@ __device__ __forceinline__ bool mag_in(float x, int lo, int hi)
     return (b << 1) == 0u || e - (unsigned)(127 + lo) <= (unsigned)(hi - lo);
 }
 
-// a / b correctly rounded, from y = RN(1/b) (__frcp_rn): q0 = RN(a y) is
-// within 2 ulp of a/b, one correction q1 = RN(q0 + RN(a - b q0) y) makes it
-// faithful, and by Markstein's theorem (P. Markstein, IBM J. Res. Dev.
-// 34(1), 1990; J.-M. Muller et al., Handbook of Floating-Point Arithmetic,
-// 2nd ed., sec. 4.7) the second, whose remainder a - b q1 the FMA forms
-// exactly, rounds it correctly: the bits of an IEEE division, in five
-// instructions once y is known.  Valid for a == 0 or 2^-60 <= |a| < 2^60 and
-// 2^-40 <= b < 2^60 (no intermediate leaves the normal range); a zero
-// numerator is returned as is (the sign of a / b).  Checked bit for bit
-// against __fdiv_rn on 1.7e10 random pairs of that range.
-__device__ __forceinline__ float div_rcp(float a, float b, float y)
+// a / b correctly rounded, from na = -a and ny = -RN(1/b) (__frcp_rn): q0 =
+// RN(a y) is within 2 ulp of a/b, one correction q1 = RN(q0 - RN(b q0 - a) y)
+// makes it faithful, and by Markstein's theorem (P. Markstein, IBM J. Res.
+// Dev. 34(1), 1990; J.-M. Muller et al., Handbook of Floating-Point
+// Arithmetic, 2nd ed., sec. 4.7) the second, whose remainder b q1 - a the FMA
+// forms exactly, rounds it correctly: the bits of an IEEE division, in five
+// instructions once y is known.  With the remainder taken as b q - a (not a -
+// b q) a zero numerator keeps the sign of a / b through both corrections, and
+// na and ny save the negations.  Valid for a == 0 or 2^-60 <= |a| < 2^60 and
+// 2^-40 <= b < 2^60, and up to |a| < 2^90 where |a / b| < 2^31 (no
+// intermediate leaves the normal range).  Checked bit for bit against
+// __fdiv_rn on 1.7e10 random pairs of that range.
+__device__ __forceinline__ float div_rcp(float na, float b, float ny)
 {
-    const float q0 = mul(a, y);
-    const float q1 = fm(fm(-q0, b, a), y, q0);
-    const float q2 = fm(fm(-q1, b, a), y, q1);
-    return a == 0.f ? a : q2;
+    const float q0 = mul(na, ny);
+    const float q1 = fm(fm(q0, b, na), ny, q0);
+    return fm(fm(q1, b, na), ny, q1);
 }
 
 // L1 photometric shrinkage of one pixel (pdflow_cudalib.cu:906-923) in the
@@ -362,26 +363,23 @@ __device__ __forceinline__ void shrink(float& du, float& dv, float of, float th,
     dv = lo ? add(dv, b1) : (hi ? sub(dv, b1) : mv_);
 }
 
-// The same with the quotients by div_rcp: den = th + 1e-10 and rden =
-// RN(1 / den) are the pixel's, fixed for the level (shrink_rcp_ok says when
-// the quotients are in div_rcp's range).
-__device__ __forceinline__ void shrink_rcp(float& du, float& dv, float of, float th, float den, float rden, float a1,
-                                           float b1)
+// Whether a pixel's shrinkage may divide by div_rcp (a pixel's a1, b1, th and
+// den = th + 1e-10 are fixed for the level): th >= 0, |a1| and |b1| zero or in
+// [2^-30, 2^30), den in [2^-40, 2^60).  The quotients a1 of / den, b1 of / den
+// are used only where |of| <= th < den (so they stay below 2^30) and are in
+// div_rcp's range when |of| is zero or at least 2^-30 (shrink_rcp_ok; false
+// for NaN).
+__device__ __forceinline__ bool shrink_rcp_level_ok(float a1, float b1, float th, float den)
 {
-    const float mu_ = sub(du, div_rcp(mul(a1, of), den, rden)), mv_ = sub(dv, div_rcp(mul(b1, of), den, rden));
-    const bool lo = of < -th, hi = of > th;
-    du = lo ? add(du, a1) : (hi ? sub(du, a1) : mu_);
-    dv = lo ? add(dv, b1) : (hi ? sub(dv, b1) : mv_);
+    return th >= 0.f && mag_in(a1, -30, 29) && mag_in(b1, -30, 29) && den >= 0x1p-40f && den < 0x1p60f;
 }
+__device__ __forceinline__ bool shrink_rcp_ok(float of) { return of == 0.f || fabsf(of) >= 0x1p-30f; }
 
-// Whether a pixel's shrinkage quotients a1 * of / den and b1 * of / den are
-// in div_rcp's range: |a1|, |b1| and |of| zero or in [2^-30, 2^30) (so the
-// numerators are zero or in [2^-60, 2^60)) and den in [2^-40, 2^60).
-__device__ __forceinline__ bool shrink_rcp_level_ok(float a1, float b1, float den)
+// a1 with the sign of optflow (the step outside the threshold), from na1 = -a1.
+__device__ __forceinline__ float signed_step(float na1, float of)
 {
-    return mag_in(a1, -30, 29) && mag_in(b1, -30, 29) && den >= 0x1p-40f && den < 0x1p60f;
+    return __uint_as_float(__float_as_uint(na1) ^ (~__float_as_uint(of) & 0x80000000u));
 }
-__device__ __forceinline__ bool shrink_rcp_ok(float of) { return mag_in(of, -30, 29); }
 
 // saturateVariables (pdflow_cudalib.cu:1018-1038).
 __device__ __forceinline__ void saturate(float& du, float& dv, float& dw, float du_prev, float dv_prev,

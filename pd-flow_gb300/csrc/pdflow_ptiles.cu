@@ -148,25 +148,25 @@ __device__ __forceinline__ void project_duals(float2& puu, float2& puv, float2& 
     }
 }
 
-// shrink_rcp (pdflow_math.cuh) for both pixels of a pair: the quotients'
-// Markstein corrections and the three cases' values in packed FP32x2 (each
-// lane the same correctly rounded operations), the case chosen per lane.
-__device__ __forceinline__ float2 div_rcp2(float2 a, float2 b, float2 y)
+// L1 photometric shrinkage (pdflow_cudalib.cu:906-923) for both pixels of a
+// pair: the step taken off du (dv) is the quotient a1 of / den inside the
+// threshold and a1 with the sign of `of` outside it (du - (-a1) is du + a1),
+// so one packed subtraction serves all three cases.  The quotients are
+// div_rcp's in packed FP32x2, from na1 = -a1 and nrden = -RN(1 / den).
+__device__ __forceinline__ float2 shrink_step2(float2 of, float2 den, float2 nrden, float2 na1, bool outx, bool outy)
 {
-    const float2 q0 = mul2(a, y);
-    const float2 q1 = fm2(fm2(neg2(q0), b, a), y, q0);
-    const float2 q2 = fm2(fm2(neg2(q1), b, a), y, q1);
-    return make_float2(a.x == 0.f ? a.x : q2.x, a.y == 0.f ? a.y : q2.y);
+    const float2 na = mul2(na1, of);
+    const float2 q0 = mul2(na, nrden);
+    const float2 q1 = fm2(fm2(q0, den, na), nrden, q0);
+    const float2 q2 = fm2(fm2(q1, den, na), nrden, q1);
+    return make_float2(outx ? signed_step(na1.x, of.x) : q2.x, outy ? signed_step(na1.y, of.y) : q2.y);
 }
-__device__ __forceinline__ void shrink_rcp2(float2& du, float2& dv, float2 of, float2 th, float2 den, float2 rden,
-                                            float2 a1, float2 b1)
+__device__ __forceinline__ void shrink_rcp2(float2& du, float2& dv, float2 of, float2 th, float2 den, float2 nrden,
+                                            float2 na1, float2 nb1)
 {
-    const float2 mu_ = sub2(du, div_rcp2(mul2(a1, of), den, rden));
-    const float2 mv_ = sub2(dv, div_rcp2(mul2(b1, of), den, rden));
-    const float2 pu = add2(du, a1), pv = add2(dv, b1), su = sub2(du, a1), sv = sub2(dv, b1);
-    const bool lox = of.x < -th.x, hix = of.x > th.x, loy = of.y < -th.y, hiy = of.y > th.y;
-    du = make_float2(lox ? pu.x : (hix ? su.x : mu_.x), loy ? pu.y : (hiy ? su.y : mu_.y));
-    dv = make_float2(lox ? pv.x : (hix ? sv.x : mv_.x), loy ? pv.y : (hiy ? sv.y : mv_.y));
+    const bool outx = fabsf(of.x) > th.x, outy = fabsf(of.y) > th.y;
+    du = sub2(du, shrink_step2(of, den, nrden, na1, outx, outy));
+    dv = sub2(dv, shrink_step2(of, den, nrden, nb1, outx, outy));
 }
 
 // One region of a CTA's walk: its origin, the rows and columns it stores,
@@ -391,8 +391,10 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
         const float2 th = fm2(a1, dcu, mul2(b1, dcv));
         // the shrinkage's denominators and their reciprocals, fixed for the level
         const float2 den = make_float2(add(th.x, 1e-10f), add(th.y, 1e-10f));
-        const float2 rden = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
-        const bool rcp_ok = shrink_rcp_level_ok(a1.x, b1.x, den.x) && shrink_rcp_level_ok(a1.y, b1.y, den.y);
+        const float2 nrden = make_float2(-__frcp_rn(den.x), -__frcp_rn(den.y));
+        const float2 na1 = neg2(a1), nb1 = neg2(b1);
+        const bool rcp_ok = shrink_rcp_level_ok(a1.x, b1.x, th.x, den.x) &&
+                            shrink_rcp_level_ok(a1.y, b1.y, th.y, den.y);
         // the iterations, with the image-border cases (kBorder) or, for a region
         // that touches no image border, without them (the same expressions)
         auto iterate = [&](auto border) {
@@ -483,10 +485,10 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
                     const float2 of = fm2(dcv, dv, fm2(dcu, du, dct));
                     // quotients by the reciprocal when the whole warp is in its range
                     if (__all_sync(0xffffffffu, rcp_ok && shrink_rcp_ok(of.x) && shrink_rcp_ok(of.y))) {
-                        shrink_rcp2(du, dv, of, th, den, rden, a1, b1);
+                        shrink_rcp2(du, dv, of, th, den, nrden, na1, nb1);
                     } else {
-                        shrink(du.x, dv.x, of.x, th.x, a1.x, b1.x);
-                        shrink(du.y, dv.y, of.y, th.y, a1.y, b1.y);
+                        shrink(du.x, dv.x, of.x, th.x, -na1.x, -nb1.x);
+                        shrink(du.y, dv.y, of.y, th.y, -na1.y, -nb1.y);
                     }
                     ua = fm2(two, du, neg2(du_old));
                     va = fm2(two, dv, neg2(dv_old));
