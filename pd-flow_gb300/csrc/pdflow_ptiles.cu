@@ -44,6 +44,16 @@
 // (the disc projection's work depends on the data) takes more of them; the
 // pieces keep the last units short.  The last CTA to finish resets the
 // counter for the next launch.
+//
+// Who does what.  Sixteen consumer warps hold the pixels; one lane of an
+// extra warpgroup walks the regions, writes each one's descriptor and starts
+// its copies as soon as the sixteen warps have read the staging planes (an
+// mbarrier they arrive on), so the walk's index arithmetic, the unit counter's
+// latency and the copies' issue are off the arithmetic's path, and a region
+// has no block barrier but the iterations' two.  Bound: instruction issue and
+// latency (16 warps an SM, the registers' limit; ~49 % issue active).  When
+// thread 0 of the consumers did the walk behind a block barrier a region, 64
+// VGA pairs took 35.74 ms and five 3.68 ms; with the producer 32.43 and 3.48.
 #include <cuda.h>
 
 #include <algorithm>
@@ -66,6 +76,14 @@ constexpr int kSR = 32;                        // region rows and columns
 // for levels whose launches are latency-bound, at four times the halo work).
 constexpr int kSPlane = kSR * kSR;             // floats per shared plane
 constexpr int kSThreads = kSR * kSR / 2;       // one thread per pixel pair (512)
+constexpr int kSWarps = kSThreads / 32;
+// The streamed launches add a producer warpgroup (setmaxnreg works on whole
+// warpgroups; one lane of it does the work).  640 threads launch with 96
+// registers each; the producer keeps 32 and the consumers take 112, which is
+// exactly the launch's total (128 * 32 + 512 * 112 = 640 * 96).
+constexpr int kSProducer = 128, kSLaunchRegs = 96, kSProducerRegs = 32, kSConsumerRegs = 112;
+static_assert(kSProducer * kSProducerRegs + kSThreads * kSConsumerRegs == (kSProducer + kSThreads) * kSLaunchRegs,
+              "the register split is the launch's total");
 
 // staging planes (TMA destinations, in the arena's order): 13 state, 19
 // constants; then the six exchange planes
@@ -180,6 +198,35 @@ struct Tile {
     int c1;                      // strips: the unit's end column
 };
 
+// What the consumer warps need of a region, as the producer writes it to
+// shared memory (two 16-byte reads): its origin, the rows and columns to
+// store (low and high halves of a word), the arena slot and flags.
+struct Region {
+    int rv0, ru0;
+    unsigned iv, iu;
+    unsigned slot, flags;
+    unsigned pad[2];
+};
+constexpr unsigned kRegMore = 1u, kRegCarryIn = 2u, kRegCarryOut = 4u, kRegLast = 8u, kRegBorder = 16u,
+                   kRegFinal = 32u;
+
+__device__ __forceinline__ Region region_of(const StreamArgs& a, const Tile& t)
+{
+    Region r;
+    const unsigned m = t.more && a.g.map ? __ldg(a.g.map + t.y) : t.y;
+    const int R = (int)a.g.R, C = (int)a.g.C;
+    r.rv0 = t.rv0;
+    r.ru0 = t.ru0;
+    r.iv = (unsigned)t.iv0 | (unsigned)t.iv1 << 16;
+    r.iu = (unsigned)t.iu0 | (unsigned)t.iu1 << 16;
+    r.slot = m & kMapSlotMask;
+    r.flags = (t.more ? kRegMore : 0u) | (t.carry_in ? kRegCarryIn : 0u) | (t.carry_out ? kRegCarryOut : 0u) |
+              (a.last || (a.g.map && (m & kMapLast)) ? kRegLast : 0u) |
+              (t.ru0 > 0 && t.ru0 + kSR < C && t.rv0 > 0 && t.rv0 + kSR < R ? 0u : kRegBorder);
+    r.pad[0] = r.pad[1] = 0u;
+    return r;
+}
+
 // Tiles: the launch's tile n (regions of every pair, dealt round-robin).
 __device__ __forceinline__ Tile tile_at(const StreamArgs& a, unsigned n)
 {
@@ -228,12 +275,12 @@ __device__ __forceinline__ Segment segment(const StreamArgs& a, unsigned k)
     return {false, 0, 0, 0};
 }
 
-// Strips: the region of unit k whose stored columns start at `col`.  With
-// the carry the region starts at that column; without it, kk columns further
-// left (their values go stale from the left, one column per iteration) or at
-// the image's first column.  Columns up to 32 - kk past the origin are exact
-// (all of them when the region reaches the image's last column).
-__device__ __forceinline__ Tile strip_at(const StreamArgs& a, unsigned k, int col, bool carry)
+// Strips: the first region of unit k.  It starts kk columns left of the
+// unit's first (their values go stale from the left, one column per
+// iteration) or at the image's first column.  Columns up to 32 - kk past the
+// origin are exact (all of them when the region reaches the image's last
+// column).
+__device__ __forceinline__ Tile strip_at(const StreamArgs& a, unsigned k)
 {
     Tile t;
     const Segment sg = segment(a, k);
@@ -241,38 +288,38 @@ __device__ __forceinline__ Tile strip_at(const StreamArgs& a, unsigned k, int co
     t.k = k;
     t.c1 = sg.c1;
     const int R = (int)a.g.R, C = (int)a.g.C, K = (int)a.kk;
-    if (col < 0) col = sg.c0;
+    const int col = sg.c0;
     t.y = sg.strip / a.tiles_v;
     const int tv = (int)(sg.strip - t.y * a.tiles_v);
     t.iv0 = tv * a.tile;
     t.iv1 = min(t.iv0 + a.tile, R);
     t.rv0 = max(t.iv0 - a.halo, 0);
-    t.ru0 = carry ? col : max(col - K, 0);
+    t.ru0 = max(col - K, 0);
     const int exact = (t.ru0 + kSR >= C) ? C : t.ru0 + kSR - K;
     t.iu0 = col;
     t.iu1 = min(exact, sg.c1);
-    t.carry_in = carry;
+    t.carry_in = false;
     t.carry_out = t.iu1 == exact && t.iu1 < sg.c1;   // the next region continues the unit
     return t;
 }
 
-// The region after t: the rest of t's unit, else unit `unit` (strips); the
-// CTA's next tile (tiles).
-template <bool kStrips>
-__device__ __forceinline__ Tile next_tile(const StreamArgs& a, const Tile& t, unsigned unit)
+// Strips: the region after t within t's unit (t.iu1 < t.c1): the same rows,
+// the columns from t's last exact one on, entered with the carry.
+__device__ __forceinline__ Tile continue_unit(const StreamArgs& a, Tile t)
 {
-    if constexpr (kStrips)
-        return t.iu1 < t.c1 ? strip_at(a, t.k, t.iu1, true) : strip_at(a, unit, -1, false);
-    else
-        return tile_at(a, t.k + gridDim.x);
+    const int C = (int)a.g.C, col = t.iu1;
+    const int exact = (col + kSR >= C) ? C : col + kSR - (int)a.kk;
+    t.ru0 = t.iu0 = col;
+    t.iu1 = min(exact, t.c1);
+    t.carry_in = true;
+    t.carry_out = t.iu1 == exact && t.iu1 < t.c1;
+    return t;
 }
 
-// Thread 0: the tensor copies of region t into the staging planes,
-// completing on `bar` (the caller's threads have finished reading staging).
-__device__ __forceinline__ void issue_region(const StreamArgs& a, const StreamMaps& tm, float* sm, uint32_t bar,
-                                             const Tile& t)
+// The tensor copies of a region into the staging planes, completing on `bar`
+// (every consumer warp has read staging).
+__device__ __forceinline__ void issue_region(const StreamMaps& tm, float* sm, uint32_t bar, const Region& r)
 {
-    const int slot = (int)(a.g.map ? (__ldg(a.g.map + t.y) & kMapSlotMask) : t.y);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier generic reads before async writes
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                  "r"((uint32_t)N_STAGE * (uint32_t)kSPlane * 4u)
@@ -280,13 +327,66 @@ __device__ __forceinline__ void issue_region(const StreamArgs& a, const StreamMa
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(sm + S_DU * kSPlane)),
-        "l"(reinterpret_cast<uint64_t>(&tm.state)), "r"(t.rv0), "r"(t.ru0), "r"(0), "r"(slot), "r"(bar)
+        "l"(reinterpret_cast<uint64_t>(&tm.state)), "r"(r.rv0), "r"(r.ru0), "r"(0), "r"((int)r.slot), "r"(bar)
         : "memory");
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(sm + K_RI * kSPlane)),
-        "l"(reinterpret_cast<uint64_t>(&tm.consts)), "r"(t.rv0), "r"(t.ru0), "r"(0), "r"(slot), "r"(bar)
+        "l"(reinterpret_cast<uint64_t>(&tm.consts)), "r"(r.rv0), "r"(r.ru0), "r"(0), "r"((int)r.slot), "r"(bar)
         : "memory");
+}
+
+// The producer lane: the CTA's walk (tiles blockIdx.x, + gridDim.x, ...; or,
+// strips, unit blockIdx.x, then the units it takes from the counter).  Per
+// region it waits until every consumer warp has read the staging planes of
+// the one before, writes the region's descriptor and starts its copies.  The
+// first region's are under way before the CTA's first barrier.  The walk ends
+// with a region marked kRegFinal (tiles: the next index is known) or with a
+// descriptor without kRegMore (strips: the next unit is taken only when the
+// last region of the one before has been issued).
+template <bool kStrips>
+__device__ __forceinline__ Region walk_region(const StreamArgs& a, const Tile& t)
+{
+    Region r = region_of(a, t);
+    if (!kStrips && t.k + gridDim.x >= a.total) r.flags |= kRegFinal;
+    return r;
+}
+template <bool kStrips>
+__device__ __forceinline__ void produce(const StreamArgs& a, const StreamMaps& tm, float* sm, Region* desc,
+                                        uint32_t full, uint32_t empty, Tile t)
+{
+    for (uint32_t n = 1; t.more; ++n) {   // region 0 is on its way (or there is none)
+        if constexpr (kStrips) {
+            t = t.iu1 < t.c1 ? continue_unit(a, t) : strip_at(a, gridDim.x + atomicAdd(a.work, 1u));
+        } else {
+            t = tile_at(a, t.k + gridDim.x);
+            if (!t.more) return;
+        }
+        const Region r = walk_region<kStrips>(a, t);
+        if (!mbar_wait(empty, (n - 1u) & 1u, kStreamWaitLimit)) {
+            atomicExch(a.status, kStreamTimeout);
+            mbar_wait(full, (n - 1u) & 1u, kStreamWaitLimit);   // bounded: the copies still in flight
+            return;
+        }
+        *desc = r;
+        if (!t.more) {
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full) : "memory");
+            break;
+        }
+        issue_region(tm, sm, full, r);
+    }
+    // strips: the last CTA to finish (every CTA has taken its last unit)
+    // clears the counter for the next launch
+    if (kStrips && atomicAdd(a.work + 1, 1u) == gridDim.x - 1) {
+        atomicExch(a.work, 0u);
+        atomicExch(a.work + 1, 0u);
+    }
+}
+
+// Barrier of the consumer warps (the producer warp takes no part).
+__device__ __forceinline__ void consumer_sync()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(kSThreads) : "memory");
 }
 
 // carry (strips): [buffer][iteration][u, v, w][region row] of the column
@@ -294,18 +394,41 @@ __device__ __forceinline__ void issue_region(const StreamArgs& a, const StreamMa
 constexpr int kCarryFloats = 2 * 4 * 3 * kSR;
 
 template <bool kStrips, bool kTma = true>
-__global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, const __grid_constant__ StreamMaps tm)
+__global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
+    k_iterate_stream(StreamArgs a, const __grid_constant__ StreamMaps tm)
 {
     static_assert(kTma || !kStrips, "the strips stream their regions");
     extern __shared__ __align__(128) float sm[];
-    __shared__ __align__(8) unsigned long long bar_mem;
-    __shared__ unsigned next_unit;   // strips: the unit thread 0 took for after the current one
+    __shared__ __align__(8) unsigned long long full_mem, empty_mem;   // staging landed / staging read
+    __shared__ __align__(16) Region desc;
+    __shared__ unsigned failed;                    // a consumer's wait ran out
     const int t = threadIdx.x;
+    const uint32_t full = smem_u32(&full_mem), empty = smem_u32(&empty_mem);
+    if constexpr (kTma) {
+        Tile first;
+        if (t == kSThreads) {
+            failed = 0u;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty), "n"(kSWarps));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            if constexpr (kStrips) first = strip_at(a, blockIdx.x);
+            else first = tile_at(a, blockIdx.x);
+            desc = walk_region<kStrips>(a, first);
+            if (first.more) issue_region(tm, sm, full, desc);
+            else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full) : "memory");
+        }
+        __syncthreads();   // the mbarriers' initialisation before anyone waits on them
+        if (t >= kSThreads) {
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSProducerRegs));
+            if (t == kSThreads) produce<kStrips>(a, tm, sm, &desc, full, empty, first);
+            return;
+        }
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSConsumerRegs));
+    }
     const int c = t >> 4, p = t & 15;              // region column, pixel pair
     const int me = c * kSR + 2 * p;                 // the pair's offset in a shared plane
     const int right = (c + 1 < kSR ? c + 1 : c) * kSR + 2 * p;   // beyond the region: own storage
     const int left = (c > 0 ? c - 1 : c) * kSR + 2 * p;
-    const uint32_t bar = smem_u32(&bar_mem);
     const int R = (int)a.g.R, C = (int)a.g.C;
     const float li = a.p.lambda_i, ld = a.p.lambda_d;
     const float2 li2 = make_float2(li, li), ld2 = make_float2(ld, ld), two = make_float2(2.f, 2.f);
@@ -319,29 +442,35 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
 
     float* carry = sm + N_PLANES * kSPlane;
     const int cc = kSR - 1 - (int)a.kk;              // strips: the column the next region needs
-    // this CTA's walk: tiles blockIdx.x, + gridDim.x, ...; or (strips) unit
-    // blockIdx.x, then the units it takes from the counter
-    Tile tl;
-    if constexpr (kStrips)
-        tl = strip_at(a, blockIdx.x, -1, false);
-    else
-        tl = tile_at(a, blockIdx.x);
-    if (kTma && t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (tl.more) issue_region(a, tm, sm, bar, tl);
-    }
-    __syncthreads();   // the mbarrier's initialisation before anyone waits on it
-    uint32_t phase = 0;
-    for (unsigned n = 0; tl.more; ++n) {
-        const size_t po = pair_off(a.g.map, a.g.pstride, tl.y);
-        const int u = tl.ru0 + c, v0 = tl.rv0 + 2 * p;
+    for (unsigned n = 0;; ++n) {
+        Region rg;
+        if constexpr (kTma) {
+            const bool ok = mbar_wait(full, n & 1u, kStreamWaitLimit);
+            rg = desc;
+            if (!ok) {   // go through this region's barriers without storing, then leave with the others
+                rg.rv0 = rg.ru0 = 0;
+                rg.iv = rg.iu = rg.slot = 0u;
+                rg.flags = kRegMore;
+                failed = 1u;
+                atomicExch(a.status, kStreamTimeout);
+            }
+            if (!(rg.flags & kRegMore)) {
+                // as many barriers as a region has, so that a warp whose wait
+                // for this descriptor ran out does not wait for the others
+                for (unsigned j = 0; j < 2 * a.kk; ++j) consumer_sync();
+                break;
+            }
+        } else {
+            rg = region_of(a, tile_at(a, blockIdx.x + n * gridDim.x));
+            if (!(rg.flags & kRegMore)) break;
+        }
+        const size_t po = (size_t)rg.slot * a.g.pstride;
+        const int u = rg.ru0 + c, v0 = rg.rv0 + 2 * p;
         const bool live = u < C && v0 < R;           // v0 < R implies v0 + 1 < R (R even)
         const bool fu = (u == 0), lu = (u == C - 1);
         const bool fv = (v0 == 0), lv = (v0 + 1 == R - 1);
-        const bool last_launch = a.last || (pair_flags(a.g.map, tl.y) & kMapLast);
+        const bool last_launch = rg.flags & kRegLast;
 
-        const bool ok = kTma ? mbar_wait(bar, phase, kStreamWaitLimit) : true;
         // the pair's value of plane k: from the staging copy, or loaded
         // directly (zero outside the image, as the tensor copy fills)
         auto ld2s = [&](int k) {
@@ -356,35 +485,18 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
                      ddu = ld2s(K_DDU), ddv = ld2s(K_DDV), s0 = ld2s(K_S0), s1 = ld2s(K_S1), s2 = ld2s(K_S2),
                      s3 = ld2s(K_S3), s4 = ld2s(K_S4), mu = ld2s(K_MU), dct = ld2s(K_DCT), dcu = ld2s(K_DCU),
                      dcv = ld2s(K_DCV), tu = ld2s(K_TU), tv = ld2s(K_TV), tw = ld2s(K_TW);
-        // staging read by every thread: the next region may land.  A wait that ran
-        // out anywhere ends the whole CTA (values read above are then unused)
-        if (__syncthreads_or(!ok)) {
-            if (t == 0) {
-                if (a.status) atomicExch(a.status, kStreamTimeout);
-                mbar_wait(bar, phase, kStreamWaitLimit);   // bounded: the copies still in flight
-            }
-            break;
-        }
-        phase ^= 1u;
-        if (kTma && t == 0) {
-            // the unit after this one (read by every thread after this tile's
-            // iteration barriers; rewritten only after the next tile's first)
-            unsigned unit = 0;
-            if (kStrips && tl.iu1 >= tl.c1) {
-                unit = gridDim.x + atomicAdd(a.work, 1u);
-                next_unit = unit;
-            }
-            const Tile nx = next_tile<kStrips>(a, tl, unit);
-            if (nx.more) issue_region(a, tm, sm, bar, nx);
+        if constexpr (kTma) {   // this warp has read staging: the next region may land once all have
+            __syncwarp();
+            if ((t & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty) : "memory");
         }
         // the left neighbour's exchange values: the carry of the previous
         // region (strips, first column) or the exchange planes; j advances
         // the carry by one iteration
-        const bool from_carry = kStrips && tl.carry_in && c == 0;
+        const bool from_carry = kStrips && (rg.flags & kRegCarryIn) && c == 0;
         const float* yl = from_carry ? carry + ((n + 1) & 1) * (4 * 3 * kSR) + 2 * p : sm + Y_U * kSPlane + left;
         const int yl_k = from_carry ? kSR : kSPlane, yl_j = from_carry ? 3 * kSR : 0;
         float* yc = carry + (n & 1) * (4 * 3 * kSR) + 2 * p;
-        const bool to_carry = kStrips && tl.carry_out && c == cc;
+        const bool to_carry = kStrips && (rg.flags & kRegCarryOut) && c == cc;
 
         const float2 mudu = mul2(mu, ddu), mudv = mul2(mu, ddv);
         const float2 a1 = mul2(tu, dcu), b1 = mul2(tv, dcv);
@@ -409,7 +521,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
                     const float Ub = __shfl_down_sync(0xffffffffu, U.x, 1, 16);   // the next pair's first row
                     const float Vb = __shfl_down_sync(0xffffffffu, V.x, 1, 16);
                     const float Wb = __shfl_down_sync(0xffffffffu, wa.x, 1, 16);
-                    __syncthreads();
+                    consumer_sync();
                     // borders by selects, not branches (the neighbour slot at the
                     // region's right edge is the thread's own: read, then dropped)
                     float2 gu1 = mul2(ri, sub2(*reinterpret_cast<const float2*>(XU + right), U));
@@ -456,7 +568,7 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
                     const float zua = __shfl_up_sync(0xffffffffu, zu.y, 1, 16);   // the previous pair's second row
                     const float zva = __shfl_up_sync(0xffffffffu, zv.y, 1, 16);
                     const float zwa = __shfl_up_sync(0xffffffffu, zw.y, 1, 16);
-                    __syncthreads();
+                    consumer_sync();
                     const float2 pu_[3] = {puu, pvu, pwu}, pv_[3] = {puv, pvv, pwv};
                     const float2 zm_[3] = {make_float2(zua, zu.x), make_float2(zva, zv.x), make_float2(zwa, zw.x)};
                     float2 div[3];
@@ -505,27 +617,23 @@ __global__ void __launch_bounds__(kSThreads, 1) k_iterate_stream(StreamArgs a, c
                 // one's first barrier, and the next stores to the same planes after it
             }
         };
-        if (tl.ru0 > 0 && tl.ru0 + kSR < C && tl.rv0 > 0 && tl.rv0 + kSR < R)   // the same for the whole CTA
-            iterate(std::false_type{});
-        else
-            iterate(std::true_type{});
+        if (rg.flags & kRegBorder) iterate(std::true_type{});   // the same for the whole CTA
+        else iterate(std::false_type{});
+        const bool lost = kTma && *reinterpret_cast<volatile unsigned*>(&failed);   // set before this region's barriers
+        if (lost) break;
 
         // ---- the interior to the destination buffer ----
-        if (live && v0 >= tl.iv0 && v0 < tl.iv1 && u >= tl.iu0 && u < tl.iu1) {
+        if (live && v0 >= int(rg.iv & 0xffffu) && v0 < int(rg.iv >> 16) && u >= int(rg.iu & 0xffffu) &&
+            u < int(rg.iu >> 16)) {
             const size_t gi = (size_t)v0 + (size_t)u * (size_t)R;
             const float2 st[13] = {du, dv, dw, ua, va, wa, pd, puu, puv, pvu, pvv, pwu, pwv};
 #pragma unroll
             for (int k = 0; k < 13; ++k) *reinterpret_cast<float2*>(at(a.dst[k], po) + gi) = st[k];
         }
-        // the next tile's staging wait is followed by a barrier before its first
-        // exchange store, so the exchange planes (and the carry) need none here
-        tl = next_tile<kStrips>(a, tl, kStrips ? next_unit : 0u);
-    }
-    // strips: the last CTA to finish (every CTA has taken its last unit)
-    // clears the counter for the next launch
-    if (kStrips && t == 0 && atomicAdd(a.work + 1, 1u) == gridDim.x - 1) {
-        atomicExch(a.work, 0u);
-        atomicExch(a.work + 1, 0u);
+        if (!kStrips && (rg.flags & kRegFinal)) break;
+        // the next region's first exchange stores (X planes, last read before
+        // this region's last barrier) and its first Y and carry stores (after
+        // its own first barrier) need no barrier here
     }
 }
 
@@ -595,6 +703,12 @@ cudaError_t prepare_stream_tiles()
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem_bytes());
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
+    // the consumers' setmaxnreg would wait for registers the launch did not bring
+    for (const void* k : {(const void*)k_iterate_stream<false>, (const void*)k_iterate_stream<true>}) {
+        cudaFuncAttributes fa{};
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k);
+        if (e == cudaSuccess && fa.numRegs != kSLaunchRegs) e = cudaErrorInvalidConfiguration;
+    }
     return e;
 }
 
@@ -654,9 +768,9 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
         !encode_plane_group(&maps.consts, cg[0], 19, cs, g.R, g.C, g.slots, g.pstride, kSR, kSR))
         return cudaErrorInvalidValue;
     if (strips)
-        k_iterate_stream<true><<<grid, kSThreads, stream_smem_bytes(), st>>>(a, maps);
+        k_iterate_stream<true><<<grid, kSThreads + kSProducer, stream_smem_bytes(), st>>>(a, maps);
     else
-        k_iterate_stream<false><<<grid, kSThreads, stream_smem_bytes(), st>>>(a, maps);
+        k_iterate_stream<false><<<grid, kSThreads + kSProducer, stream_smem_bytes(), st>>>(a, maps);
     return cudaGetLastError();
 }
 
