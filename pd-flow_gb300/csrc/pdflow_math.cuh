@@ -324,13 +324,6 @@ __device__ __forceinline__ void primal_update(float& du, float& dv, float& dw, f
     dwa = fm(2.f, dw, -dw_old);
 }
 
-// Whether x is 0 or 2^lo <= |x| < 2^(hi + 1) (from its exponent field).
-__device__ __forceinline__ bool mag_in(float x, int lo, int hi)
-{
-    const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xffu;
-    return (b << 1) == 0u || e - (unsigned)(127 + lo) <= (unsigned)(hi - lo);
-}
-
 // a / b correctly rounded, from na = -a and ny = -RN(1/b) (__frcp_rn): q0 =
 // RN(a y) is within 2 ulp of a/b, one correction q1 = RN(q0 - RN(b q0 - a) y)
 // makes it faithful, and by Markstein's theorem (P. Markstein, IBM J. Res.
@@ -364,14 +357,16 @@ __device__ __forceinline__ void shrink(float& du, float& dv, float of, float th,
 }
 
 // Whether a pixel's shrinkage may divide by div_rcp (a pixel's a1, b1, th and
-// den = th + 1e-10 are fixed for the level): th >= 0, |a1| and |b1| zero or in
-// [2^-30, 2^30), den in [2^-40, 2^60).  The quotients a1 of / den, b1 of / den
-// are used only where |of| <= th < den (so they stay below 2^30) and are in
-// div_rcp's range when |of| is zero or at least 2^-30 (shrink_rcp_ok; false
-// for NaN).
+// den = th + 1e-10 are fixed for the level): th >= 0 (so den > 2^-34), |a1| and
+// |b1| zero or in [2^-30, 2^30), den < 2^60; false for NaN.  The quotients a1
+// of / den, b1 of / den are used only where |of| <= th < den (so they stay
+// below 2^30) and are in div_rcp's range when |of| is zero or at least 2^-30
+// (shrink_rcp_ok; false for NaN).  Compares, not exponent fields: the test runs
+// once a region, 64 VGA pairs 32.46 -> 32.13 ms on a GB300.
 __device__ __forceinline__ bool shrink_rcp_level_ok(float a1, float b1, float th, float den)
 {
-    return th >= 0.f && mag_in(a1, -30, 29) && mag_in(b1, -30, 29) && den >= 0x1p-40f && den < 0x1p60f;
+    return th >= 0.f && (a1 == 0.f || fabsf(a1) >= 0x1p-30f) && (b1 == 0.f || fabsf(b1) >= 0x1p-30f) &&
+           fabsf(a1) < 0x1p30f && fabsf(b1) < 0x1p30f && den < 0x1p60f;
 }
 __device__ __forceinline__ bool shrink_rcp_ok(float of) { return of == 0.f || fabsf(of) >= 0x1p-30f; }
 
