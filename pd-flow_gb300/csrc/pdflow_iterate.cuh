@@ -93,6 +93,14 @@ size_t stream_smem_bytes();
 cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State dst, Params p, const float* depth_old,
                                   unsigned kk, bool last, cudaStream_t st, unsigned* status, unsigned ctas,
                                   StreamLayout layout);
+// Resident tiles (pdflow_resident.cu): every iteration of a small level in one
+// launch, a cluster per pair with a tile per CTA (the deep tiles' form, 9,
+// where the level fits a cluster); same preconditions as the streamed tiles
+// on direct loads and the same bits.  The final state is in `dst`.
+bool resident_eligible(const LevelGeom& g, const LevelConsts& L, const State& src, const State& dst, unsigned sms);
+cudaError_t prepare_resident();
+cudaError_t launch_iterate_resident(LevelGeom g, LevelConsts L, State src, State dst, Params p,
+                                    const float* depth_old, unsigned iters, cudaStream_t st);
 // L2 prefetch distance of the quad tiles in CTAs (0 = off).
 void set_quad_prefetch(unsigned ctas_ahead);
 size_t quads_smem_bytes();

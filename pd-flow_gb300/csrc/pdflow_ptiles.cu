@@ -62,13 +62,14 @@
 #include "pdflow_iterate.cuh"
 #include "pdflow_math.cuh"
 #include "pdflow_pack.cuh"
+#include "pdflow_region.cuh"
 #include "pdflow_tmap.h"
 
 namespace pdflow {
 
 namespace {
 
-using namespace pack;
+using namespace region;
 
 constexpr int kSR = 32;                        // region rows and columns
 // Interior and halo (= iterations per launch at most) are launch parameters:
@@ -119,73 +120,6 @@ struct StreamMaps {
 
 constexpr unsigned kStreamTimeout = 0x5354524Du;
 constexpr uint32_t kStreamWaitLimit = 1u << 22;
-
-__device__ __forceinline__ float clamp1(float pd) { return (fabsf(pd) > 1.f) ? ((pd > 1.f) ? 1.f : -1.f) : pd; }
-
-// The three TV duals' projections onto the unit disc (updateDualVariables,
-// pdflow_cudalib.cu:813-887) for both pixels of a pair, with disc_factor's
-// expressions in packed FP32x2.  A warp whose 64 pixels have all three duals
-// inside the disc (where the factors are 1 and the values stay) skips them:
-// one vote for the three.  On a GB300 against no vote: 64 VGA pairs 36.83 ->
-// 36.62 ms and 16 warm-started ones 8.94 -> 8.77 ms, five pairs 3.71 -> 3.76
-// ms; a vote a dual instead: 36.71, 8.87 and 3.75 ms.  A thread with a sum
-// beyond disc_factor's range takes the scalar form.
-struct Disc2 {
-    float2 s;
-    __device__ __forceinline__ Disc2(float2 a, float2 b)
-    {
-        const float2 hi = make_float2(max_nan(fabsf(a.x), fabsf(b.x)), max_nan(fabsf(a.y), fabsf(b.y)));
-        const float2 lo = make_float2(fminf(fabsf(a.x), fabsf(b.x)), fminf(fabsf(a.y), fabsf(b.y)));
-        s = fm2(hi, hi, mul2(lo, lo));
-    }
-    __device__ __forceinline__ float peak() const { return max_nan(s.x, s.y); }
-    __device__ __forceinline__ void apply(float2& a, float2& b) const
-    {
-        const float2 f = make_float2(rsqrt_min1(s.x), rsqrt_min1(s.y));
-        a = mul2(a, f);
-        b = mul2(b, f);
-    }
-};
-__device__ __forceinline__ void project_duals(float2& puu, float2& puv, float2& pvu, float2& pvv, float2& pwu,
-                                              float2& pwv)
-{
-    const Disc2 u(puu, puv), v(pvu, pvv), w(pwu, pwv);
-    const float peak = max_nan(max_nan(u.peak(), v.peak()), w.peak());
-    if (__all_sync(0xffffffffu, peak < 0.999f)) return;
-    if (peak < kDiscLimit) {
-        u.apply(puu, puv);
-        v.apply(pvu, pvv);
-        w.apply(pwu, pwv);
-    } else {
-        project_disc(puu.x, puv.x);
-        project_disc(puu.y, puv.y);
-        project_disc(pvu.x, pvv.x);
-        project_disc(pvu.y, pvv.y);
-        project_disc(pwu.x, pwv.x);
-        project_disc(pwu.y, pwv.y);
-    }
-}
-
-// L1 photometric shrinkage (pdflow_cudalib.cu:906-923) for both pixels of a
-// pair: the step taken off du (dv) is the quotient a1 of / den inside the
-// threshold and a1 with the sign of `of` outside it (du - (-a1) is du + a1),
-// so one packed subtraction serves all three cases.  The quotients are
-// div_rcp's in packed FP32x2, from na1 = -a1 and nrden = -RN(1 / den).
-__device__ __forceinline__ float2 shrink_step2(float2 of, float2 den, float2 nrden, float2 na1, bool outx, bool outy)
-{
-    const float2 na = mul2(na1, of);
-    const float2 q0 = mul2(na, nrden);
-    const float2 q1 = fm2(fm2(q0, den, na), nrden, q0);
-    const float2 q2 = fm2(fm2(q1, den, na), nrden, q1);
-    return make_float2(outx ? signed_step(na1.x, of.x) : q2.x, outy ? signed_step(na1.y, of.y) : q2.y);
-}
-__device__ __forceinline__ void shrink_rcp2(float2& du, float2& dv, float2 of, float2 th, float2 den, float2 nrden,
-                                            float2 na1, float2 nb1)
-{
-    const bool outx = fabsf(of.x) > th.x, outy = fabsf(of.y) > th.y;
-    du = sub2(du, shrink_step2(of, den, nrden, na1, outx, outy));
-    dv = sub2(dv, shrink_step2(of, den, nrden, nb1, outx, outy));
-}
 
 // One region of a CTA's walk: its origin, the rows and columns it stores,
 // and (strips) where the walk goes next.
@@ -430,16 +364,7 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
     const int right = (c + 1 < kSR ? c + 1 : c) * kSR + 2 * p;   // beyond the region: own storage
     const int left = (c > 0 ? c - 1 : c) * kSR + 2 * p;
     const int R = (int)a.g.R, C = (int)a.g.C;
-    const float li = a.p.lambda_i, ld = a.p.lambda_d;
-    const float2 li2 = make_float2(li, li), ld2 = make_float2(ld, ld), two = make_float2(2.f, 2.f);
     const float2 zero = make_float2(0.f, 0.f);
-    float* XU = sm + X_U * kSPlane;
-    float* XV = sm + X_V * kSPlane;
-    float* XW = sm + X_W * kSPlane;
-    float* YU = sm + Y_U * kSPlane;
-    float* YV = sm + Y_V * kSPlane;
-    float* YW = sm + Y_W * kSPlane;
-
     float* carry = sm + N_PLANES * kSPlane;
     const int cc = kSR - 1 - (int)a.kk;              // strips: the column the next region needs
     for (unsigned n = 0;; ++n) {
@@ -467,8 +392,7 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
         const size_t po = (size_t)rg.slot * a.g.pstride;
         const int u = rg.ru0 + c, v0 = rg.rv0 + 2 * p;
         const bool live = u < C && v0 < R;           // v0 < R implies v0 + 1 < R (R even)
-        const bool fu = (u == 0), lu = (u == C - 1);
-        const bool fv = (v0 == 0), lv = (v0 + 1 == R - 1);
+        const PairPlace place{u == 0, u == C - 1, v0 == 0, v0 + 1 == R - 1};
         const bool last_launch = rg.flags & kRegLast;
 
         // the pair's value of plane k: from the staging copy, or loaded
@@ -478,13 +402,11 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
             return live ? __ldg(reinterpret_cast<const float2*>(at(a.planes[k], po) + v0 + (size_t)u * (size_t)R))
                         : zero;
         };
-        float2 du = ld2s(S_DU), dv = ld2s(S_DV), dw = ld2s(S_DW), ua = ld2s(S_UA), va = ld2s(S_VA),
-               wa = ld2s(S_WA), pd = ld2s(S_PD), puu = ld2s(S_PUU), puv = ld2s(S_PUV), pvu = ld2s(S_PVU),
-               pvv = ld2s(S_PVV), pwu = ld2s(S_PWU), pwv = ld2s(S_PWV);
-        const float2 dup = ld2s(K_DUP), dvp = ld2s(K_DVP), ri = ld2s(K_RI), rj = ld2s(K_RJ), ddt = ld2s(K_DDT),
-                     ddu = ld2s(K_DDU), ddv = ld2s(K_DDV), s0 = ld2s(K_S0), s1 = ld2s(K_S1), s2 = ld2s(K_S2),
-                     s3 = ld2s(K_S3), s4 = ld2s(K_S4), mu = ld2s(K_MU), dct = ld2s(K_DCT), dcu = ld2s(K_DCU),
-                     dcv = ld2s(K_DCV), tu = ld2s(K_TU), tv = ld2s(K_TV), tw = ld2s(K_TW);
+        PairState s{ld2s(S_DU), ld2s(S_DV), ld2s(S_DW), ld2s(S_UA), ld2s(S_VA), ld2s(S_WA), ld2s(S_PD),
+                    ld2s(S_PUU), ld2s(S_PUV), ld2s(S_PVU), ld2s(S_PVV), ld2s(S_PWU), ld2s(S_PWV)};
+        const PairConsts k{ld2s(K_RI), ld2s(K_RJ), ld2s(K_DCT), ld2s(K_DCU), ld2s(K_DCV), ld2s(K_DDT), ld2s(K_DDU),
+                           ld2s(K_DDV), ld2s(K_MU), ld2s(K_DUP), ld2s(K_DVP), ld2s(K_S0), ld2s(K_S1), ld2s(K_S2),
+                           ld2s(K_S3), ld2s(K_S4), ld2s(K_TU), ld2s(K_TV), ld2s(K_TW)};
         if constexpr (kTma) {   // this warp has read staging: the next region may land once all have
             __syncwarp();
             if ((t & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty) : "memory");
@@ -498,123 +420,39 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
         float* yc = carry + (n & 1) * (4 * 3 * kSR) + 2 * p;
         const bool to_carry = kStrips && (rg.flags & kRegCarryOut) && c == cc;
 
-        const float2 mudu = mul2(mu, ddu), mudv = mul2(mu, ddv);
-        const float2 a1 = mul2(tu, dcu), b1 = mul2(tv, dcv);
-        const float2 th = fm2(a1, dcu, mul2(b1, dcv));
-        // the shrinkage's denominators and their reciprocals, fixed for the level
-        const float2 den = make_float2(add(th.x, 1e-10f), add(th.y, 1e-10f));
-        const float2 nrden = make_float2(-__frcp_rn(den.x), -__frcp_rn(den.y));
-        const float2 na1 = neg2(a1), nb1 = neg2(b1);
-        const bool rcp_ok = shrink_rcp_level_ok(a1.x, b1.x, th.x, den.x) &&
-                            shrink_rcp_level_ok(a1.y, b1.y, th.y, den.y);
+        const PairDerived d(k);
         // the iterations, with the image-border cases (kBorder) or, for a region
         // that touches no image border, without them (the same expressions)
+        struct Hooks {
+            const float* yl;
+            int yl_k;
+            float* yc;
+            bool to_carry;
+            __device__ __forceinline__ void sync() const { consumer_sync(); }
+            __device__ __forceinline__ void carry(float2 yu, float2 yv, float2 yw) const
+            {
+                if (to_carry) {
+                    *reinterpret_cast<float2*>(yc) = yu;
+                    *reinterpret_cast<float2*>(yc + kSR) = yv;
+                    *reinterpret_cast<float2*>(yc + 2 * kSR) = yw;
+                }
+            }
+            __device__ __forceinline__ const float* left(int c) const { return yl + c * yl_k; }
+        };
+        // saturated after the level's last iteration (strips: inside the loop, tiles:
+        // after it; the strips' loop with it outside takes 64 VGA pairs from 32.1 to
+        // 33.2 ms, the tiles' with it inside five from 3.44 to 3.46 ms)
+        auto finish = [&]() {
+            if (last_launch && live)
+                saturate_pair(s, k, __ldg(reinterpret_cast<const float2*>(at(a.depth_old, po) + v0 +
+                                                                          (size_t)u * (size_t)R)));
+        };
         auto iterate = [&](auto border) {
-            constexpr bool kBorder = decltype(border)::value;
             for (unsigned j = 0; j < a.kk; ++j) {
-                // ---------------- dual step (computeGradient + updateDualVariables) ----------------
-                {
-                    const float2 U = add2(ua, dup), V = add2(va, dvp);
-                    *reinterpret_cast<float2*>(XU + me) = U;
-                    *reinterpret_cast<float2*>(XV + me) = V;
-                    *reinterpret_cast<float2*>(XW + me) = wa;
-                    const float Ub = __shfl_down_sync(0xffffffffu, U.x, 1, 16);   // the next pair's first row
-                    const float Vb = __shfl_down_sync(0xffffffffu, V.x, 1, 16);
-                    const float Wb = __shfl_down_sync(0xffffffffu, wa.x, 1, 16);
-                    consumer_sync();
-                    // borders by selects, not branches (the neighbour slot at the
-                    // region's right edge is the thread's own: read, then dropped)
-                    float2 gu1 = mul2(ri, sub2(*reinterpret_cast<const float2*>(XU + right), U));
-                    float2 gv1 = mul2(ri, sub2(*reinterpret_cast<const float2*>(XV + right), V));
-                    float2 gw1 = mul2(ri, sub2(*reinterpret_cast<const float2*>(XW + right), wa));
-                    if (kBorder && lu) {
-                        gu1 = zero;
-                        gv1 = zero;
-                        gw1 = zero;
-                    }
-                    float2 gu2 = mul2(rj, sub2(make_float2(U.y, Ub), U));
-                    float2 gv2 = mul2(rj, sub2(make_float2(V.y, Vb), V));
-                    float2 gw2 = mul2(rj, sub2(make_float2(wa.y, Wb), wa));
-                    if (kBorder && lv) {
-                        gu2.y = 0.f;
-                        gv2.y = 0.f;
-                        gw2.y = 0.f;
-                    }
-                    const float2 X = fm2(ddv, va, fm2(ddu, ua, sub2(ddt, wa)));
-                    pd = fm2(s0, X, pd);
-                    puu = fm2(s1, gu1, puu);
-                    puv = fm2(s2, gu2, puv);
-                    pvu = fm2(s1, gv1, pvu);
-                    pvv = fm2(s2, gv2, pvv);
-                    pwu = fm2(s3, gw1, pwu);
-                    pwv = fm2(s4, gw2, pwv);
-                    pd.x = clamp1(pd.x);
-                    pd.y = clamp1(pd.y);
-                    project_duals(puu, puv, pvu, pvv, pwu, pwv);
-                }
-                // ---------------- primal step (computeDivergence + updatePrimalVariables) ----------------
-                {
-                    const float2 yu = mul2(ri, puu), yv = mul2(ri, pvu), yw = mul2(ri, pwu);
-                    *reinterpret_cast<float2*>(YU + me) = yu;
-                    *reinterpret_cast<float2*>(YV + me) = yv;
-                    *reinterpret_cast<float2*>(YW + me) = yw;
-                    if (to_carry) {
-                        float* y = yc + j * (3 * kSR);
-                        *reinterpret_cast<float2*>(y) = yu;
-                        *reinterpret_cast<float2*>(y + kSR) = yv;
-                        *reinterpret_cast<float2*>(y + 2 * kSR) = yw;
-                    }
-                    const float2 zu = mul2(rj, puv), zv = mul2(rj, pvv), zw = mul2(rj, pwv);
-                    const float zua = __shfl_up_sync(0xffffffffu, zu.y, 1, 16);   // the previous pair's second row
-                    const float zva = __shfl_up_sync(0xffffffffu, zv.y, 1, 16);
-                    const float zwa = __shfl_up_sync(0xffffffffu, zw.y, 1, 16);
-                    consumer_sync();
-                    const float2 pu_[3] = {puu, pvu, pwu}, pv_[3] = {puv, pvv, pwv};
-                    const float2 zm_[3] = {make_float2(zua, zu.x), make_float2(zva, zv.x), make_float2(zwa, zw.x)};
-                    float2 div[3];
-    #pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const float2 ym = neg2(*reinterpret_cast<const float2*>(yl + k * yl_k + (int)j * yl_j));
-                        float2 d = fm2(ri, pu_[k], ym);
-                        // first / last / inner column
-                        if constexpr (kBorder) d = fu ? mul2(ri, pu_[k]) : (lu ? ym : d);
-                        float2 g = add2(d, fm2(rj, pv_[k], neg2(zm_[k])));
-                        if constexpr (kBorder) {
-                            if (fv) g.x = fm(rj.x, pv_[k].x, d.x);
-                            if (lv) g.y = fm(-rj.x, pv_[k].x, d.y);
-                        }
-                        div[k] = g;
-                    }
-                    const float2 du_old = du, dv_old = dv, dw_old = dw;
-                    du = fm2(neg2(tu), fm2(mudu, pd, neg2(mul2(li2, div[0]))), du);
-                    dv = fm2(neg2(tv), fm2(mudv, pd, neg2(mul2(li2, div[1]))), dv);
-                    {
-                        // per lane: see pdflow_pack.cuh on contraction of packed products
-                        const float2 tq = fm2(neg2(mu), pd, neg2(mul2(ld2, div[2])));
-                        dw.x = add(dw.x, mul(-tw.x, tq.x));
-                        dw.y = add(dw.y, mul(-tw.y, tq.y));
-                    }
-                    const float2 of = fm2(dcv, dv, fm2(dcu, du, dct));
-                    // quotients by the reciprocal when the whole warp is in its range
-                    if (__all_sync(0xffffffffu, rcp_ok && shrink_rcp_ok(of.x) && shrink_rcp_ok(of.y))) {
-                        shrink_rcp2(du, dv, of, th, den, nrden, na1, nb1);
-                    } else {
-                        shrink(du.x, dv.x, of.x, th.x, -na1.x, -nb1.x);
-                        shrink(du.y, dv.y, of.y, th.y, -na1.y, -nb1.y);
-                    }
-                    ua = fm2(two, du, neg2(du_old));
-                    va = fm2(two, dv, neg2(dv_old));
-                    wa = fm2(two, dw, neg2(dw_old));
-                    if (last_launch && j + 1 == a.kk && live) {
-                        // saturateVariables (pdflow_cudalib.cu:1018-1038) after the level's last iteration
-                        const float2 z = __ldg(reinterpret_cast<const float2*>(at(a.depth_old, po) + v0 +
-                                                                                (size_t)u * (size_t)R));
-                        saturate(du.x, dv.x, dw.x, dup.x, dvp.x, z.x);
-                        saturate(du.y, dv.y, dw.y, dup.y, dvp.y, z.y);
-                    }
-                }
-                // no barrier here: this iteration's exchange reads happen before the next
-                // one's first barrier, and the next stores to the same planes after it
+                iterate_pair<decltype(border)::value, kSR / 2>(
+                    s, k, d, sm + X_U * kSPlane, sm + Y_U * kSPlane, kSPlane, me, right, place, a.p.lambda_i,
+                    a.p.lambda_d, Hooks{yl + (int)j * yl_j, yl_k, yc + (int)j * (3 * kSR), to_carry});
+                if (kStrips && j + 1 == a.kk) finish();
             }
         };
         if (rg.flags & kRegBorder) iterate(std::true_type{});   // the same for the whole CTA
@@ -622,13 +460,14 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
         const bool lost = kTma && *reinterpret_cast<volatile unsigned*>(&failed);   // set before this region's barriers
         if (lost) break;
 
+        if (!kStrips) finish();
         // ---- the interior to the destination buffer ----
         if (live && v0 >= int(rg.iv & 0xffffu) && v0 < int(rg.iv >> 16) && u >= int(rg.iu & 0xffffu) &&
             u < int(rg.iu >> 16)) {
             const size_t gi = (size_t)v0 + (size_t)u * (size_t)R;
-            const float2 st[13] = {du, dv, dw, ua, va, wa, pd, puu, puv, pvu, pvv, pwu, pwv};
+            const float2 st[13] = {s.du, s.dv, s.dw, s.ua, s.va, s.wa, s.pd, s.puu, s.puv, s.pvu, s.pvv, s.pwu, s.pwv};
 #pragma unroll
-            for (int k = 0; k < 13; ++k) *reinterpret_cast<float2*>(at(a.dst[k], po) + gi) = st[k];
+            for (int q = 0; q < 13; ++q) *reinterpret_cast<float2*>(at(a.dst[q], po) + gi) = st[q];
         }
         if (!kStrips && (rg.flags & kRegFinal)) break;
         // the next region's first exchange stores (X planes, last read before

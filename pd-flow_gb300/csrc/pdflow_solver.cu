@@ -224,6 +224,7 @@ static int level_form(const pdflow_solver* s, const LevelGeom& g, unsigned pairs
 {
     const int forced = level < 8 ? s->level_form[level] : -1;
     if (forced >= 0) return forced;
+    if (s->iter_form == 10 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms))) return 9;
     if (s->iter_form == 10 && (pairs * ((g.R + 23u) / 24u) < unsigned(s->num_sms) ||
                                !stream_eligible(g, s->L, s->S, s->S, 10)))
         return pairs * ((g.R + 15u) / 16u) * ((g.C + 15u) / 16u) <= unsigned(s->num_sms) ? 9 : 8;
@@ -269,7 +270,12 @@ static int enqueue_iterations(pdflow_solver* s, cudaStream_t st, const LevelGeom
     const bool quads = tiles && level_runs_quads(s, g, iters, pairs, level);
     const bool paired = tiles && form >= 3;
     const int shape = form >= 7 ? 2 : form - 3;   // 40x40, 40x34, 24x24 or 24x28 tiles (forms 7-10 elsewhere: 24x24)
-    if (tiles) {
+    if (quads && form == 9 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms))) {
+        *fin = State{s->alt_d[0], s->alt_d[1], s->alt_d[2], s->alt[0], s->alt[1], s->alt[2], s->alt[3], s->alt[4],
+                     s->alt[5], s->alt[6], s->alt[7], s->alt[8], s->alt[9]};
+        CUDA_TRY(launch_iterate_resident(g, s->L, s->S, *fin, p, o.dep, iters, st), "resident tile iteration launch");
+        *count += 1;
+    } else if (tiles) {
         State cur = s->S;
         State nxt{s->alt_d[0], s->alt_d[1], s->alt_d[2], s->alt[0], s->alt[1], s->alt[2], s->alt[3], s->alt[4],
                   s->alt[5], s->alt[6], s->alt[7], s->alt[8], s->alt[9]};
@@ -546,6 +552,7 @@ int pdflow_create_batch(unsigned rows, unsigned width, unsigned height, const pd
             CUDA_TRY(prepare_tiles2(), "kernel attributes");
             CUDA_TRY(prepare_quads(), "kernel attributes");
             CUDA_TRY(prepare_stream_tiles(), "kernel attributes");
+            CUDA_TRY(prepare_resident(), "kernel attributes");
             if (dev < 64) prepared |= 1ull << dev;
         }
     }
