@@ -197,18 +197,16 @@ LevelGeom level_geom(const pdflow_solver* s, unsigned i, unsigned* level_image, 
 // run as one launch (k_iterate: one CTA, one cluster, or, for a single pair,
 // the cooperative full grid) or, for a batch of pairs at a level that needs
 // the full grid, as two batched kernels per iteration.
-// Whether level `level`'s iterations run as shared-memory tiles (which
-// recompute the step sizes in registers).  Batches: tiles at every level
-// (measured faster than the cluster-persistent form from 15x20 up to 120x160
-// too); a single pair: tiles above 15x20 (per iteration at 30x40 .. 120x160
-// about half the time of the one-launch form; whole VGA solves 2.00 against
-// 2.34 ms, QVGA 1.22 against 1.55 ms), the one-CTA launch at 15x20.
-static bool level_runs_tiles(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned pairs,
-                             unsigned level)
+// Whether level `level`'s iterations run as tiles.  The 15x20 level runs as one
+// launch with a CTA per pair (register-resident, one pixel a thread) instead:
+// per VGA solve 0.034 ms for any batch up to an SM per pair, against 0.085 ms of
+// paired tiles (64 pairs).  Everything larger runs tiles (per iteration at
+// 30x40 .. 120x160 about half the time of the one-launch form).
+static bool level_runs_tiles(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned level)
 {
     const int forced = level < 8 ? s->level_form[level] : -1;
     if (forced >= 0) return forced >= 2 && iters > 0;
-    return s->iter_form >= 2 && iters > 0 && (pairs > 1 || g.N > 300u);
+    return s->iter_form >= 2 && iters > 0 && g.N > 300u;
 }
 
 // The level's iteration form: its autotuned or hand-set form, else the
@@ -238,7 +236,7 @@ static int level_form(const pdflow_solver* s, const LevelGeom& g, unsigned pairs
 static bool level_runs_quads(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned pairs,
                              unsigned level)
 {
-    if (!level_runs_tiles(s, g, iters, pairs, level)) return false;
+    if (!level_runs_tiles(s, g, iters, level)) return false;
     const int form = level_form(s, g, pairs, level);
     return (form >= 7 && form <= 10) && stream_eligible(g, s->L, s->S, s->S, form);
 }
@@ -248,7 +246,7 @@ static int level_steps(const pdflow_solver* s, const LevelGeom& g, unsigned iter
                        bool all_steps)
 {
     if (all_steps) return kStepsAll;
-    if (!level_runs_tiles(s, g, iters, pairs, level)) return kStepsRaw;
+    if (!level_runs_tiles(s, g, iters, level)) return kStepsRaw;
     return level_runs_quads(s, g, iters, pairs, level) ? kStepsQuads : kStepsNone;
 }
 
@@ -263,7 +261,7 @@ static int enqueue_iterations(pdflow_solver* s, cudaStream_t st, const LevelGeom
     const IterPlan pl = plan_iterate(g, s->num_sms);
     const int forced = level < 8 ? s->level_form[level] : -1;
     const bool one_launch_ok = (pairs == 1 || pl.mode != kIterGrid) && pl.smem_bytes <= iterate_smem_limit();
-    const bool tiles = level_runs_tiles(s, g, iters, pairs, level);
+    const bool tiles = level_runs_tiles(s, g, iters, level);
     const int form = level_form(s, g, pairs, level);
     const bool one_launch = forced >= 0 ? (forced == 1 && iters > 0 && one_launch_ok)
                                         : (s->iter_form >= 1 && iters > 0 && !tiles && one_launch_ok);
