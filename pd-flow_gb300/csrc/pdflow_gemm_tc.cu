@@ -12,7 +12,9 @@
 // commits them to the stage's mbarrier, which frees the stage for the chunk
 // three ahead.  The epilogue
 // reads the accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 =
-// rows of the tile), adds the bias, applies ReLU and stores FP32 or BF16.
+// rows of the tile), adds the bias, applies ReLU and stores FP32 or BF16, 16
+// bytes at a time where rows are aligned (a value at a time, a 64-input
+// gradient took 6.87 ms on a GB300 instead of 5.36).
 // grid.z splits K (split-K partials go to C + z * split_stride).
 //
 // Every wait is bounded: a wait that gives up records kGemmTimeout in
@@ -272,17 +274,33 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(GemmArgs a)
                 if (a.relu) x = fmaxf(x, 0.f);
                 v[j] = x;
             }
+            const bool whole = a.vec && col0 + 16 <= a.N;   // 16-byte stores
             if (a.out_bf16) {
                 __nv_bfloat16* C = static_cast<__nv_bfloat16*>(a.C) + (size_t)row * a.ldc + col0;
+                if (whole) {
+                    uint4 q[2];
+                    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(q);
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (col0 + j < a.N) C[j] = __float2bfloat16_rn(v[j]);
+                    for (int j = 0; j < 8; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                    reinterpret_cast<uint4*>(C)[0] = q[0];
+                    reinterpret_cast<uint4*>(C)[1] = q[1];
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (col0 + j < a.N) C[j] = __float2bfloat16_rn(v[j]);
+                }
             } else {
                 float* C =
                     static_cast<float*>(a.C) + (size_t)blockIdx.z * a.split_stride + (size_t)row * a.ldc + col0;
+                if (whole) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (col0 + j < a.N) C[j] = v[j];
+                    for (int j = 0; j < 4; ++j)
+                        reinterpret_cast<float4*>(C)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (col0 + j < a.N) C[j] = v[j];
+                }
             }
         }
         __syncwarp();
@@ -323,6 +341,9 @@ cudaError_t launch_gemm_tc(const GemmArgs& args, cudaStream_t st)
         a.N <= 0 || a.K <= 0)
         return cudaErrorInvalidValue;
     if (a.k_per_split <= 0) a.k_per_split = a.K;
+    // the epilogue's 16-byte stores: every row and split starts on one
+    const int unit = a.out_bf16 ? 8 : 4;
+    a.vec = reinterpret_cast<uintptr_t>(a.C) % 16u == 0 && a.ldc % unit == 0 && a.split_stride % unit == 0;
     a.k_per_split = (a.k_per_split + kBK - 1) / kBK * kBK;
     const unsigned splits = (unsigned)((a.K + a.k_per_split - 1) / a.k_per_split);
     if (splits > 1 && a.out_bf16) return cudaErrorInvalidValue;

@@ -36,6 +36,7 @@ struct GemmArgs {
     int k_per_split = 0;          // 0: no split
     size_t split_stride = 0;      // elements
     unsigned* status = nullptr;   // device word, kGemmTimeout on a bounded-wait timeout
+    int vec = 0;                  // set by the launcher: the epilogue may store 16 bytes at once
     int conv_a = 0;               // 1: A is conv's im2col (A, lda unused)
     ConvGather conv;
 };
