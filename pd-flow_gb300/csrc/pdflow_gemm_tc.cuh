@@ -38,6 +38,8 @@ struct GemmArgs {
     unsigned* status = nullptr;   // device word, kGemmTimeout on a bounded-wait timeout
     int vec = 0;                  // set by the launcher: the epilogue may store 16 bytes at once
     int conv_a = 0;               // 1: A is conv's im2col (A, lda unused)
+    int weight_grad = 0;          // 1: C[M][N] = im2col^T * B: A = conv's im2col (M values a pixel, K pixels),
+                                  // B [K][ldb] with N contiguous (conv_a set, lda unused)
     ConvGather conv;
 };
 

@@ -276,28 +276,6 @@ __global__ void __launch_bounds__(512) k_bias_sum(const float* __restrict__ part
     if (threadIdx.y == 0 && c < cout) out[c] = red[0][threadIdx.x];
 }
 
-// out[c][r] = in[r][c] for a rows x cols bf16 matrix (32 x 32 tiles); out's
-// rows are rows_pad long, zero beyond `rows`.
-__global__ void k_transpose(const __nv_bfloat16* __restrict__ in, size_t rows, size_t rows_pad, int cols,
-                            __nv_bfloat16* __restrict__ out)
-{
-    __shared__ __nv_bfloat16 t[32][33];
-    const size_t r0 = (size_t)blockIdx.x * 32;
-    const int c0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const size_t r = r0 + k;
-        const int c = c0 + threadIdx.x;
-        if (r < rows && c < cols) t[k][threadIdx.x] = in[r * cols + c];
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c = c0 + k;
-        const size_t r = r0 + threadIdx.x;
-        if (r < rows_pad && c < cols)
-            out[(size_t)c * rows_pad + r] = r < rows ? t[threadIdx.x][k] : __float2bfloat16_rn(0.f);
-    }
-}
-
 // Masked mean-squared error of the head output [P][16] against labels
 // [n][3][HW] (du, dv, 20 dw) on pixels whose old depth is valid; writes
 // dOut and one partial loss per block.
@@ -440,7 +418,7 @@ struct pdflow_net {
     float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;   // fp32 [nparams]
     std::vector<__nv_bfloat16*> Wb, WTb;                               // per conv bf16 weights
     std::vector<float*> gT;                                            // per conv dW^T [K][cout_pad]
-    __nv_bfloat16 *col = nullptr, *colT = nullptr, *dy = nullptr, *dyT = nullptr;
+    __nv_bfloat16 *col = nullptr, *dy = nullptr;
     float *dcol = nullptr, *dcat = nullptr, *head = nullptr, *dhead = nullptr, *part = nullptr;
     float *loss_part = nullptr, *input = nullptr;
     unsigned* count = nullptr;
@@ -606,6 +584,22 @@ T* dalloc(pdflow_net* n, size_t count, cudaError_t* e)
 // latency-bound.  Both give the same bits.
 constexpr int kImplicitConvMinBatch = 16;
 
+// A operand of `g`: the im2col of convolution c over its source activations.
+void set_gather(GemmArgs& g, const Conv& c, const Act& a1, const Act* a2)
+{
+    g.conv_a = 1;
+    g.conv.s1 = a1.x;
+    g.conv.s2 = a2 ? a2->x : nullptr;
+    g.conv.c1 = c.c1;
+    g.conv.c2 = c.c2;
+    g.conv.up1 = c.up1;
+    g.conv.H1 = a1.H;
+    g.conv.W1 = a1.W;
+    g.conv.H = c.H;
+    g.conv.W = c.W;
+    g.A = a1.x;
+}
+
 int conv_forward(pdflow_net* n, const Conv& c, size_t ci, int nb)
 {
     cudaStream_t st = n->stream;
@@ -616,17 +610,7 @@ int conv_forward(pdflow_net* n, const Conv& c, size_t ci, int nb)
     const int K = c.K();
     GemmArgs g;
     if (nb >= kImplicitConvMinBatch) {
-        g.conv_a = 1;
-        g.conv.s1 = a1.x;
-        g.conv.s2 = a2 ? a2->x : nullptr;
-        g.conv.c1 = c.c1;
-        g.conv.c2 = c.c2;
-        g.conv.up1 = c.up1;
-        g.conv.H1 = a1.H;
-        g.conv.W1 = a1.W;
-        g.conv.H = c.H;
-        g.conv.W = c.W;
-        g.A = a1.x;
+        set_gather(g, c, a1, a2);
     } else {
         k_im2col<<<blocks(P * 9 * (K / 72)), 256, 0, st>>>(a1.x, c.c1, c.up1, a1.H, a1.W, a2 ? a2->x : nullptr,
                                                            c.c2, nb, c.H, c.W, n->col);
@@ -730,39 +714,30 @@ int backward(pdflow_net* n, int nb)
         k_bias_sum<<<unsigned((c.cout_pad + 31) / 32), dim3(32, 16), 0, st>>>(n->part, int(nsum), c.cout_pad, c.cout,
                                                                              n->grad + c.boff);
         NET_TRY(cudaGetLastError(), "bias grad launch");
-        // weight gradient: dW^T [K][cout_pad] = col^T [K][P] * dY^T [cout_pad][P]^T
+        // weight gradient: dW^T [K][cout_pad] = im2col^T [K][P] * dY [P][cout_pad], both
+        // operands gathered as they lie (no im2col matrix, no transposed copies)
         {
             const Act& a1 = n->act[c.src1];
             const Act* a2 = c.src2 >= 0 ? &n->act[c.src2] : nullptr;
-            k_im2col<<<blocks(P * 9 * (K / 72)), 256, 0, st>>>(a1.x, c.c1, c.up1, a1.H, a1.W, a2 ? a2->x : nullptr,
-                                                               c.c2, nb, c.H, c.W, n->col);
-            NET_TRY(cudaGetLastError(), "im2col launch");
-            // the transposed operands have P (the GEMM's K) padded to a multiple of 8 with zeros
-            const size_t Pp = (P + 7) / 8 * 8;
-            dim3 tb(32, 8);
-            k_transpose<<<dim3(unsigned((Pp + 31) / 32), unsigned((K + 31) / 32)), tb, 0, st>>>(n->col, P, Pp, K,
-                                                                                                n->colT);
-            k_transpose<<<dim3(unsigned((Pp + 31) / 32), unsigned((c.cout_pad + 31) / 32)), tb, 0, st>>>(
-                n->dy, P, Pp, c.cout_pad, n->dyT);
-            NET_TRY(cudaGetLastError(), "transpose launch");
             GemmArgs g;
-            g.A = n->colT;
-            g.B = n->dyT;
+            g.weight_grad = 1;
+            set_gather(g, c, a1, a2);
+            g.B = n->dy;
             g.M = K;
             g.N = c.cout_pad;
-            g.K = int(Pp);
-            g.lda = int(Pp);
-            g.ldb = int(Pp);
+            g.K = int(P);
+            g.ldb = c.cout_pad;
             g.C = n->part;
             g.ldc = c.cout_pad;
             g.bn = c.cout_pad;
             const int target_splits = 256 / ((K + 127) / 128);
-            int kps = int((Pp + target_splits - 1) / target_splits);
+            const size_t target = (P + 7) / 8 * 8;   // pixels per split: a multiple of the GEMM's 64
+            int kps = int((target + target_splits - 1) / target_splits);
             kps = (kps + 63) / 64 * 64;
             g.k_per_split = kps;
             g.split_stride = size_t(K) * c.cout_pad;
             g.status = n->status;
-            const unsigned splits = gemm_splits(int(Pp), kps);
+            const unsigned splits = gemm_splits(int(P), kps);
             if (size_t(splits) * g.split_stride > n->part_elems) return net_fail(PDFLOW_ERR_ARG, "split-K buffer");
             NET_TRY(launch_gemm_tc(g, st), "weight-gradient GEMM launch");
             NET_TRY(launch_splitk_sum(n->part, int(splits), g.split_stride, K, c.cout_pad, c.cout_pad, n->gT[ci], st),
@@ -922,11 +897,9 @@ int pdflow_net_create(unsigned max_batch, unsigned long long seed, pdflow_net** 
     }
     n->col_elems = maxPK;
     n->col = dalloc<__nv_bfloat16>(n, maxPK, &e);
-    n->colT = dalloc<__nv_bfloat16>(n, maxPK, &e);
     n->dcol = dalloc<float>(n, maxPK, &e);
     n->dcat = dalloc<float>(n, maxPcin, &e);
     n->dy = dalloc<__nv_bfloat16>(n, B * kHW * 96, &e);
-    n->dyT = dalloc<__nv_bfloat16>(n, B * kHW * 96, &e);
     n->head = dalloc<float>(n, B * kHW * 16, &e);
     n->dhead = dalloc<float>(n, B * kHW * 16, &e);
     n->part_elems = 300 * maxK;

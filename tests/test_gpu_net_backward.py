@@ -47,3 +47,25 @@ def test_head_bias_gradient_is_the_sum_of_the_output_gradients(torch, n):
     terms = no.bf16((2 * d / (3 * int((inp[:, 2] > 0).sum()))).astype(np.float32)).astype(np.float64)
     got = g[head["boff"]:head["boff"] + 3].astype(np.float64)
     assert np.all(np.abs(got - terms.sum((0, 2))) <= 2e-5 * np.abs(terms).sum((0, 2)))
+
+
+@pytest.mark.parametrize("n", [1, 5])
+def test_gradients_against_the_oracle_at_ragged_pixel_counts(torch, n):
+    """1 and 5 inputs: the deep levels' pixel counts (80 and 400 at 10x8) are no
+    multiples of the GEMMs' 128 rows or of their split of the pixels.  Same
+    bound as for two inputs: well inside what bf16 rounding itself moves."""
+    net = Net(n, seed=3)
+    p = no.init_params(21)
+    net.set_params(p)
+    inp, label = _batch(30 + n, n)
+    d_in, d_lab = torch.from_numpy(inp).cuda(), torch.from_numpy(label).cuda()
+    loss, g = net.gradients(n, d_in.data_ptr(), d_lab.data_ptr())
+    net.close()
+    rloss, rq = no.NetOracle(p, quantize=True).loss_and_grads(inp, label)
+    _, rf = no.NetOracle(p, quantize=False).loss_and_grads(inp, label)
+    assert abs(loss - rloss) <= 1e-5 * rloss
+    rel = lambda x, y: np.linalg.norm(x - y) / max(np.linalg.norm(y), 1e-30)
+    for i, c in enumerate(no.GRAPH.convs):
+        lo, hi = c["woff"], c["woff"] + c["cout"] * c["K"]
+        e_gpu, e_bf16 = rel(g[lo:hi].astype(np.float64), rq[lo:hi]), rel(rq[lo:hi], rf[lo:hi])
+        assert e_gpu <= 0.75 * e_bf16 + 2e-3, (i, e_gpu, e_bf16)
