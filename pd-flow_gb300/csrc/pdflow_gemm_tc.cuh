@@ -45,6 +45,12 @@ struct GemmArgs {
 
 cudaError_t prepare_gemm_tc();
 cudaError_t launch_gemm_tc(const GemmArgs& a, cudaStream_t st);
+// out [P][cin] (FP32) = the input gradient of a 3x3 "same" convolution over n x H x
+// W pixels (P = n H W) from dY [P][co] and W^T [9 cin][co] (bf16): every tap's
+// product rounded to FP32 by itself, the taps added in order.  cin one of the
+// network's channel counts, co a multiple of 16 up to 96; out 16-byte aligned.
+cudaError_t launch_conv_dgrad(const void* dy, const void* wt, int P, int H, int W, int cin, int co, float* out,
+                              unsigned* status, cudaStream_t st);
 unsigned gemm_splits(int K, int k_per_split);
 cudaError_t launch_splitk_sum(const float* part, int splits, size_t stride, int M, int N, int ldc, float* out,
                               cudaStream_t st);

@@ -110,28 +110,6 @@ __global__ void k_im2col(const __nv_bfloat16* __restrict__ s1, int c1, int up1, 
     *reinterpret_cast<uint4*>(col + p * (size_t)(9 * cin) + tap * cin + ch * 8) = v;
 }
 
-// Gradient of im2col: d_in[q][c] = sum over taps of dcol[q - off(tap)][tap * Cin + c]
-// (FP32), written (not accumulated) into dcat [P][Cin].
-__global__ void k_col2im(const float* __restrict__ dcol, int cin, int n, int H, int W, float* __restrict__ dcat)
-{
-    const size_t total = (size_t)n * H * W * cin;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const int c = (int)(i % cin);
-    const size_t q = i / cin;
-    const int b = (int)(q / ((size_t)H * W)), r = (int)(q % ((size_t)H * W));
-    const int h = r / W, w = r % W;
-    float s = 0.f;
-#pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-        const int ph = h - (tap / 3 - 1), pw = w - (tap % 3 - 1);
-        if (ph < 0 || ph >= H || pw < 0 || pw >= W) continue;
-        const size_t p = ((size_t)b * H + ph) * W + pw;
-        s += dcol[p * (size_t)(9 * cin) + tap * cin + c];
-    }
-    dcat[i] = s;
-}
-
 // Splits the concatenated input gradient: channels [c1, c1 + c2) are added to
 // d2 (same resolution), channels [0, c1) to d1, summed over the 2x2 children
 // when src1 was upsampled from H1 x W1.
@@ -419,7 +397,7 @@ struct pdflow_net {
     std::vector<__nv_bfloat16*> Wb, WTb;                               // per conv bf16 weights
     std::vector<float*> gT;                                            // per conv dW^T [K][cout_pad]
     __nv_bfloat16 *col = nullptr, *dy = nullptr;
-    float *dcol = nullptr, *dcat = nullptr, *head = nullptr, *dhead = nullptr, *part = nullptr;
+    float *dcat = nullptr, *head = nullptr, *dhead = nullptr, *part = nullptr;
     float *loss_part = nullptr, *input = nullptr;
     unsigned* count = nullptr;
     unsigned* status = nullptr;
@@ -744,24 +722,11 @@ int backward(pdflow_net* n, int nb)
                     "split-K sum launch");
         }
         if (ci == 0) break;   // no gradient w.r.t. the input
-        // input gradient: dCol [P][K] = dY [P][cout_pad] * W^T  (B = WT [K][cout_pad])
+        // input gradient of the concatenated sources
         {
-            GemmArgs g;
-            g.A = n->dy;
-            g.B = n->WTb[ci];
-            g.M = int(P);
-            g.N = K;
-            g.K = c.cout_pad;
-            g.lda = c.cout_pad;
-            g.ldb = c.cout_pad;
-            g.C = n->dcol;
-            g.ldc = K;
-            g.bn = 128;
-            g.status = n->status;
-            NET_TRY(launch_gemm_tc(g, st), "input-gradient GEMM launch");
-            const int cin = c.c1 + c.c2;
-            k_col2im<<<blocks(P * cin), 256, 0, st>>>(n->dcol, cin, nb, c.H, c.W, n->dcat);
-            NET_TRY(cudaGetLastError(), "col2im launch");
+            NET_TRY(launch_conv_dgrad(n->dy, n->WTb[ci], int(P), c.H, c.W, c.c1 + c.c2, c.cout_pad, n->dcat,
+                                      n->status, st),
+                    "input-gradient launch");
             const Act& a1 = n->act[c.src1];
             const size_t t1 = c.up1 ? size_t(nb) * a1.H * a1.W * c.c1 : P * c.c1;
             const size_t t2 = P * c.c2;
@@ -897,7 +862,6 @@ int pdflow_net_create(unsigned max_batch, unsigned long long seed, pdflow_net** 
     }
     n->col_elems = maxPK;
     n->col = dalloc<__nv_bfloat16>(n, maxPK, &e);
-    n->dcol = dalloc<float>(n, maxPK, &e);
     n->dcat = dalloc<float>(n, maxPcin, &e);
     n->dy = dalloc<__nv_bfloat16>(n, B * kHW * 96, &e);
     n->head = dalloc<float>(n, B * kHW * 16, &e);
