@@ -535,16 +535,28 @@ __global__ void __launch_bounds__(kThreads) k_conv_dgrad(DgradArgs a)
     }
 }
 
-// Sums split-K partials [splits][M][ldc] into out [M][ldc] (fixed order).
+// Sums split-K partials [splits][M][ldc] in order into out: [M][ldc], or, with
+// `ldt`, its transpose [N][ldt].  Bound by the partials' latency: 16 of a
+// value's loads are in flight at once (a load at a time took 6-19 us for
+// matrices of a few kilobytes).
 __global__ void k_splitk_sum(const float* __restrict__ part, int splits, size_t stride, int M, int N, int ldc,
-                             float* __restrict__ out)
+                             float* __restrict__ out, int ldt)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)M * N) return;
-    const size_t r = i / N, c = i % N, o = r * ldc + c;
+    const size_t r = i / N, c = i % N;
+    const float* q = part + r * ldc + c;
     float s = 0.f;
-    for (int z = 0; z < splits; ++z) s += part[z * stride + o];
-    out[o] = s;
+    int z = 0;
+    for (; z + 16 <= splits; z += 16) {
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = q[(z + j) * stride];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s += v[j];
+    }
+    for (; z < splits; ++z) s += q[z * stride];
+    out[ldt ? c * ldt + r : r * ldc + c] = s;
 }
 
 }  // namespace
@@ -621,10 +633,10 @@ unsigned gemm_splits(int K, int k_per_split)
 }
 
 cudaError_t launch_splitk_sum(const float* part, int splits, size_t stride, int M, int N, int ldc, float* out,
-                              cudaStream_t st)
+                              cudaStream_t st, int ldt)
 {
     const size_t n = (size_t)M * N;
-    k_splitk_sum<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, splits, stride, M, N, ldc, out);
+    k_splitk_sum<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, splits, stride, M, N, ldc, out, ldt);
     return cudaGetLastError();
 }
 

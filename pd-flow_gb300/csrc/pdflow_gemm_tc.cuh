@@ -52,7 +52,9 @@ cudaError_t launch_gemm_tc(const GemmArgs& a, cudaStream_t st);
 cudaError_t launch_conv_dgrad(const void* dy, const void* wt, int P, int H, int W, int cin, int co, float* out,
                               unsigned* status, cudaStream_t st);
 unsigned gemm_splits(int K, int k_per_split);
+// Sums the partials of a split GEMM in order into out [M][ldc], or with ldt > 0
+// into its transpose [N][ldt].
 cudaError_t launch_splitk_sum(const float* part, int splits, size_t stride, int M, int N, int ldc, float* out,
-                              cudaStream_t st);
+                              cudaStream_t st, int ldt = 0);
 
 }  // namespace pdflow

@@ -306,11 +306,10 @@ __global__ void k_head_out(const float* __restrict__ out, int n, float* __restri
     s[2 * kHW + p] = out[(size_t)i * 16 + 2] * (1.f / kWScale);
 }
 
-// Adam on FP32 master weights w [cout][k] (gradient in the GEMM's transposed
-// layout gT [k][cout_pad]), then the bf16 copies W [cout_pad][k] and
+// Adam on FP32 master weights w [cout][k] (gradient g [cout][k]), then the bf16 copies W [cout_pad][k] and
 // WT [k][cout_pad] (padding rows stay zero).
 __global__ void k_adam_w(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                         const float* __restrict__ gT, int cout, int cout_pad, int k, float lr, float b1, float b2,
+                         const float* __restrict__ grad, int cout, int cout_pad, int k, float lr, float b1, float b2,
                          float eps, float c1, float c2, int update, __nv_bfloat16* __restrict__ W,
                          __nv_bfloat16* __restrict__ WT)
 {
@@ -319,7 +318,7 @@ __global__ void k_adam_w(float* __restrict__ w, float* __restrict__ m, float* __
     const int o = i / k, j = i % k;
     float x = w[i];
     if (update) {
-        const float g = gT[(size_t)j * cout_pad + o];
+        const float g = grad[i];
         const float mm = b1 * m[i] + (1.f - b1) * g;
         const float vv = b2 * v[i] + (1.f - b2) * g * g;
         m[i] = mm;
@@ -395,7 +394,6 @@ struct pdflow_net {
     // device buffers
     float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;   // fp32 [nparams]
     std::vector<__nv_bfloat16*> Wb, WTb;                               // per conv bf16 weights
-    std::vector<float*> gT;                                            // per conv dW^T [K][cout_pad]
     __nv_bfloat16 *col = nullptr, *dy = nullptr;
     float *dcat = nullptr, *head = nullptr, *dhead = nullptr, *part = nullptr;
     float *loss_part = nullptr, *input = nullptr;
@@ -661,8 +659,7 @@ int forward_full(pdflow_net* n, int nb, const float* input)
     return PDFLOW_OK;
 }
 
-// Backward pass from n->dhead ([P][16], FP32): fills n->gT (dW^T per conv)
-// and n->grad bias entries.
+// Backward pass from n->dhead ([P][16], FP32): fills n->grad (the parameters' layout).
 int backward(pdflow_net* n, int nb)
 {
     cudaStream_t st = n->stream;
@@ -718,7 +715,8 @@ int backward(pdflow_net* n, int nb)
             const unsigned splits = gemm_splits(int(P), kps);
             if (size_t(splits) * g.split_stride > n->part_elems) return net_fail(PDFLOW_ERR_ARG, "split-K buffer");
             NET_TRY(launch_gemm_tc(g, st), "weight-gradient GEMM launch");
-            NET_TRY(launch_splitk_sum(n->part, int(splits), g.split_stride, K, c.cout_pad, c.cout_pad, n->gT[ci], st),
+            NET_TRY(launch_splitk_sum(n->part, int(splits), g.split_stride, K, c.cout, c.cout_pad, n->grad + c.woff, st,
+                                      K),
                     "split-K sum launch");
         }
         if (ci == 0) break;   // no gradient w.r.t. the input
@@ -850,7 +848,6 @@ int pdflow_net_create(unsigned max_batch, unsigned long long seed, pdflow_net** 
     for (auto& c : n->conv) {
         n->Wb.push_back(dalloc<__nv_bfloat16>(n, size_t(c.cout_pad) * c.K(), &e));
         n->WTb.push_back(dalloc<__nv_bfloat16>(n, size_t(c.K()) * c.cout_pad, &e));
-        n->gT.push_back(dalloc<float>(n, size_t(c.K()) * c.cout_pad, &e));
         const size_t P = B * c.H * c.W, Pp = (P + 7) / 8 * 8;
         maxK = std::max(maxK, size_t(c.K()) * c.cout_pad);
         maxPK = std::max(maxPK, Pp * c.K());
@@ -956,20 +953,9 @@ int pdflow_net_gradients(pdflow_net* n, unsigned nb, const float* d_input, const
     rc = check_net_status(n);
     if (rc) return rc;
     if (grads) {
-        // canonical layout: per conv, dW [cout][K] then db [cout]
-        for (size_t i = 0; i < n->conv.size(); ++i) {
-            const Conv& c = n->conv[i];
-            std::vector<float> gt(size_t(c.K()) * c.cout_pad);
-            NET_TRY(cudaMemcpyAsync(gt.data(), n->gT[i], sizeof(float) * gt.size(), cudaMemcpyDeviceToHost,
-                                    n->stream),
-                    "D2H grads");
-            NET_TRY(cudaMemcpyAsync(grads + c.boff, n->grad + c.boff, sizeof(float) * c.cout, cudaMemcpyDeviceToHost,
-                                    n->stream),
-                    "D2H grads");
-            NET_TRY(cudaStreamSynchronize(n->stream), "synchronize");
-            for (int o = 0; o < c.cout; ++o)
-                for (int k = 0; k < c.K(); ++k) grads[c.woff + size_t(o) * c.K() + k] = gt[size_t(k) * c.cout_pad + o];
-        }
+        NET_TRY(cudaMemcpyAsync(grads, n->grad, sizeof(float) * n->nparams, cudaMemcpyDeviceToHost, n->stream),
+                "D2H grads");
+        NET_TRY(cudaStreamSynchronize(n->stream), "synchronize");
     }
     return PDFLOW_OK;
 }
@@ -990,7 +976,7 @@ int pdflow_net_train_step(pdflow_net* n, unsigned nb, const float* d_input, cons
     for (size_t i = 0; i < n->conv.size(); ++i) {
         const Conv& c = n->conv[i];
         k_adam_w<<<blocks(size_t(c.cout) * c.K()), 256, 0, n->stream>>>(
-            n->w + c.woff, n->m + c.woff, n->v + c.woff, n->gT[i], c.cout, c.cout_pad, c.K(), lr, b1, b2, eps, c1, c2,
+            n->w + c.woff, n->m + c.woff, n->v + c.woff, n->grad + c.woff, c.cout, c.cout_pad, c.K(), lr, b1, b2, eps, c1, c2,
             1, n->Wb[i], n->WTb[i]);
         k_adam_b<<<blocks(size_t(c.cout)), 256, 0, n->stream>>>(n->w + c.boff, n->m + c.boff, n->v + c.boff,
                                                                   n->grad + c.boff, c.cout, lr, b1, b2, eps, c1, c2);
