@@ -535,27 +535,37 @@ __global__ void __launch_bounds__(kThreads) k_conv_dgrad(DgradArgs a)
     }
 }
 
-// Sums split-K partials [splits][M][ldc] in order into out: [M][ldc], or, with
-// `ldt`, its transpose [N][ldt].  Bound by the partials' latency: 16 of a
-// value's loads are in flight at once (a load at a time took 6-19 us for
-// matrices of a few kilobytes).
-__global__ void k_splitk_sum(const float* __restrict__ part, int splits, size_t stride, int M, int N, int ldc,
-                             float* __restrict__ out, int ldt)
+// Sums split-K partials [splits][M][ldc] into out: [M][ldc], or, with `ldt`,
+// its transpose [N][ldt].  Bound by the partials' latency (a value has up to
+// 608 of them): eight threads a value add an eighth each in order, with 16
+// loads in flight, then the eighths are added in order.
+constexpr int kSumGroups = 8;
+__global__ void __launch_bounds__(32 * kSumGroups) k_splitk_sum(const float* __restrict__ part, int splits,
+                                                               size_t stride, int M, int N, int ldc,
+                                                               float* __restrict__ out, int ldt)
 {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M * N) return;
-    const size_t r = i / N, c = i % N;
+    __shared__ float red[kSumGroups][33];
+    const size_t i = (size_t)blockIdx.x * 32 + threadIdx.x;
+    const bool in = i < (size_t)M * N;
+    const size_t r = in ? i / N : 0, c = in ? i % N : 0;
     const float* q = part + r * ldc + c;
+    const int each = (splits + kSumGroups - 1) / kSumGroups;
+    int z = threadIdx.y * each;
+    const int end = min(splits, z + each);
     float s = 0.f;
-    int z = 0;
-    for (; z + 16 <= splits; z += 16) {
+    for (; z + 16 <= end; z += 16) {
         float v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] = q[(z + j) * stride];
 #pragma unroll
         for (int j = 0; j < 16; ++j) s += v[j];
     }
-    for (; z < splits; ++z) s += q[z * stride];
+    for (; z < end; ++z) s += q[z * stride];
+    red[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y != 0 || !in) return;
+#pragma unroll
+    for (int g = 1; g < kSumGroups; ++g) s += red[g][threadIdx.x];
     out[ldt ? c * ldt + r : r * ldc + c] = s;
 }
 
@@ -636,7 +646,7 @@ cudaError_t launch_splitk_sum(const float* part, int splits, size_t stride, int 
                               cudaStream_t st, int ldt)
 {
     const size_t n = (size_t)M * N;
-    k_splitk_sum<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, splits, stride, M, N, ldc, out, ldt);
+    k_splitk_sum<<<(unsigned)((n + 31) / 32), dim3(32, kSumGroups), 0, st>>>(part, splits, stride, M, N, ldc, out, ldt);
     return cudaGetLastError();
 }
 
