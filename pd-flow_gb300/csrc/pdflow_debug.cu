@@ -160,9 +160,12 @@ int pdflow_debug_solve(pdflow_solver* s, pdflow_dump_fn fn, void* ctx)
         unsigned li;
         const LevelGeom g = level_geom(s, i, &li);
         const PyrLevel o = s->pyr[fo][li], n = s->pyr[fn_][li];
-        cudaError_t e = launch_level_init(g, i == 0, s->sol, o, n, L, S, st);
-        if (e == cudaSuccess) e = launch_im_gradients(g, n, L, st);
-        if (e == cudaSuccess) e = launch_warp_steps(g, o, n, L, p, st);
+        const size_t aux = aux_offset(s, i);
+        cudaError_t e = launch_im_gradients(&g, &n, &aux, 1, L, st);
+        if (e == cudaSuccess)
+            e = launch_level_setup(g, i == 0 ? LevelStart::Zeros : LevelStart::Coarse, s->sol, o, n, L, S, p, kStepsRaw,
+                                   aux, st);
+        if (e == cudaSuccess) e = launch_rij2(g, n, L, st);
         if (e != cudaSuccess) return fail("set-up launch", e);
         const struct { const char* name; const float* ptr; } setup[] = {
             {"dct", L.dct}, {"dcu", L.dcu}, {"dcv", L.dcv}, {"ddt", L.ddt}, {"ddu", L.ddu}, {"ddv", L.ddv},

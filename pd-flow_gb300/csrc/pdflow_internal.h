@@ -111,6 +111,8 @@ int enqueue_energy(pdflow_solver* s, cudaStream_t st, unsigned pairs, unsigned l
 unsigned scaled_iters(unsigned iters, float scale);
 // Float offset of level `level`'s six planes in a slot of the per-level record.
 size_t level_keep_offset(const pdflow_solver* s, unsigned level);
+// Float offset of level `level`'s image gradients in the aux planes.
+size_t aux_offset(const pdflow_solver* s, unsigned level);
 // Runs fn(s, stream, pairs, ctx) on the handle's stream, through a cached CUDA
 // graph keyed by (new frame slot, pairs, iteration form, kind) in graph mode.
 // Whatever fn reads from ctx is baked into the graph: equal kinds must mean

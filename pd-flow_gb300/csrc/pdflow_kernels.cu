@@ -1,9 +1,9 @@
 // Stage kernels of the PD-Flow solver on sm_103a.
 //
 // One thread per pixel, column-major planes (idx = v + u*R, rows contiguous,
-// so a warp reads 32 consecutive rows of one column: coalesced).  The per-level
-// set-up is fused into three kernels (init = zero/upsample + connectivity,
-// image gradients, warp + step sizes), an iteration is two kernels
+// so a warp reads 32 consecutive rows of one column: coalesced).  The image
+// gradients of all levels are one kernel, a level's set-up two (starting point
+// and connectivity; warping and step sizes), an iteration is two kernels
 // (gradient+dual, divergence+primal; the reference uses four) and the last
 // primal kernel of a level also saturates; the weighted median and the motion
 // field are one kernel.  All per-pixel arithmetic lives in pdflow_math.cuh.
@@ -177,240 +177,217 @@ __global__ void k_pyr_down(PyrLevel prev, unsigned R, unsigned C, PyrLevel out, 
 // Level set-up
 // ---------------------------------------------------------------------------
 
-// upsampleCopy + upsampleFilterPrevSolution (pdflow_cudalib.cu:460-569) at one
-// pixel, as a gather over the coarse solution (the zero-inserted taps
-// contribute exactly zero and are skipped): acc = du dv dw pd puu puv pvu pvv
-// pwu pwv, the taps in the reference's order (row offset, then column).
-__device__ __forceinline__ void upsample_px(const LevelSol& cs, unsigned v, unsigned u, unsigned R, unsigned C,
-                                            float (&acc)[10])
+// Connectivity weight (computeRij, pdflow_cudalib.cu:725-779) of the step from
+// pixel i to i + d of back-projected coordinate x and depth z.
+__device__ __forceinline__ float rij(const float* __restrict__ x, const float* __restrict__ z, unsigned i, unsigned d)
 {
-    const unsigned Rc = R / 2;
-    const bool inner = (v > 1) && (v < R - 2) && (u > 1) && (u < C - 2);
-#pragma unroll
-    for (int q = 0; q < 10; ++q) acc[q] = 0.f;
-    float acu_weight = 1.f;
-#pragma unroll
-    for (int k = -2; k < 3; k++)
-#pragma unroll
-        for (int l = -2; l < 3; l++) {
-            const int indv = (int)v + k, indu = (int)u + l;
-            const float gm4 = mul(4.f, gmask(k, l));
-            if ((indv < 0) || (indv >= (int)R) || (indu < 0) || (indu >= (int)C)) {
-                acu_weight = sub(acu_weight, mul(0.25f, gm4));
-                continue;
-            }
-            if ((indv & 1) || (indu & 1)) continue;  // zero-inserted tap
-            const unsigned ci = (unsigned)(indv >> 1) + (unsigned)(indu >> 1) * Rc;
-            acc[0] = fm(gm4, mul(2.f, cs.du[ci]), acc[0]);
-            acc[1] = fm(gm4, mul(2.f, cs.dv[ci]), acc[1]);
-            acc[2] = fm(gm4, cs.dw[ci], acc[2]);
-            acc[3] = fm(gm4, cs.pd[ci], acc[3]);
-            acc[4] = fm(gm4, cs.puu[ci], acc[4]);
-            acc[5] = fm(gm4, cs.puv[ci], acc[5]);
-            acc[6] = fm(gm4, cs.pvu[ci], acc[6]);
-            acc[7] = fm(gm4, cs.pvv[ci], acc[7]);
-            acc[8] = fm(gm4, cs.pwu[ci], acc[8]);
-            acc[9] = fm(gm4, cs.pwv[ci], acc[9]);
-        }
-    if (!inner) {
-        const float inv_acu_weight = fdividef(1.f, acu_weight);
-#pragma unroll
-        for (int q = 0; q < 10; ++q) acc[q] = mul(acc[q], inv_acu_weight);
-    }
+    return rfac(sub(x[i + d], x[i]), sub(z[i + d], z[i]));
 }
 
-// assignZeros (pdflow_cudalib.cu:439-455) with the upsampled solution acc
-// (du dv dw pd puu puv pvu pvv pwu pwv, zero at the coarsest level), then
-// computeRij (:725-779), at one pixel.
-__device__ __forceinline__ void level_init_store(unsigned index, unsigned v, unsigned u, unsigned R, unsigned C,
-                                                 const PyrLevel& o, const PyrLevel& n, const LevelConsts& L,
-                                                 const State& S, const float (&acc)[10])
+// computeImGradients (pdflow_cudalib.cu:574-627) on the new frame, for every
+// level of a solve in one launch: it needs the pyramid only, so it is off the
+// path from one level's solution to the next level's iterations.  The new
+// frame's weights (ri_2, rj_2) at the pixel, left of and above it are formed
+// here instead of being stored and read back (16 VGA pairs: 0.088 ms for all
+// six levels against 0.117 a launch a level, besides those planes' writes).
+struct GradLevels {
+    PyrLevel n[8];
+    unsigned R[8], C[8], first_block[9];   // 256 pixels a block
+    size_t aux[8];                         // the level's floats in the aux planes
+    unsigned count;
+};
+__global__ void k_im_gradients(const __grid_constant__ GradLevels lv, LevelConsts L, size_t pstride,
+                               const unsigned* __restrict__ map)
 {
-    L.du_prev[index] = acc[0];
-    L.dv_prev[index] = acc[1];
-    S.du[index] = 0.f;
-    S.dv[index] = 0.f;
-    S.dw[index] = acc[2];
-    S.dua[index] = 0.f;
-    S.dva[index] = 0.f;
-    S.dwa[index] = acc[2];
-    S.pd[index] = acc[3];
-    S.puu[index] = acc[4];
-    S.puv[index] = acc[5];
-    S.pvu[index] = acc[6];
-    S.pvv[index] = acc[7];
-    S.pwu[index] = acc[8];
-    S.pwv[index] = acc[9];
-
-    // computeRij
-    float dxu = 0.f, dzu = 0.f, dxu_2 = 0.f, dzu_2 = 0.f, dyv = 0.f, dzv = 0.f, dyv_2 = 0.f, dzv_2 = 0.f;
-    if (u != C - 1) {
-        dxu = sub(o.xx[index + R], o.xx[index]);
-        dzu = sub(o.dep[index + R], o.dep[index]);
-        dxu_2 = sub(n.xx[index + R], n.xx[index]);
-        dzu_2 = sub(n.dep[index + R], n.dep[index]);
-    }
-    if (v != R - 1) {
-        dyv = sub(o.yy[index + 1], o.yy[index]);
-        dzv = sub(o.dep[index + 1], o.dep[index]);
-        dyv_2 = sub(n.yy[index + 1], n.yy[index]);
-        dzv_2 = sub(n.dep[index + 1], n.dep[index]);
-    }
-    L.ri[index] = rfac(dxu, dzu);
-    L.rj[index] = rfac(dyv, dzv);
-    L.ri2[index] = rfac(dxu_2, dzu_2);
-    L.rj2[index] = rfac(dyv_2, dzv_2);
-}
-
-// Level set-up, one pixel per thread: the coarsest level (zeros), a warm
-// start's seed (its flow, duals from zero), or the upsampled coarse solution.
-__global__ void k_level_init(LevelGeom g, bool first, LevelSol cs, PyrLevel o, PyrLevel n, LevelConsts L, State S,
-                             const float* __restrict__ seed)
-{
-    const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
-    cs = at(cs, po);
-    o = at(o, po);
-    n = at(n, po);
+    unsigned q = 0;
+    while (q + 1 < lv.count && blockIdx.x >= lv.first_block[q + 1]) ++q;
+    const size_t po = pair_off(map, pstride, blockIdx.y);
+    const PyrLevel n = at(lv.n[q], po);
     L = at(L, po);
-    S = at(S, po);
-    const unsigned index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= g.N) return;
-    const unsigned R = g.R, C = g.C;
+    const unsigned index = (blockIdx.x - lv.first_block[q]) * blockDim.x + threadIdx.x;
+    const unsigned R = lv.R[q], C = lv.C[q];
+    if (index >= R * C) return;
     const unsigned v = index % R, u = index / R;
-    float acc[10] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (seed) {   // warm start: a predicted solution of this level, duals from zero
-        const float* sp = seed + (size_t)blockIdx.y * 3 * g.N;
-        acc[0] = sp[index];
-        acc[1] = sp[g.N + index];
-        acc[2] = sp[2 * g.N + index];
-    } else if (!first) {
-        upsample_px(cs, v, u, R, C, acc);
-    }
-    level_init_store(index, v, u, R, C, o, n, L, S, acc);
-}
-
-// Level set-up with the upsampled coarse solution, one vertical pixel pair
-// (rows 2a, 2a+1 of column u) per thread.  In a pair whose pixels are both
-// inner, the even row's taps with a coarse sample are rows -2, 0, +2 and the
-// odd row's -1, +1, and the column's parity fixes the columns (-2, 0, +2 or
-// -1, +1): both pixels read the same 3 x 3 (or 3 x 2) coarse neighbourhood,
-// loaded once per plane, and accumulate their taps in the reference's order.
-// Border pairs take the per-pixel gather.  Same bits as k_level_init.
-__global__ void k_level_init_pairs(LevelGeom g, LevelSol cs, PyrLevel o, PyrLevel n, LevelConsts L, State S)
-{
-    const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
-    cs = at(cs, po);
-    o = at(o, po);
-    n = at(n, po);
-    L = at(L, po);
-    S = at(S, po);
-    const unsigned R = g.R, C = g.C, Rc = R / 2;
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= Rc * C) return;
-    const unsigned a = t % Rc, u = t / Rc, v0 = 2 * a, index0 = v0 + u * R;
-    float acc0[10], acc1[10];
-    if (a >= 1 && v0 + 3 < R && u > 1 && u + 2 < C) {
-        const unsigned b = u >> 1;
-        const float* planes[10] = {cs.du, cs.dv, cs.dw, cs.pd, cs.puu, cs.puv, cs.pvu, cs.pvv, cs.pwu, cs.pwv};
-        if ((u & 1u) == 0) {   // column taps -2, 0, +2: coarse columns b-1, b, b+1
-#pragma unroll
-            for (int q = 0; q < 10; ++q) {
-                float c[3][3];
-#pragma unroll
-                for (int r = 0; r < 3; ++r)
-#pragma unroll
-                    for (int e = 0; e < 3; ++e) {
-                        const float x = planes[q][(a - 1 + r) + (b - 1 + e) * Rc];
-                        c[r][e] = q < 2 ? mul(2.f, x) : x;
-                    }
-                float x0 = 0.f, x1 = 0.f;
-#pragma unroll
-                for (int r = 0; r < 3; ++r)   // even row: row taps -2, 0, +2 = coarse rows a-1, a, a+1
-#pragma unroll
-                    for (int e = 0; e < 3; ++e) x0 = fm(mul(4.f, gmask(2 * r - 2, 2 * e - 2)), c[r][e], x0);
-#pragma unroll
-                for (int r = 1; r < 3; ++r)   // odd row: row taps -1, +1 = coarse rows a, a+1
-#pragma unroll
-                    for (int e = 0; e < 3; ++e) x1 = fm(mul(4.f, gmask(2 * r - 3, 2 * e - 2)), c[r][e], x1);
-                acc0[q] = x0;
-                acc1[q] = x1;
-            }
-        } else {   // column taps -1, +1: coarse columns b, b+1
-#pragma unroll
-            for (int q = 0; q < 10; ++q) {
-                float c[3][2];
-#pragma unroll
-                for (int r = 0; r < 3; ++r)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float x = planes[q][(a - 1 + r) + (b + e) * Rc];
-                        c[r][e] = q < 2 ? mul(2.f, x) : x;
-                    }
-                float x0 = 0.f, x1 = 0.f;
-#pragma unroll
-                for (int r = 0; r < 3; ++r)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) x0 = fm(mul(4.f, gmask(2 * r - 2, 2 * e - 1)), c[r][e], x0);
-#pragma unroll
-                for (int r = 1; r < 3; ++r)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) x1 = fm(mul(4.f, gmask(2 * r - 3, 2 * e - 1)), c[r][e], x1);
-                acc0[q] = x0;
-                acc1[q] = x1;
-            }
-        }
-    } else {
-        upsample_px(cs, v0, u, R, C, acc0);
-        upsample_px(cs, v0 + 1, u, R, C, acc1);
-    }
-    level_init_store(index0, v0, u, R, C, o, n, L, S, acc0);
-    level_init_store(index0 + 1, v0 + 1, u, R, C, o, n, L, S, acc1);
-}
-
-// computeImGradients (pdflow_cudalib.cu:574-627) on the new frame.
-__global__ void k_im_gradients(LevelGeom g, PyrLevel n, LevelConsts L)
-{
-    const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
-    n = at(n, po);
-    L = at(L, po);
-    const unsigned index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= g.N) return;
-    const unsigned R = g.R, C = g.C;
-    const unsigned v = index % R, u = index / R;
+    const size_t out = lv.aux[q] + index;
     const float* __restrict__ c = n.col;
     const float* __restrict__ d = n.dep;
-    const float* __restrict__ ri2 = L.ri2;
-    const float* __restrict__ rj2 = L.rj2;
     if (u == 0) {
-        L.dcu_aux[index] = sub(c[index + R], c[index]);
-        L.ddu_aux[index] = sub(d[index + R], d[index]);
+        L.dcu_aux[out] = sub(c[index + R], c[index]);
+        L.ddu_aux[out] = sub(d[index + R], d[index]);
     } else if (u == C - 1) {
-        L.dcu_aux[index] = sub(c[index], c[index - R]);
-        L.ddu_aux[index] = sub(d[index], d[index - R]);
+        L.dcu_aux[out] = sub(c[index], c[index - R]);
+        L.ddu_aux[out] = sub(d[index], d[index - R]);
     } else {
-        L.dcu_aux[index] = wgrad(ri2[index], ri2[index - R], c[index + R], c[index], c[index - R]);
-        L.ddu_aux[index] = (d[index] > 0.f) ? wgrad(ri2[index], ri2[index - R], d[index + R], d[index], d[index - R])
-                                            : 0.f;
+        const float r = rij(n.xx, d, index, R), rm = rij(n.xx, d, index - R, R);
+        L.dcu_aux[out] = wgrad(r, rm, c[index + R], c[index], c[index - R]);
+        L.ddu_aux[out] = (d[index] > 0.f) ? wgrad(r, rm, d[index + R], d[index], d[index - R]) : 0.f;
     }
     if (v == 0) {
-        L.dcv_aux[index] = sub(c[index + 1], c[index]);
-        L.ddv_aux[index] = sub(d[index + 1], d[index]);
+        L.dcv_aux[out] = sub(c[index + 1], c[index]);
+        L.ddv_aux[out] = sub(d[index + 1], d[index]);
     } else if (v == R - 1) {
-        L.dcv_aux[index] = sub(c[index], c[index - 1]);
-        L.ddv_aux[index] = sub(d[index], d[index - 1]);
+        L.dcv_aux[out] = sub(c[index], c[index - 1]);
+        L.ddv_aux[out] = sub(d[index], d[index - 1]);
     } else {
-        L.dcv_aux[index] = wgrad(rj2[index], rj2[index - 1], c[index + 1], c[index], c[index - 1]);
-        L.ddv_aux[index] = (d[index] > 0.f) ? wgrad(rj2[index], rj2[index - 1], d[index + 1], d[index], d[index - 1])
-                                            : 0.f;
+        const float r = rij(n.yy, d, index, 1), rm = rij(n.yy, d, index - 1, 1);
+        L.dcv_aux[out] = wgrad(r, rm, c[index + 1], c[index], c[index - 1]);
+        L.ddv_aux[out] = (d[index] > 0.f) ? wgrad(r, rm, d[index + 1], d[index], d[index - 1]) : 0.f;
     }
 }
 
-// performWarping (pdflow_cudalib.cu:629-652) + computeMu/computeStepSizes (:781-808).
-// steps = false: only mu of the step fields (the tile kernels recompute the
-// step sizes from mu, ri, rj, ddu, ddv in registers); the free spd plane then
-// holds powf(ddt, 2) for the level's median, so each pixel's square is taken
-// once instead of once per neighbour.
-__global__ void k_warp_steps(LevelGeom g, PyrLevel o, PyrLevel n, LevelConsts L, Params p, int steps)
+// performWarping (pdflow_cudalib.cu:629-652) at one pixel: both frames at (u +
+// du, v + dv); aux: the level's offset in the gradient planes.
+struct Warped {
+    float dct, dcu, dcv, ddt, ddu, ddv;
+};
+__device__ __forceinline__ Warped warp_px(const PyrLevel& o, const PyrLevel& n, const LevelConsts& L, size_t aux,
+                                          unsigned R, unsigned C, unsigned v, unsigned u, float du, float dv)
+{
+    const unsigned index = v + u * R;
+    // the five plain interpolations at one position share their case analysis
+    const Bilin b = bilin(R, C, add(float(u), du), add(float(v), dv));
+    const float* const mats[5] = {n.col, L.dcu_aux + aux, L.dcv_aux + aux, L.ddu_aux + aux, L.ddv_aux + aux};
+    float w5[5];
+    bilin_blend_n<5>(mats, R, b, w5);
+    const float wz = interp_depth_at(n.dep, R, b);
+    return {sub(w5[0], o.col[index]), w5[1], w5[2], (wz > 0.f) ? sub(wz, o.dep[index]) : 0.f, w5[3], w5[4]};
+}
+
+// upsampleCopy + upsampleFilterPrevSolution (pdflow_cudalib.cu:460-569) of one
+// coarse plane at a vertical pixel pair (rows 2a, 2a+1 of column u), as a
+// gather over the coarse solution (the zero-inserted taps contribute exactly
+// zero and are skipped): the even row's taps with a coarse sample are rows -2,
+// 0, +2 and the odd row's -1, +1, and the column's parity fixes the columns
+// (-2, 0, +2 or -1, +1), so both pixels read the same 3 x 3 (or 3 x 2) coarse
+// neighbourhood and accumulate their taps in the reference's order (row, then
+// column).  Bit r * 3 + e of `in`: the sample lies inside the level.
+template <int kColTaps>
+__device__ __forceinline__ float2 upsample_pair(const float* __restrict__ plane, const int (&at)[9], unsigned in,
+                                                float scale)
+{
+    float c[3][kColTaps];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int e = 0; e < kColTaps; ++e) c[r][e] = (in >> (r * 3 + e)) & 1u ? mul(scale, plane[at[r * 3 + e]]) : 0.f;
+    constexpr int l0 = kColTaps == 3 ? -2 : -1;
+    float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)   // even row: row taps -2, 0, +2 = coarse rows a-1, a, a+1
+#pragma unroll
+        for (int e = 0; e < kColTaps; ++e)
+            if ((in >> (r * 3 + e)) & 1u) x0 = fm(mul(4.f, gmask(2 * r - 2, 2 * e + l0)), c[r][e], x0);
+#pragma unroll
+    for (int r = 1; r < 3; ++r)   // odd row: row taps -1, +1 = coarse rows a, a+1
+#pragma unroll
+        for (int e = 0; e < kColTaps; ++e)
+            if ((in >> (r * 3 + e)) & 1u) x1 = fm(mul(4.f, gmask(2 * r - 3, 2 * e + l0)), c[r][e], x1);
+    return make_float2(x0, x1);
+}
+
+// The mask's weight inside the image along one axis, in sixteenths: 16 less
+// the taps of pixel x beyond [0, n).
+__device__ __forceinline__ int mask_inside(int x, int n)
+{
+    return 16 - (x < 1 ? 5 : x < 2 ? 1 : 0) - (x > n - 2 ? 5 : x > n - 3 ? 1 : 0);
+}
+
+// A level's starting point: assignZeros / the upsampled solution
+// (pdflow_cudalib.cu:439-569) and computeRij of the old frame (:725-779).  kPx
+// pixels of a column per thread (2: rows 2a, 2a+1, stored as float2; 1: the
+// coarsest level, whose rows are odd).
+// start 0: zeros; 1: a predicted flow, duals from zero; 2: the coarse solution.
+// Bound by instruction issue on a batch, by latency on one pair's small levels.
+// One kernel with the warp below (the flow and weights in registers between
+// them) needs 95 registers a thread and 0.57 ms for 16 pairs at 480x640 where
+// the two take 0.33, and gains nothing on the small levels.
+template <int kPx>
+__global__ void __launch_bounds__(kBlock) k_level_start(LevelGeom g, int start, LevelSol cs, PyrLevel o,
+                                                        LevelConsts L, State S, const float* __restrict__ seed)
+{
+    const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
+    cs = at(cs, po);
+    o = at(o, po);
+    L = at(L, po);
+    S = at(S, po);
+    const unsigned R = g.R, C = g.C, rows = R / kPx;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= rows * C) return;
+    const unsigned a = t % rows, u = t / rows, v0 = kPx * a, index = v0 + u * R;
+    auto put = [&](float* plane, float2 x) {
+        if constexpr (kPx == 2) *reinterpret_cast<float2*>(plane + index) = x;
+        else plane[index] = x.x;
+    };
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 du = zero, dv = zero, dw = zero;
+    float* const duals[7] = {S.pd, S.puu, S.puv, S.pvu, S.pvv, S.pwu, S.pwv};
+    if (kPx == 2 && start == 2) {
+        const int Rc = int(R / 2), Cc = int(C / 2), b = int(u >> 1), ca = int(a);
+        const bool odd = u & 1u;
+        int from[9];
+        unsigned in = 0;
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                const int row = ca - 1 + r, col = odd ? b + e : b - 1 + e;
+                from[r * 3 + e] = row + col * Rc;
+                if (row >= 0 && row < Rc && col >= 0 && col < Cc) in |= 1u << (r * 3 + e);
+            }
+        // beyond the image's inner part the sum is divided by the mask's weight
+        // inside the image, a multiple of 1/256 (elsewhere the factor is 1)
+        const int wu = mask_inside(int(u), int(C));
+        const float i0 = fdividef(1.f, float(mask_inside(int(v0), int(R)) * wu) / 256.f);
+        const float i1 = fdividef(1.f, float(mask_inside(int(v0) + 1, int(R)) * wu) / 256.f);
+        const bool inner = v0 > 1 && v0 + 1 < R - 2 && u > 1 && u < C - 2;
+        auto up = [&](const float* plane, float scale) {
+            float2 x = odd ? upsample_pair<2>(plane, from, in, scale) : upsample_pair<3>(plane, from, in, scale);
+            if (!inner) x = make_float2(mul(x.x, i0), mul(x.y, i1));
+            return x;
+        };
+        du = up(cs.du, 2.f);
+        dv = up(cs.dv, 2.f);
+        dw = up(cs.dw, 1.f);
+        const float* const coarse[7] = {cs.pd, cs.puu, cs.puv, cs.pvu, cs.pvv, cs.pwu, cs.pwv};
+#pragma unroll
+        for (int q = 0; q < 7; ++q) put(duals[q], up(coarse[q], 1.f));
+    } else {
+        if (start == 1) {
+            const float* sp = seed + (size_t)blockIdx.y * 3 * g.N + index;
+            du = make_float2(sp[0], kPx == 2 ? sp[1] : 0.f);
+            dv = make_float2(sp[g.N], kPx == 2 ? sp[g.N + 1] : 0.f);
+            dw = make_float2(sp[2 * g.N], kPx == 2 ? sp[2 * g.N + 1] : 0.f);
+        }
+#pragma unroll
+        for (int q = 0; q < 7; ++q) put(duals[q], zero);
+    }
+    put(L.du_prev, du);
+    put(L.dv_prev, dv);
+    put(S.du, zero);
+    put(S.dv, zero);
+    put(S.dua, zero);
+    put(S.dva, zero);
+    put(S.dw, dw);
+    put(S.dwa, dw);
+    float2 ri = make_float2(1.f, 1.f), rj = make_float2(1.f, 1.f);   // rfac(0, 0) at the far borders
+    if (u != C - 1) {
+        ri.x = rij(o.xx, o.dep, index, R);
+        if (kPx == 2) ri.y = rij(o.xx, o.dep, index + 1, R);
+    }
+    if (v0 != R - 1) rj.x = rij(o.yy, o.dep, index, 1);
+    if (kPx == 2 && v0 + 1 != R - 1) rj.y = rij(o.yy, o.dep, index + 1, 1);
+    put(L.ri, ri);
+    put(L.rj, rj);
+}
+
+// performWarping (pdflow_cudalib.cu:629-652) + computeMu/computeStepSizes
+// (:781-808), from the planes k_level_start wrote.  steps: which step-size
+// planes to write (kStepsNone: only mu, the tile kernels recompute the step
+// sizes from mu, ri, rj, ddu, ddv; there and beside the quad products the free
+// spd plane holds powf(ddt, 2) for the level's median, so each pixel's square is
+// taken once instead of once per neighbour).
+__global__ void __launch_bounds__(kBlock) k_level_warp(LevelGeom g, PyrLevel o, PyrLevel n, LevelConsts L, Params p,
+                                                       int steps, size_t aux)
 {
     const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
     o = at(o, po);
@@ -420,32 +397,22 @@ __global__ void k_warp_steps(LevelGeom g, PyrLevel o, PyrLevel n, LevelConsts L,
     if (index >= g.N) return;
     const unsigned R = g.R, C = g.C;
     const unsigned v = index % R, u = index / R;
-    const float ind_uf = add(float(u), L.du_prev[index]);
-    const float ind_vf = add(float(v), L.dv_prev[index]);
-    // the five plain interpolations at one position share their case analysis
-    const Bilin b = bilin(R, C, ind_uf, ind_vf);
-    const float* const mats[5] = {n.col, L.dcu_aux, L.dcv_aux, L.ddu_aux, L.ddv_aux};
-    float w5[5];
-    bilin_blend_n<5>(mats, R, b, w5);
-    const float dct = sub(w5[0], o.col[index]);
-    const float dcu = w5[1], dcv = w5[2], ddu = w5[3], ddv = w5[4];
-    const float wz = interp_depth_at(n.dep, R, b);
-    const float ddt = (wz > 0.f) ? sub(wz, o.dep[index]) : 0.f;
-    L.dct[index] = dct;
-    L.dcu[index] = dcu;
-    L.dcv[index] = dcv;
-    L.ddt[index] = ddt;
-    L.ddu[index] = ddu;
-    L.ddv[index] = ddv;
+    const Warped w = warp_px(o, n, L, aux, R, C, v, u, L.du_prev[index], L.dv_prev[index]);
+    L.dct[index] = w.dct;
+    L.dcu[index] = w.dcu;
+    L.dcv[index] = w.dcv;
+    L.ddt[index] = w.ddt;
+    L.ddu[index] = w.ddu;
+    L.ddv[index] = w.ddv;
+    if (steps == kStepsNone || steps == kStepsQuads) L.spd[index] = powf(w.ddt, 2.f);   // the median's weight
     if (steps == kStepsNone) {
-        L.mu[index] = data_weight(p.mu, ddu, ddv, ddt);
-        L.spd[index] = powf(ddt, 2.f);
+        L.mu[index] = data_weight(p.mu, w.ddu, w.ddv, w.ddt);
         return;
     }
     const float ri = L.ri[index], rj = L.rj[index];
     const float ri_m = (u > 0) ? L.ri[index - R] : 0.f;
     const float rj_m = (v > 0) ? L.rj[index - 1] : 0.f;
-    const Steps s = mu_and_steps(p.mu, p.lambda_i, p.lambda_d, ddu, ddv, ddt, ri, rj, ri_m, rj_m, u > 0, v > 0);
+    const Steps s = mu_and_steps(p.mu, p.lambda_i, p.lambda_d, w.ddu, w.ddv, w.ddt, ri, rj, ri_m, rj_m, u > 0, v > 0);
     L.mu[index] = s.mu;
     if (steps == kStepsRaw || steps == kStepsAll) {
         L.spd[index] = s.spd;
@@ -456,8 +423,6 @@ __global__ void k_warp_steps(LevelGeom g, PyrLevel o, PyrLevel n, LevelConsts L,
         L.tu[index] = s.tu;
         L.tv[index] = s.tv;
         L.tw[index] = s.tw;
-    } else {
-        L.spd[index] = powf(ddt, 2.f);   // the median's depth-change weight
     }
     if (steps == kStepsQuads || steps == kStepsAll) {
         // the products the dual update forms (dual_update: mul(spd, mu), mul(spuvx, li), ...)
@@ -470,6 +435,17 @@ __global__ void k_warp_steps(LevelGeom g, PyrLevel o, PyrLevel n, LevelConsts L,
         L.qs[6][index] = s.tv;
         L.qs[7][index] = s.tw;
     }
+}
+
+// The new frame's weights as planes (the stage dump: the solve forms them
+// where it needs them).
+__global__ void k_rij2(LevelGeom g, PyrLevel n, LevelConsts L)
+{
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= g.N) return;
+    const unsigned v = i % g.R, u = i / g.R;
+    L.ri2[i] = u != g.C - 1 ? rij(n.xx, n.dep, i, g.R) : 1.f;
+    L.rj2[i] = v != g.R - 1 ? rij(n.yy, n.dep, i, 1) : 1.f;
 }
 
 // ---------------------------------------------------------------------------
@@ -787,14 +763,18 @@ __global__ void k_pyr_copy(PyrLevel src, PyrLevel dst, unsigned n, size_t pstrid
     }
 }
 
-// The warp point of the energy: the solution's total image-plane flow.
-__global__ void k_energy_prep(LevelGeom g, LevelSol sol, LevelConsts L)
+// Both frames at the solution's total image-plane flow, for the energy.
+__global__ void k_energy_warp(LevelGeom g, LevelSol sol, PyrLevel o, PyrLevel n, LevelConsts L, Params p, size_t aux)
 {
     const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.N) return;
-    at(L.du_prev, po)[i] = at(sol.du, po)[i];
-    at(L.dv_prev, po)[i] = at(sol.dv, po)[i];
+    L = at(L, po);
+    const Warped w = warp_px(at(o, po), at(n, po), L, aux, g.R, g.C, i % g.R, i / g.R, at(sol.du, po)[i],
+                             at(sol.dv, po)[i]);
+    L.dct[i] = w.dct;
+    L.ddt[i] = w.ddt;
+    L.mu[i] = data_weight(p.mu, w.ddu, w.ddv, w.ddt);
 }
 
 // 1024 accumulators per pair: accumulator t sums pixels t, t + 1024, ... in
@@ -886,26 +866,44 @@ cudaError_t launch_pyr_copy(PyrLevel src, PyrLevel dst, unsigned n, unsigned pai
 
 static dim3 level_grid(const LevelGeom& g) { return dim3(blocks_for(g.N), g.pairs); }
 
-cudaError_t launch_level_init(LevelGeom g, bool first, LevelSol coarse, PyrLevel old_l, PyrLevel new_l,
-                              LevelConsts L, State S, cudaStream_t st, const float* seed)
+cudaError_t launch_im_gradients(const LevelGeom* levels, const PyrLevel* images, const size_t* aux, unsigned count,
+                                LevelConsts L, cudaStream_t st)
 {
-    if (!first && !seed && g.R % 2 == 0)
-        k_level_init_pairs<<<dim3(blocks_for(g.N / 2), g.pairs), kBlock, 0, st>>>(g, coarse, old_l, new_l, L, S);
+    if (count == 0 || count > 8) return cudaErrorInvalidValue;
+    GradLevels lv{};
+    lv.count = count;
+    for (unsigned q = 0; q < count; ++q) {
+        lv.n[q] = images[q];
+        lv.R[q] = levels[q].R;
+        lv.C[q] = levels[q].C;
+        lv.aux[q] = aux[q];
+        lv.first_block[q + 1] = lv.first_block[q] + blocks_for(levels[q].N);
+    }
+    k_im_gradients<<<dim3(lv.first_block[count], levels[0].pairs), kBlock, 0, st>>>(lv, L, levels[0].pstride,
+                                                                                  levels[0].map);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_level_setup(LevelGeom g, LevelStart start, LevelSol coarse, PyrLevel old_l, PyrLevel new_l,
+                               LevelConsts L, State S, Params p, int steps, size_t aux, cudaStream_t st,
+                               const float* seed)
+{
+    if (g.R % 2 == 0)
+        k_level_start<2><<<dim3(blocks_for(g.N / 2), g.pairs), kBlock, 0, st>>>(g, int(start), coarse, old_l, L, S,
+                                                                               seed);
+    else if (start == LevelStart::Coarse)
+        return cudaErrorInvalidValue;   // a level above another has even rows
     else
-        k_level_init<<<level_grid(g), kBlock, 0, st>>>(g, first, coarse, old_l, new_l, L, S, seed);
+        k_level_start<1><<<level_grid(g), kBlock, 0, st>>>(g, int(start), coarse, old_l, L, S, seed);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_level_warp<<<level_grid(g), kBlock, 0, st>>>(g, old_l, new_l, L, p, steps, aux);
     return cudaGetLastError();
 }
 
-cudaError_t launch_im_gradients(LevelGeom g, PyrLevel new_l, LevelConsts L, cudaStream_t st)
+cudaError_t launch_rij2(LevelGeom g, PyrLevel new_l, LevelConsts L, cudaStream_t st)
 {
-    k_im_gradients<<<level_grid(g), kBlock, 0, st>>>(g, new_l, L);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_warp_steps(LevelGeom g, PyrLevel old_l, PyrLevel new_l, LevelConsts L, Params p, cudaStream_t st,
-                              int steps)
-{
-    k_warp_steps<<<level_grid(g), kBlock, 0, st>>>(g, old_l, new_l, L, p, steps);
+    k_rij2<<<level_grid(g), kBlock, 0, st>>>(g, new_l, L);
     return cudaGetLastError();
 }
 
@@ -948,9 +946,10 @@ cudaError_t launch_median(LevelGeom g, bool finest, PyrLevel old_l, LevelConsts 
     return cudaGetLastError();
 }
 
-cudaError_t launch_energy_prep(LevelGeom g, LevelSol sol, LevelConsts L, cudaStream_t st)
+cudaError_t launch_energy_warp(LevelGeom g, LevelSol sol, PyrLevel old_l, PyrLevel new_l, LevelConsts L, Params p,
+                               size_t aux, cudaStream_t st)
 {
-    k_energy_prep<<<level_grid(g), kBlock, 0, st>>>(g, sol, L);
+    k_energy_warp<<<level_grid(g), kBlock, 0, st>>>(g, sol, old_l, new_l, L, p, aux);
     return cudaGetLastError();
 }
 

@@ -25,7 +25,7 @@ struct LevelConsts {
     float* qs[8];
 };
 
-// Which step-size planes the warping kernel writes (launch_warp_steps).
+// Which step-size planes the level set-up writes (launch_level_setup).
 enum StepPlanes : int {
     kStepsNone = 0,     // mu, and powf(ddt, 2) in spd for the median (tile levels that recompute their steps)
     kStepsRaw = 1,      // mu and the eight raw step-size planes (spd .. tw)
@@ -133,22 +133,30 @@ cudaError_t launch_pyr_down(PyrLevel prev, unsigned R, unsigned C, PyrLevel out,
 // Copies the planes of `src` over `dst` for the mapped slots (frame t becomes t-1).
 cudaError_t launch_pyr_copy(PyrLevel src, PyrLevel dst, unsigned n, unsigned pairs, size_t pstride,
                             const unsigned* map, cudaStream_t st);
+// The new frame's weighted image gradients of `count` levels of the same pairs
+// (levels[q]'s geometry and pyramid image), into the aux planes at float aux[q].
+cudaError_t launch_im_gradients(const LevelGeom* levels, const PyrLevel* images, const size_t* aux, unsigned count,
+                                LevelConsts L, cudaStream_t st);
+// Everything between the coarse solution and the level's iterations: the
+// starting flow and duals, the old frame's weights, the warp (gradients at float
+// `aux` of the aux planes) and the step-size planes `steps` (StepPlanes).  Seed:
 // `seed` (device, [pairs][3][N]: du, dv, dw in this level's pixels / metres)
-// replaces the upsampled coarser solution; the duals then start at zero.
-cudaError_t launch_level_init(LevelGeom g, bool first, LevelSol coarse, PyrLevel old_l, PyrLevel new_l,
-                              LevelConsts L, State S, cudaStream_t st, const float* seed = nullptr);
+// replaces the upsampled solution and the duals start at zero.
+enum class LevelStart : int { Zeros = 0, Seed = 1, Coarse = 2 };
+cudaError_t launch_level_setup(LevelGeom g, LevelStart start, LevelSol coarse, PyrLevel old_l, PyrLevel new_l,
+                               LevelConsts L, State S, Params p, int steps, size_t aux, cudaStream_t st,
+                               const float* seed = nullptr);
+// The new frame's weights as planes ri2, rj2 (the stage dump).
+cudaError_t launch_rij2(LevelGeom g, PyrLevel new_l, LevelConsts L, cudaStream_t st);
 // Energy of the level's solution `sol` (total du, dv in pixels, dw in metres),
-// for the warp point set by launch_energy_prep + gradients + warping:
-// sum over pixels of |dct| + mu |ddt - dw| + lambda_i (|r grad du| + |r grad dv|)
-// + lambda_d |r grad dw|; energies[y] for grid index y.
-cudaError_t launch_energy_prep(LevelGeom g, LevelSol sol, LevelConsts L, cudaStream_t st);
+// at the warp point set by launch_im_gradients + launch_energy_warp (which
+// overwrite dct, ddt and mu): sum over pixels of |dct| + mu |ddt - dw| + lambda_i
+// (|r grad du| + |r grad dv|) + lambda_d |r grad dw|; energies[y] for grid index y.
+cudaError_t launch_energy_warp(LevelGeom g, LevelSol sol, PyrLevel old_l, PyrLevel new_l, LevelConsts L, Params p,
+                               size_t aux, cudaStream_t st);
 // part: device scratch of 1024 doubles per pair.
 cudaError_t launch_energy(LevelGeom g, LevelSol sol, LevelConsts L, Params p, float* energies, double* part,
                           cudaStream_t st);
-cudaError_t launch_im_gradients(LevelGeom g, PyrLevel new_l, LevelConsts L, cudaStream_t st);
-// steps: which step-size planes to write (StepPlanes).
-cudaError_t launch_warp_steps(LevelGeom g, PyrLevel old_l, PyrLevel new_l, LevelConsts L, Params p,
-                              cudaStream_t st, int steps = kStepsRaw);
 cudaError_t launch_dual(LevelGeom g, LevelConsts L, State S, Params p, cudaStream_t st);
 cudaError_t launch_primal(LevelGeom g, LevelConsts L, State S, Params p, bool last, const float* depth_old,
                           cudaStream_t st);

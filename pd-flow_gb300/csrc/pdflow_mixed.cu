@@ -178,11 +178,11 @@ int enqueue_mixed(pdflow_solver* s, cudaStream_t st, const std::vector<LaunchRec
         const PyrLevel o = s->pyr[fo][li], n = s->pyr[fn][li];
         cudaError_t e = cudaSuccess;
         if (r.kind == 0) {
-            e = launch_level_init(g, r.step == 0, s->sol, o, n, s->L, s->S, st);
-            if (e == cudaSuccess) e = launch_im_gradients(g, n, s->L, st);
+            const size_t aux = 0;   // one step's gradients at a time: the steps' pairs differ
+            e = launch_im_gradients(&g, &n, &aux, 1, s->L, st);
             if (e == cudaSuccess)
-                e = launch_warp_steps(g, o, n, s->L, p, st,
-                                      all_steps ? kStepsAll : (form >= 7 ? kStepsQuads : kStepsNone));
+                e = launch_level_setup(g, r.step == 0 ? LevelStart::Zeros : LevelStart::Coarse, s->sol, o, n, s->L,
+                                       s->S, p, all_steps ? kStepsAll : (form >= 7 ? kStepsQuads : kStepsNone), aux, st);
             *count += 3;
             cur = s->S;
             nxt = alt;

@@ -121,7 +121,9 @@ void carve_solver(pdflow_solver* s, char* base, size_t* used)
                     &L.qs[3], &L.qs[4], &L.qs[5],   &L.qs[6],  &L.qs[7],  &L.ri2,     &L.rj2,
                     &L.dcu_aux, &L.dcv_aux, &L.ddu_aux, &L.ddv_aux, &L.spd, &L.spuvx, &L.spuvy,
                     &L.spwx, &L.spwy, &L.tu, &L.tv, &L.tw};
-    for (float** p : lp) *p = cv.plane(N);
+    // the gradient planes hold every level of a solve (aux_offset): N + N/4 + ...
+    for (float** p : lp)
+        *p = cv.plane(p == &L.dcu_aux || p == &L.dcv_aux || p == &L.ddu_aux || p == &L.ddv_aux ? N + (N + 2) / 3 : N);
     State& S = s->S;
     float** sp[] = {&S.du, &S.dv, &S.dw, &S.dua, &S.dva, &S.dwa, &S.pd, &S.puu, &S.puv, &S.pvu, &S.pvv, &S.pwu,
                     &S.pwv};
@@ -170,6 +172,13 @@ size_t level_keep_offset(const pdflow_solver* s, unsigned level)
         const LevelGeom g = level_geom(s, k, nullptr);
         off += 6 * size_t(g.N);
     }
+    return off;
+}
+
+size_t aux_offset(const pdflow_solver* s, unsigned level)
+{
+    size_t off = 0;
+    for (unsigned k = s->ctf_levels - 1; k > level; --k) off += level_geom(s, k, nullptr).N;
     return off;
 }
 
@@ -363,11 +372,11 @@ int enqueue_energy(pdflow_solver* s, cudaStream_t st, unsigned pairs, unsigned l
     LevelGeom g = level_geom(s, level, &li, pairs);
     g.map = map;
     const PyrLevel o = s->pyr[s->new_slot ^ 1][li], n = s->pyr[s->new_slot][li];
-    CUDA_TRY(launch_energy_prep(g, s->sol, s->L, st), "energy prep launch");
-    CUDA_TRY(launch_im_gradients(g, n, s->L, st), "image gradients launch");
-    CUDA_TRY(launch_warp_steps(g, o, n, s->L, p, st, false), "warping launch");   // the energy needs mu only
+    const size_t aux = aux_offset(s, level);
+    CUDA_TRY(launch_im_gradients(&g, &n, &aux, 1, s->L, st), "image gradients launch");
+    CUDA_TRY(launch_energy_warp(g, s->sol, o, n, s->L, p, aux, st), "energy warping launch");
     CUDA_TRY(launch_energy(g, s->sol, s->L, p, out, s->energy_part, st), "energy launch");
-    s->launches += 5;
+    s->launches += 4;
     return PDFLOW_OK;
 }
 
@@ -379,6 +388,22 @@ int enqueue_solve(pdflow_solver* s, cudaStream_t st, unsigned pairs, const Solve
     const int fn = s->new_slot, fo = fn ^ 1;
     unsigned count = 0;
     const unsigned last = plan.last < s->ctf_levels ? plan.last : s->ctf_levels - 1;
+    {
+        // the image gradients of every level at once
+        LevelGeom gs[8];
+        PyrLevel images[8];
+        size_t aux[8];
+        unsigned m = 0;
+        for (unsigned i = plan.first; i <= last; ++i, ++m) {
+            unsigned li;
+            gs[m] = level_geom(s, i, &li, pairs);
+            gs[m].map = plan.map;
+            images[m] = s->pyr[fn][li];
+            aux[m] = aux_offset(s, i);
+        }
+        CUDA_TRY(launch_im_gradients(gs, images, aux, m, s->L, st), "image gradients launch");
+        ++count;
+    }
     for (unsigned i = plan.first; i <= last; ++i) {
         unsigned li;
         LevelGeom g = level_geom(s, i, &li, pairs);
@@ -390,12 +415,12 @@ int enqueue_solve(pdflow_solver* s, cudaStream_t st, unsigned pairs, const Solve
         const NvtxRange level_range(kLevelNames[i < 8 ? i : 7]);
         cudaEvent_t* tr = plan.trace ? plan.trace + 3 * (i - plan.first) : nullptr;
         if (tr) CUDA_TRY(cudaEventRecord(tr[0], st), "trace event");
-        CUDA_TRY(launch_level_init(g, i == 0, s->sol, o, n, s->L, s->S, st, seed), "level init launch");
         const unsigned iters = scaled_iters(s->prm.num_max_iter[i], plan.iter_scale);
         const int steps = level_steps(s, g, iters, pairs, i, plan.all_steps);
-        CUDA_TRY(launch_im_gradients(g, n, s->L, st), "image gradients launch");
-        CUDA_TRY(launch_warp_steps(g, o, n, s->L, p, st, steps), "warping launch");
-        count += 3;
+        const LevelStart start = seed ? LevelStart::Seed : (i == 0 ? LevelStart::Zeros : LevelStart::Coarse);
+        CUDA_TRY(launch_level_setup(g, start, s->sol, o, n, s->L, s->S, p, steps, aux_offset(s, i), st, seed),
+                 "level set-up launch");
+        count += 2;
         if (tr) CUDA_TRY(cudaEventRecord(tr[1], st), "trace event");
         State fin;
         int rc = enqueue_iterations(s, st, g, o, iters, pairs, &fin, &count, i);
