@@ -693,14 +693,17 @@ __global__ void __launch_bounds__(kMedRows * kMedCols) k_median(LevelGeom g, boo
     out.du[index] = ru;
     out.dv[index] = rv;
     out.dw[index] = rw;
-    if (!out.pd) return;  // stage form: no duals to carry
-    out.pd[index] = S.pd[index];
-    out.puu[index] = S.puu[index];
-    out.puv[index] = S.puv[index];
-    out.pvu[index] = S.pvu[index];
-    out.pvv[index] = S.pvv[index];
-    out.pwu[index] = S.pwu[index];
-    out.pwv[index] = S.pwv[index];
+    // the duals go on to the next level (14 of the finest level's 27 planes of
+    // traffic would be duals nobody reads; the stage form carries none)
+    if (out.pd && !finest) {
+        out.pd[index] = S.pd[index];
+        out.puu[index] = S.puu[index];
+        out.puv[index] = S.puv[index];
+        out.pvu[index] = S.pvu[index];
+        out.pvv[index] = S.pvv[index];
+        out.pwu[index] = S.pwu[index];
+        out.pwv[index] = S.pwv[index];
+    }
     if (finest) {
         if (depth_old > 0) {
             // the finest level is cols wide (g.C == p.cols), also for a mixed batch's smaller pairs
