@@ -153,5 +153,8 @@ struct TuneCandidate {
 TuneCandidate tune_candidate(int c);
 int check_status(pdflow_solver* s);
 void set_last_error(const char* text);   // the text pdflow_last_error returns on this thread
+// The iteration form a level (of g.pairs pairs) runs in unless one was chosen
+// for it; `resident`: its iterations may run in one launch (form 9).
+int default_level_form(const pdflow_solver* s, const LevelGeom& g, bool resident = true);
 LevelGeom level_geom(const pdflow_solver* s, unsigned i, unsigned* level_image, unsigned pairs = 1);
 }  // namespace pdflow

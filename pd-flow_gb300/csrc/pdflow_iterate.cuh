@@ -84,6 +84,9 @@ struct StripUnits {
     unsigned whole, tier_n[3], tier_p[3];
 };
 StripUnits strip_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid);
+// When a launch of the level's strips ends on `ctas` CTAs at 4 iterations per
+// launch, in regions a CTA (the 24x24 tiles' end is their rounds of CTAs).
+float strips_end(const LevelGeom& g, unsigned ctas);
 inline StreamLayout stream_layout(int form)
 {
     return form == 9 ? StreamLayout::Tiles16 : (form == 10 ? StreamLayout::Strips : StreamLayout::Tiles24);

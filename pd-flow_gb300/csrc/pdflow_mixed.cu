@@ -60,9 +60,7 @@ unsigned step_kk(const pdflow_solver* s, unsigned i, int form)
 int step_form(const pdflow_solver* s, unsigned i, const LevelGeom& g)
 {
     int f = s->mixed_form[i] >= 3 ? s->mixed_form[i] : (s->iter_form >= 3 ? s->iter_form : 5);
-    if (s->mixed_form[i] < 3 && f == 10 &&
-        (g.pairs * ((g.R + 23u) / 24u) < unsigned(s->num_sms) || !stream_eligible(g, s->L, s->S, s->S, 10)))
-        f = g.pairs * ((g.R + 15u) / 16u) * ((g.C + 15u) / 16u) <= unsigned(s->num_sms) ? 9 : 8;
+    if (s->mixed_form[i] < 3 && f == 10) f = default_level_form(s, g, false);
     if (f >= 7 && !stream_eligible(g, s->L, s->S, s->S, f)) f = 5;
     return f;
 }

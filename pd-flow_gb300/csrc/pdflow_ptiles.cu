@@ -480,20 +480,86 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
 
 size_t stream_smem_bytes() { return sizeof(float) * (N_PLANES * kSPlane + kCarryFloats); }
 
-// Strip units: the last grid / 8 strips in 8 pieces (grid / 4 for strips
-// of 16 regions or more), the grid / 8 before them in 4, the grid / 8 before
-// those in 2, the rest whole; no more strips than CTAs: every strip in as
-// many pieces as CTAs allow.  Pieces are at least one restart region's
-// 32 - 2 kk exact columns wide.  Each piece recomputes a left halo, so the
-// tail is kept short: on 64-pair VGA solves (1 280 strips of 23 regions at
-// 480x640, 640 of 12 at 240x320) the last grid / 4, grid / 2 and grid strips
-// in 8, 4 and 2 pieces took 38.06 ms, these tiers 37.3 ms.
-StripUnits strip_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid)
+namespace {
+
+// Regions of a unit's columns [c0, c1) (strip_at, continue_unit).
+unsigned unit_regions(int c0, int c1, int C, int kk)
+{
+    unsigned n = 0;
+    for (int col = c0; col < c1; ++n) {
+        const int ru0 = n ? col : std::max(col - kk, 0);
+        col = std::min(ru0 + kSR >= C ? C : ru0 + kSR - kk, c1);
+    }
+    return n;
+}
+
+// When the last CTA ends, in regions: CTAs take units in order as they finish.
+// CTAs that end at the same time are one entry.  Regions take a little longer or
+// shorter with the data, so a tenth of a last unit is added: short last units
+// even that out.
+class UnitQueue {
+public:
+    explicit UnitQueue(unsigned grid) { at_[0] = {0.f, grid}; }
+    // n strips of m equal pieces each, piece by piece.
+    void add(unsigned n, unsigned m, unsigned C, unsigned kk)
+    {
+        for (unsigned i = 0; i < m && n > 0; ++i)
+            add(n, kUnitStart + float(unit_regions(int(C * i / m), int(C * (i + 1) / m), int(C), int(kk))));
+    }
+    float end() const { return at_[used_ - 1].time + 0.1f * last_; }
+
+private:
+    static constexpr float kUnitStart = 0.15f;   // what starting a unit costs beyond its regions
+    static constexpr int kMost = 64;
+    struct Group {
+        float time;
+        unsigned ctas;
+    };
+    Group at_[kMost];
+    int used_ = 1;
+    float last_ = 0.f;
+    void add(unsigned n, float cost)
+    {
+        last_ = cost;
+        while (n > 0) {
+            const unsigned k = std::min(n, at_[0].ctas);
+            const float time = at_[0].time + cost;
+            n -= k;
+            if ((at_[0].ctas -= k) == 0) {
+                for (int i = 1; i < used_; ++i) at_[i - 1] = at_[i];
+                --used_;
+            }
+            int i = 0;   // the first entry that ends no earlier
+            while (i < used_ && at_[i].time < time - 1e-3f) ++i;
+            if (i < used_ && at_[i].time < time + 1e-3f) {
+                at_[i].ctas += k;
+            } else if (used_ == kMost) {   // never seen: keep the bound, lose the detail
+                at_[used_ - 1].ctas += k;
+                at_[used_ - 1].time = std::max(at_[used_ - 1].time, time);
+            } else {
+                for (int q = used_; q > i; --q) at_[q] = at_[q - 1];
+                at_[i] = {time, k};
+                ++used_;
+            }
+        }
+    }
+};
+
+float units_end(const StripUnits& u, unsigned C, unsigned kk, unsigned grid)
+{
+    UnitQueue q(grid);
+    q.add(u.whole, 1, C, kk);
+    for (int i = 0; i < 3; ++i) q.add(u.tier_n[i], u.tier_p[i], C, kk);
+    return q.end();
+}
+
+StripUnits plan_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid)
 {
     StripUnits su{};
     if (strips_n == 0 || C == 0 || kk == 0 || 2 * kk >= (unsigned)kSR || grid == 0) return su;
     const unsigned most = (C + (kSR - 2 * kk) - 1) / (kSR - 2 * kk);
     const unsigned regions = (C + (kSR - kk) - 1) / (kSR - kk);   // of a whole strip walked with the carry
+    // many strips: whole ones, then the last grid / 8 in 2 pieces, in 4 and in 8
     unsigned left = strips_n;
     const unsigned tn[3] = {grid / 8, grid / 8, regions >= 16 ? grid / 4 : grid / 8}, tp[3] = {2, 4, 8};
     for (int i = 2; i >= 0; --i) {
@@ -507,7 +573,72 @@ StripUnits strip_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid
         left = 0;
     }
     su.whole = left;
+    if (strips_n > 4 * grid) return su;
+    // few strips a CTA: the first n in p1 pieces, the rest in p2 >= p1, of pieces
+    // that waste few regions on restarts, if that ends clearly earlier (differences
+    // below 4 % are within the model's error: 10 VGA pairs at 480x640, 32.9 against
+    // 32.1 regions, took 3.55 against 3.61 ms)
+    float best = units_end(su, C, kk, grid) * 0.96f;
+    unsigned cuts[32], n_cuts = 0, fewest = ~0u, total[33];
+    for (unsigned m = 1; m <= std::min(most, 32u); ++m) {
+        total[m] = 0;
+        for (unsigned i = 0; i < m; ++i)
+            total[m] += unit_regions(int(C * i / m), int(C * (i + 1) / m), int(C), int(kk));
+        fewest = std::min(fewest, total[m]);
+    }
+    for (unsigned m = 1; m <= std::min(most, 32u); ++m)
+        if (total[m] * 8 <= fewest * 9) cuts[n_cuts++] = m;
+    const unsigned step = std::max(1u, strips_n / 32);
+    for (unsigned i = 0; i < n_cuts; ++i)
+        for (unsigned j = i; j < n_cuts; ++j)
+            for (unsigned n = i == j ? strips_n : step; n <= strips_n; n += step) {
+                // no plan ends before its work spread evenly
+                if (float(n * total[cuts[i]] + (strips_n - n) * total[cuts[j]]) >= best * float(grid)) continue;
+                const StripUnits c{0, {n, strips_n - n, 0}, {cuts[i], cuts[j], 1}};
+                const float end = units_end(c, C, kk, grid);
+                if (end < best) {
+                    best = end * 0.999f;
+                    su = c;
+                }
+            }
     return su;
+}
+
+}  // namespace
+
+// Strip units.  Each piece of a strip recomputes a left halo, so many strips
+// (over four a CTA) stay whole but for a short tail: on 64-pair VGA solves (1
+// 280 strips of 23 regions at 480x640, 640 of 12 at 240x320) the last grid /
+// 4, grid / 2 and grid strips in 8, 4 and 2 pieces took 38.06 ms, these tiers
+// 37.3 ms.  With fewer the last round is nearly empty however the tail is cut
+// (24 pairs at 240x320: 240 strips of 12 regions on 152 CTAs end after 24.3
+// regions, the work is 18.9), so the cuts are chosen by when the queue ends:
+// there 200 strips in 3 pieces and 40 in 4 end after 19.8 (85 iterations 2.76 ->
+// 2.26 ms on a GB300; 13 pairs at 480x640 5.10 -> 4.56, 20 pairs 7.47 -> 6.78).
+// The choice is a function of its arguments; the last few are kept.
+StripUnits strip_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid)
+{
+    struct Kept {
+        unsigned key[4];
+        StripUnits units;
+    };
+    thread_local Kept kept[16] = {};
+    thread_local unsigned next = 0;
+    const unsigned key[4] = {strips_n, C, kk, grid};
+    for (const Kept& k : kept)
+        if (std::equal(key, key + 4, k.key)) return k.units;
+    const StripUnits su = plan_units(strips_n, C, kk, grid);
+    Kept& k = kept[next++ % 16u];
+    std::copy(key, key + 4, k.key);
+    k.units = su;
+    return su;
+}
+
+float strips_end(const LevelGeom& g, unsigned ctas)
+{
+    constexpr unsigned kk = 4, rows = kSR - 2 * kk;
+    const unsigned strips_n = g.pairs * ((g.R + rows - 1) / rows);
+    return units_end(strip_units(strips_n, g.C, kk, ctas), g.C, kk, ctas);
 }
 
 // The direct loads and stores move a pixel pair as one float2: even rows and

@@ -218,24 +218,35 @@ static bool level_runs_tiles(const pdflow_solver* s, const LevelGeom& g, unsigne
     return s->iter_form >= 2 && iters > 0 && g.N > 300u;
 }
 
+}  // namespace pdflow
+
+// By default: resident tiles where the level fits a cluster a pair; the deep
+// tiles (form 9: twice the iterations per launch where launches are
+// latency-bound, e.g. a single pair's 120x160) where the 16x16 tiles fit one
+// round of CTAs; else the strips (form 10) or the 24x24 tiles (form 8),
+// whichever end earlier on the SMs (strips need tensor copies).  Measured on
+// either side of that line on a GB300 (100 iterations at 480x640, tiles / strips):
+// 2 pairs 0.981 / 0.928 ms, 6 pairs 2.41 / 2.25, 3 pairs 1.300 / 1.302, 7 pairs 2.71
+// / 2.75.
+int pdflow::default_level_form(const pdflow_solver* s, const LevelGeom& g, bool resident)
+{
+    const unsigned sms = unsigned(s->num_sms);
+    if (resident && resident_eligible(g, s->L, s->S, s->S, sms)) return 9;
+    if (g.pairs * ((g.R + 15u) / 16u) * ((g.C + 15u) / 16u) <= sms) return 9;
+    if (!stream_eligible(g, s->L, s->S, s->S, 10)) return 8;
+    const unsigned tiles = g.pairs * ((g.R + 23u) / 24u) * ((g.C + 23u) / 24u);
+    return strips_end(g, sms) < 0.97f * float((tiles + sms - 1) / sms) ? 10 : 8;
+}
+
+namespace pdflow {
+
 // The level's iteration form: its autotuned or hand-set form, else the
-// handle's.  By default the strips (form 10) run only where the level has a
-// strip (a pair's 24-row band) for every SM; smaller levels run the streamed
-// tiles (form 8), which deal fewer pixels to every SM, and levels whose 16x16
-// tiles all fit in one round of CTAs the deep tiles (form 9: twice the
-// iterations per launch where the launches are latency-bound, as the
-// autotuner finds for a single pair's 60x80 and 120x160 levels).  Levels
-// whose rows are even but not a multiple of 4 (30x40) cannot run the strips'
-// tensor copies and take the same tile rule.
-static int level_form(const pdflow_solver* s, const LevelGeom& g, unsigned pairs, unsigned level)
+// handle's (the default form 10 chooses by the level).
+static int level_form(const pdflow_solver* s, const LevelGeom& g, unsigned level)
 {
     const int forced = level < 8 ? s->level_form[level] : -1;
     if (forced >= 0) return forced;
-    if (s->iter_form == 10 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms))) return 9;
-    if (s->iter_form == 10 && (pairs * ((g.R + 23u) / 24u) < unsigned(s->num_sms) ||
-                               !stream_eligible(g, s->L, s->S, s->S, 10)))
-        return pairs * ((g.R + 15u) / 16u) * ((g.C + 15u) / 16u) <= unsigned(s->num_sms) ? 9 : 8;
-    return s->iter_form;
+    return s->iter_form == 10 ? default_level_form(s, g) : s->iter_form;
 }
 
 // Whether level `level`'s tiles run register-resident (quad tiles, form 7, or
@@ -246,7 +257,7 @@ static bool level_runs_quads(const pdflow_solver* s, const LevelGeom& g, unsigne
                              unsigned level)
 {
     if (!level_runs_tiles(s, g, iters, level)) return false;
-    const int form = level_form(s, g, pairs, level);
+    const int form = level_form(s, g, level);
     return (form >= 7 && form <= 10) && stream_eligible(g, s->L, s->S, s->S, form);
 }
 
@@ -271,7 +282,7 @@ static int enqueue_iterations(pdflow_solver* s, cudaStream_t st, const LevelGeom
     const int forced = level < 8 ? s->level_form[level] : -1;
     const bool one_launch_ok = (pairs == 1 || pl.mode != kIterGrid) && pl.smem_bytes <= iterate_smem_limit();
     const bool tiles = level_runs_tiles(s, g, iters, level);
-    const int form = level_form(s, g, pairs, level);
+    const int form = level_form(s, g, level);
     const bool one_launch = forced >= 0 ? (forced == 1 && iters > 0 && one_launch_ok)
                                         : (s->iter_form >= 1 && iters > 0 && !tiles && one_launch_ok);
     const bool quads = tiles && level_runs_quads(s, g, iters, pairs, level);
