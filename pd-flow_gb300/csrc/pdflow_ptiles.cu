@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
         };
         auto iterate = [&](auto border) {
             for (unsigned j = 0; j < a.kk; ++j) {
-                iterate_pair<decltype(border)::value, kSR / 2>(
+                iterate_pair<decltype(border)::value, kSR / 2, kStrips>(
                     s, k, d, sm + X_U * kSPlane, sm + Y_U * kSPlane, kSPlane, me, right, place, a.p.lambda_i,
                     a.p.lambda_d, Hooks{yl + (int)j * yl_j, yl_k, yc + (int)j * (3 * kSR), to_carry});
                 if (kStrips && j + 1 == a.kk) finish();

@@ -27,12 +27,14 @@ __device__ __forceinline__ float clamp1(float pd) { return (fabsf(pd) > 1.f) ? (
 
 // The three TV duals' projections onto the unit disc (updateDualVariables,
 // pdflow_cudalib.cu:813-887) for both pixels of a pair, with disc_factor's
-// expressions in packed FP32x2.  A warp whose 64 pixels have all three duals
-// inside the disc (where the factors are 1 and the values stay) skips them:
-// one vote for the three.  On a GB300 against no vote: 64 VGA pairs 36.83 ->
-// 36.62 ms and 16 warm-started ones 8.94 -> 8.77 ms, five pairs 3.71 -> 3.76
-// ms; a vote a dual instead: 36.71, 8.87 and 3.75 ms.  A thread with a sum
-// beyond disc_factor's range takes the scalar form.
+// expressions in packed FP32x2.  With kVote a warp whose 64 pixels have all three
+// duals inside the disc (where the factors are 1 and the values stay) skips
+// them: one vote for the three.  That pays where launches are many regions a CTA
+// (the strips; GB300, against no vote: 64 VGA pairs 36.83 -> 36.62 ms, 16
+// warm-started ones 8.94 -> 8.77; a vote a dual instead: 36.71, 8.87), and costs
+// where a launch's time is its dependent chain (one VGA pair 1.020 -> 1.028 ms,
+// five as tiles 3.71 -> 3.76).  A thread with a sum beyond disc_factor's range
+// takes the scalar form.
 struct Disc2 {
     float2 s;
     __device__ __forceinline__ Disc2(float2 a, float2 b)
@@ -49,12 +51,13 @@ struct Disc2 {
         b = mul2(b, f);
     }
 };
+template <bool kVote>
 __device__ __forceinline__ void project_duals(float2& puu, float2& puv, float2& pvu, float2& pvv, float2& pwu,
                                               float2& pwv)
 {
     const Disc2 u(puu, puv), v(pvu, pvv), w(pwu, pwv);
     const float peak = max_nan(max_nan(u.peak(), v.peak()), w.peak());
-    if (__all_sync(0xffffffffu, peak < 0.999f)) return;
+    if (kVote && __all_sync(0xffffffffu, peak < 0.999f)) return;
     if (peak < kDiscLimit) {
         u.apply(puu, puv);
         v.apply(pvu, pvv);
@@ -122,10 +125,10 @@ struct PairPlace {
 // One iteration.  X: the three planes of the dual step's published values, me
 // and right the pair's and its right neighbour's offsets in a plane (the own
 // one beyond the region: read, then not needed); Y: the primal step's.  kBorder:
-// the region touches the image border.  h.sync() is the barrier of the threads
+// the region touches the image border; kVote: project_duals'.  h.sync() is the barrier of the threads
 // that exchange, h.carry(yu, yv, yw) sees the published primal-step values, and
 // h.left(k) is where the left neighbour's value of component k is read.
-template <bool kBorder, int kLanes, class Hooks>
+template <bool kBorder, int kLanes, bool kVote, class Hooks>
 __device__ __forceinline__ void iterate_pair(PairState& s, const PairConsts& k, const PairDerived& d, float* X,
                                              float* Y, int plane, int me, int right, const PairPlace& at, float li,
                                              float ld, Hooks h)
@@ -170,7 +173,7 @@ __device__ __forceinline__ void iterate_pair(PairState& s, const PairConsts& k, 
         s.pwv = fm2(k.s4, gw2, s.pwv);
         s.pd.x = clamp1(s.pd.x);
         s.pd.y = clamp1(s.pd.y);
-        project_duals(s.puu, s.puv, s.pvu, s.pvv, s.pwu, s.pwv);
+        project_duals<kVote>(s.puu, s.puv, s.pvu, s.pvv, s.pwu, s.pwv);
     }
     // ---------------- primal step (computeDivergence + updatePrimalVariables) ----------------
     {

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kLanes* kCols) k_iterate_resident(const __grid
     for (unsigned done = 0;; buffer ^= 1u) {
         const unsigned kk = min(a.iters - done, (unsigned)kHalo);
         for (unsigned j = 0; j < kk; ++j)
-            iterate_pair<true, kLanes>(s, k, d, X, Y, T::kPlane, me, right, place, a.lambda_i, a.lambda_d,
+            iterate_pair<true, kLanes, false>(s, k, d, X, Y, T::kPlane, me, right, place, a.lambda_i, a.lambda_d,
                                        Hooks{Y + left});
         done += kk;
         if (done >= a.iters) break;

@@ -227,15 +227,16 @@ static bool level_runs_tiles(const pdflow_solver* s, const LevelGeom& g, unsigne
 // whichever end earlier on the SMs (strips need tensor copies).  Measured on
 // either side of that line on a GB300 (100 iterations at 480x640, tiles / strips):
 // 2 pairs 0.981 / 0.928 ms, 6 pairs 2.41 / 2.25, 3 pairs 1.300 / 1.302, 7 pairs 2.71
-// / 2.75.
+// / 2.75.  From two strips an SM on the queue evens out what the tiles' fixed deal
+// leaves (64 pairs at 120x160, 14.9 regions against 15 rounds: 1.24 / 1.17 ms).
 int pdflow::default_level_form(const pdflow_solver* s, const LevelGeom& g, bool resident)
 {
     const unsigned sms = unsigned(s->num_sms);
     if (resident && resident_eligible(g, s->L, s->S, s->S, sms)) return 9;
     if (g.pairs * ((g.R + 15u) / 16u) * ((g.C + 15u) / 16u) <= sms) return 9;
     if (!stream_eligible(g, s->L, s->S, s->S, 10)) return 8;
-    const unsigned tiles = g.pairs * ((g.R + 23u) / 24u) * ((g.C + 23u) / 24u);
-    return strips_end(g, sms) < 0.97f * float((tiles + sms - 1) / sms) ? 10 : 8;
+    const unsigned bands = g.pairs * ((g.R + 23u) / 24u), tiles = bands * ((g.C + 23u) / 24u);
+    return bands >= 2 * sms || strips_end(g, sms) < 0.97f * float((tiles + sms - 1) / sms) ? 10 : 8;
 }
 
 namespace pdflow {
