@@ -517,8 +517,8 @@ def ours(args):
         if ws > 1:
             torch.distributed.barrier()
         v, tot = replica_value(torch, t_all0.elapsed_time(t_all1), B, K, device=dev)
-        # 2 pushes x (decode + 5 pyramid levels) + the solve's own launches
-        return v, tot, [a_.elapsed_time(e_) for a_, e_ in ev], 2 * 6 + cnt.value, fb
+        # 2 pushes x 3 pyramid passes (levels 0-2, 3-4, 5) + the solve's own launches
+        return v, tot, [a_.elapsed_time(e_) for a_, e_ in ev], 2 * 3 + cnt.value, fb
 
     sampler.wait_first()
     mark = len(sampler.lines)

@@ -104,7 +104,6 @@ constexpr unsigned kSeedLevel = 2;       // the 60x80 level (15x20 -> 30x40 -> 6
 constexpr unsigned kSeedN = 60 * 80;
 
 void carve_solver(pdflow_solver* s, char* base, size_t* used);
-int enqueue_pyramid(pdflow_solver* s, cudaStream_t st, unsigned pairs, const unsigned* map = nullptr);
 int enqueue_solve(pdflow_solver* s, cudaStream_t st, unsigned pairs, const SolvePlan& plan = SolvePlan());
 int enqueue_energy(pdflow_solver* s, cudaStream_t st, unsigned pairs, unsigned level, float* out,
                    const unsigned* map = nullptr);

@@ -7,6 +7,8 @@
 // (gradient+dual, divergence+primal; the reference uses four) and the last
 // primal kernel of a level also saturates; the weighted median and the motion
 // field are one kernel.  All per-pixel arithmetic lives in pdflow_math.cuh.
+#include <algorithm>
+
 #include "pdflow_kernels.cuh"
 #include "pdflow_math.cuh"
 
@@ -21,156 +23,199 @@ __host__ __device__ inline unsigned blocks_for(unsigned n) { return (n + kBlock 
 // ---------------------------------------------------------------------------
 // Pyramid (computePyramidLevel, pdflow_cudalib.cu:331-434)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void write_xy(PyrLevel out, unsigned R, unsigned C, unsigned v, unsigned u,
-                                         unsigned idx, float depth, float fovh)
-{
-    const float inv_f_i = inv_focal(fovh, C);
-    out.xx[idx] = backproject(u, C, depth, inv_f_i);
-    out.yy[idx] = backproject(v, R, depth, inv_f_i);
-}
 
-// Row-major uint8/uint16 camera images -> column-major level 0 (decode +
-// transpose through a 32x33 shared tile so that both sides are coalesced).
-__global__ void __launch_bounds__(1024) k_decode_u16(const uint8_t* __restrict__ img,
-                                                     const uint16_t* __restrict__ depth, unsigned W, unsigned H,
-                                                     PyrLevel out, float fovh, size_t pstride,
-                                                     const unsigned* __restrict__ map)
+// One pixel (v, u) of an R x C level from the level above it: the depth-weighted
+// 5x5 mask; above(k, l) is (intensity, depth) of the level above at row 2v + k,
+// column 2u + l.  sumc and sumd fuse their products; the depth weight is added after
+// rounding (acu_weights_d += aux_w), as in the reference build.
+template <class Above>
+__device__ __forceinline__ float2 down_px(unsigned v, unsigned u, unsigned R, unsigned C, Above above)
 {
-    img += (size_t)blockIdx.z * W * H;
-    depth += (size_t)blockIdx.z * W * H;
-    out = at(out, pair_off(map, pstride, blockIdx.z));
-    __shared__ float sc[32][33];
-    __shared__ float sz[32][33];
-    const unsigned x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    {
-        const unsigned x = x0 + threadIdx.x, y = y0 + threadIdx.y;
-        if (x < W && y < H) {
-            const size_t i = (size_t)y * W + x;
-            sc[threadIdx.y][threadIdx.x] = float(img[i]);
-            sz[threadIdx.y][threadIdx.x] = decode_depth(depth[i]);
-        }
-    }
-    __syncthreads();
-    const unsigned v = y0 + threadIdx.x, u = x0 + threadIdx.y;  // writes walk along v
-    if (u < W && v < H) {
-        const unsigned idx = v + u * H;
-        const float z = sz[threadIdx.x][threadIdx.y];
-        out.col[idx] = sc[threadIdx.x][threadIdx.y];
-        out.dep[idx] = z;
-        write_xy(out, H, W, v, u, idx, z, fovh);
-    }
-}
-
-// Row-major RGB888 + uint16 millimetre depth -> column-major level 0 with the
-// live application's conversion (gray_rgb, decode_depth_mm).  rotate180: its
-// camera loop (scene_flow_visualization.cpp:313-323) stores camera pixel
-// (y, x) at row H-1-y, column W-1-x.
-__global__ void __launch_bounds__(1024) k_decode_rgb8_mm(const uint8_t* __restrict__ rgb,
-                                                         const uint16_t* __restrict__ depth, unsigned W, unsigned H,
-                                                         PyrLevel out, float fovh, size_t pstride,
-                                                         const unsigned* __restrict__ map, int rotate180)
-{
-    rgb += (size_t)blockIdx.z * W * H * 3;
-    depth += (size_t)blockIdx.z * W * H;
-    out = at(out, pair_off(map, pstride, blockIdx.z));
-    __shared__ float sc[32][33];
-    __shared__ float sz[32][33];
-    const unsigned x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-    {
-        const unsigned x = x0 + threadIdx.x, y = y0 + threadIdx.y;   // stored (row y, column x)
-        if (x < W && y < H) {
-            const size_t i = rotate180 ? (size_t)(H - 1 - y) * W + (W - 1 - x) : (size_t)y * W + x;
-            sc[threadIdx.y][threadIdx.x] = gray_rgb(rgb[3 * i], rgb[3 * i + 1], rgb[3 * i + 2]);
-            sz[threadIdx.y][threadIdx.x] = decode_depth_mm(depth[i]);
-        }
-    }
-    __syncthreads();
-    const unsigned v = y0 + threadIdx.x, u = x0 + threadIdx.y;  // writes walk along v
-    if (u < W && v < H) {
-        const unsigned idx = v + u * H;
-        const float z = sz[threadIdx.x][threadIdx.y];
-        out.col[idx] = sc[threadIdx.x][threadIdx.y];
-        out.dep[idx] = z;
-        write_xy(out, H, W, v, u, idx, z, fovh);
-    }
-}
-
-__global__ void k_pyr_level0(const float* __restrict__ I, const float* __restrict__ Z, unsigned R, unsigned C,
-                             PyrLevel out, float fovh, size_t pstride, const unsigned* __restrict__ map)
-{
-    const size_t po = pair_off(map, pstride, blockIdx.y);
-    I = at(I, po);
-    Z = at(Z, po);
-    out = at(out, po);
-    const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= R * C) return;
-    const unsigned v = idx % R, u = idx / R;
-    out.col[idx] = I[idx];
-    const float z = Z[idx];
-    out.dep[idx] = z;
-    write_xy(out, R, C, v, u, idx, z, fovh);
-}
-
-__global__ void k_pyr_down(PyrLevel prev, unsigned R, unsigned C, PyrLevel out, float fovh, size_t pstride,
-                           const unsigned* __restrict__ map)
-{
-    const size_t po = pair_off(map, pstride, blockIdx.y);
-    prev = at(prev, po);
-    out = at(out, po);
-    const unsigned index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= R * C) return;
-    const unsigned v = index % R, u = index / R;
     const float max_depth_dif = 0.1f;
-    const float* __restrict__ cp = prev.col;
-    const float* __restrict__ dp = prev.dep;
+    const float dcenter = above(0, 0).y;
     float sumd = 0.f, sumc = 0.f, acu_weights_d = 0.f, acu_weights_c = 0.f;
-    const unsigned ind_cent_prev = 2 * v + 4 * u * R;
-    const float dcenter = dp[ind_cent_prev];
-    float dres, cres;
-    // sumc and sumd fuse their products; the depth weight is added after
-    // rounding (acu_weights_d += aux_w), as in the reference build.
+    auto depth_tap = [&](float gm, float d) {
+        const float ad = fabsf(sub(d, dcenter));
+        if ((d > 0.f) && (ad < max_depth_dif)) {
+            const float aux_w = mul(gm, sub(max_depth_dif, ad));
+            acu_weights_d = add(acu_weights_d, aux_w);
+            sumd = fm(aux_w, d, sumd);
+        }
+    };
+    float cres;
     if ((v > 0) && (v < R - 1) && (u > 0) && (u < C - 1)) {
 #pragma unroll
         for (int k = -2; k < 3; k++)
 #pragma unroll
             for (int l = -2; l < 3; l++) {
-                const unsigned ind_loop_prev = 2 * v + k + 2 * (2 * u + l) * R;
                 const float gm = gmask(k, l);
-                sumc = fm(gm, cp[ind_loop_prev], sumc);
-                const float d = dp[ind_loop_prev];
-                const float ad = fabsf(sub(d, dcenter));
-                if ((d > 0.f) && (ad < max_depth_dif)) {
-                    const float aux_w = mul(gm, sub(max_depth_dif, ad));
-                    acu_weights_d = add(acu_weights_d, aux_w);
-                    sumd = fm(aux_w, d, sumd);
-                }
+                const float2 x = above(k, l);
+                sumc = fm(gm, x.x, sumc);
+                depth_tap(gm, x.y);
             }
-        dres = (sumd > 0.f) ? qt(sumd, acu_weights_d) : 0.f;
         cres = sumc;
     } else {
         for (int k = -2; k < 3; k++)
             for (int l = -2; l < 3; l++) {
                 const int indv = 2 * (int)v + k, indu = 2 * (int)u + l;
                 if ((indv >= 0) && (indv < 2 * (int)R) && (indu >= 0) && (indu < 2 * (int)C)) {
-                    const unsigned ind_loop_prev = 2 * v + k + 2 * (2 * u + l) * R;
                     const float gm = gmask(k, l);
-                    sumc = fm(gm, cp[ind_loop_prev], sumc);
+                    const float2 x = above(k, l);
+                    sumc = fm(gm, x.x, sumc);
                     acu_weights_c = add(acu_weights_c, gm);
-                    const float d = dp[ind_loop_prev];
-                    const float ad = fabsf(sub(d, dcenter));
-                    if ((d > 0.f) && (ad < max_depth_dif)) {
-                        const float aux_w = mul(gm, sub(max_depth_dif, ad));
-                        acu_weights_d = add(acu_weights_d, aux_w);
-                        sumd = fm(aux_w, d, sumd);
-                    }
+                    depth_tap(gm, x.y);
                 }
             }
         cres = qt(sumc, acu_weights_c);
-        dres = (sumd > 0.f) ? qt(sumd, acu_weights_d) : 0.f;
     }
-    out.col[index] = cres;
-    out.dep[index] = dres;
-    write_xy(out, R, C, v, u, index, dres, fovh);
+    return make_float2(cres, (sumd > 0.f) ? qt(sumd, acu_weights_d) : 0.f);
+}
+
+__device__ __forceinline__ void put_px(const PyrLevel& out, unsigned R, unsigned C, unsigned v, unsigned u, float2 cz,
+                                       float inv_f_i)
+{
+    const unsigned idx = v + u * R;
+    out.col[idx] = cz.x;
+    out.dep[idx] = cz.y;
+    out.xx[idx] = backproject(u, C, cz.y, inv_f_i);
+    out.yy[idx] = backproject(v, R, cz.y, inv_f_i);
+}
+
+// Where a pyramid starts: (intensity, metres) of pixel (row v, column u).
+// Row-major camera images ([pair][H][W]) are read along their rows, column-major
+// planes along their columns.
+struct SourceU16 {   // uint8 intensity, uint16 depth
+    static constexpr bool kRowMajor = true;
+    const uint8_t* img;
+    const uint16_t* depth;
+    unsigned W, H;
+    __device__ __forceinline__ void pair(unsigned z, size_t)
+    {
+        img += (size_t)z * W * H;
+        depth += (size_t)z * W * H;
+    }
+    __device__ __forceinline__ float2 at(unsigned v, unsigned u) const
+    {
+        const size_t i = (size_t)v * W + u;
+        return make_float2(float(img[i]), decode_depth(depth[i]));
+    }
+};
+// RGB888 + millimetre depth with the live application's conversion (gray_rgb,
+// decode_depth_mm).  rotate180: its camera loop
+// (scene_flow_visualization.cpp:313-323) stores camera pixel (y, x) at row
+// H-1-y, column W-1-x.
+struct SourceRgb {
+    static constexpr bool kRowMajor = true;
+    const uint8_t* rgb;
+    const uint16_t* depth;
+    unsigned W, H;
+    int rotate180;
+    __device__ __forceinline__ void pair(unsigned z, size_t)
+    {
+        rgb += (size_t)z * W * H * 3;
+        depth += (size_t)z * W * H;
+    }
+    __device__ __forceinline__ float2 at(unsigned v, unsigned u) const
+    {
+        const size_t i = rotate180 ? (size_t)(H - 1 - v) * W + (W - 1 - u) : (size_t)v * W + u;
+        return make_float2(gray_rgb(rgb[3 * i], rgb[3 * i + 1], rgb[3 * i + 2]), decode_depth_mm(depth[i]));
+    }
+};
+struct SourcePlanes {   // column-major float planes of the pair's arena slice
+    static constexpr bool kRowMajor = false;
+    const float *col, *dep;
+    unsigned W, H;
+    __device__ __forceinline__ void pair(unsigned, size_t po)
+    {
+        col = pdflow::at(col, po);
+        dep = pdflow::at(dep, po);
+    }
+    __device__ __forceinline__ float2 at(unsigned v, unsigned u) const
+    {
+        const size_t i = v + (size_t)u * H;
+        return make_float2(col[i], dep[i]);
+    }
+};
+
+// A frame's 32 x 32 tile through three pyramid levels in one pass: the source
+// (levels + 0, W x H) is read once with a halo of 6 into shared memory, written
+// as the first level where kWriteFirst, reduced to the tile's 16 x 16 of the
+// second level with a halo of 2 (the halo pixels are the neighbours', computed
+// again) and to its 8 x 8 of the third (count 2: stop at the second).  Bound by
+// shared-memory reads and instruction issue of the 25 taps on a batch, by launch
+// latency for one frame.  Against a launch a level, two pushes on a GB300: one 320x240
+// frame 71 -> 34 us, one 640x480 89 -> 52, 64 716 -> 428.
+constexpr int kPyrTile = 32, kPyrHalo = 6, kPyrSide = kPyrTile + 2 * kPyrHalo, kPyrMid = kPyrTile / 2 + 4;
+
+// A tile's (intensity, depth) pixels, a column's even rows before its odd ones:
+// the taps of consecutive pixels of the next level, two rows apart, are then
+// consecutive in shared memory.
+template <int kSide>
+struct PyrTile {
+    float2 px[kSide][kSide + 1];
+    static __device__ __forceinline__ int slot(int row) { return (row & 1) * (kSide / 2) + (row >> 1); }
+    __device__ __forceinline__ float2& operator()(int col, int row) { return px[col][slot(row)]; }
+    // the tap k rows, l columns from (col, 2 half) of the next level's pixel
+    __device__ __forceinline__ float2 tap(int col, int half, int k, int l) const
+    {
+        return px[col + l][(k & 1) * (kSide / 2) + half + (k >> 1)];
+    }
+};
+
+template <class Source, bool kWriteFirst, unsigned kThreads>
+__global__ void __launch_bounds__(kThreads) k_pyramid(Source src, PyrLevel l0, PyrLevel l1, PyrLevel l2, int count,
+                                                        float fovh, size_t pstride, const unsigned* __restrict__ map)
+{
+    __shared__ PyrTile<kPyrSide> t0;
+    __shared__ PyrTile<kPyrMid> t1;
+    __shared__ float inv[3];   // the levels' focal factors (a tanf and a division each: once a tile)
+    if (threadIdx.x < 3) inv[threadIdx.x] = inv_focal(fovh, src.W >> threadIdx.x);
+    const size_t po = pair_off(map, pstride, blockIdx.z);
+    src.pair(blockIdx.z, po);
+    l1 = at(l1, po);
+    const int W = (int)src.W, H = (int)src.H;
+    const int U0 = (int)blockIdx.x * kPyrTile, V0 = (int)blockIdx.y * kPyrTile;
+    // a warp a row (row-major sources) or a column of the tile and its halo (of
+    // which two levels need 2 pixels)
+    const int skip = count > 2 ? 0 : kPyrHalo - 2;
+    for (int slow = skip + threadIdx.x / 32; slow < kPyrSide - skip; slow += kThreads / 32)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int fast = skip + q * 32 + (int)(threadIdx.x & 31);
+            const int i = Source::kRowMajor ? fast : slow, j = Source::kRowMajor ? slow : fast;   // column, row
+            const int u = U0 - kPyrHalo + i, v = V0 - kPyrHalo + j;
+            if (fast < kPyrSide - skip && u >= 0 && u < W && v >= 0 && v < H) t0(i, j) = src.at((unsigned)v, (unsigned)u);
+        }
+    __syncthreads();
+    if constexpr (kWriteFirst) {
+        l0 = at(l0, po);
+        for (int e = threadIdx.x; e < kPyrTile * kPyrTile; e += kThreads) {
+            const int j = e % kPyrTile, i = e / kPyrTile, u = U0 + i, v = V0 + j;
+            if (u < W && v < H)
+                put_px(l0, H, W, v, u, t0(kPyrHalo + i, kPyrHalo + j), inv[0]);
+        }
+    }
+    const int R1 = H / 2, C1 = W / 2, V1 = V0 / 2, U1 = U0 / 2;
+    const int halo1 = count > 2 ? 2 : 0, side1 = kPyrTile / 2 + 2 * halo1;
+    for (int e = threadIdx.x; e < side1 * side1; e += kThreads) {
+        const int j = e % side1, i = e / side1, u = U1 - halo1 + i, v = V1 - halo1 + j;
+        if (u < 0 || u >= C1 || v < 0 || v >= R1) continue;
+        const int col = 2 * (i - halo1) + kPyrHalo, half = j - halo1 + kPyrHalo / 2;   // (2u, 2v) in t0
+        const float2 x = down_px(v, u, R1, C1, [&](int k, int l) { return t0.tap(col, half, k, l); });
+        if (i >= halo1 && i < halo1 + kPyrTile / 2 && j >= halo1 && j < halo1 + kPyrTile / 2)
+            put_px(l1, R1, C1, v, u, x, inv[1]);
+        if (count > 2) t1(i, j) = x;
+    }
+    if (count < 3) return;
+    __syncthreads();
+    l2 = at(l2, po);
+    const int R2 = H / 4, C2 = W / 4;
+    for (int e = threadIdx.x; e < kPyrTile / 4 * (kPyrTile / 4); e += kThreads) {
+        const int j = e % (kPyrTile / 4), i = e / (kPyrTile / 4), u = U0 / 4 + i, v = V0 / 4 + j;
+        if (u >= C2 || v >= R2) continue;
+        put_px(l2, R2, C2, v, u,
+               down_px(v, u, R2, C2, [&](int k, int l) { return t1.tap(2 * i + 2, j + 1, k, l); }), inv[2]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -742,28 +787,15 @@ __global__ void k_level_keep(LevelGeom g, LevelSol sol, PyrLevel o, Params p, fl
     k[5 * g.N + i] = dz;
 }
 
-// Frame t's pyramid level becomes frame t-1's, for the mapped slots (float4
-// copies; level planes are 16-byte aligned and padded to whole float4s).
-__global__ void k_pyr_copy(PyrLevel src, PyrLevel dst, unsigned n, size_t pstride, const unsigned* __restrict__ map)
+// Frame t's pyramid becomes frame t-1's, for the mapped slots: the planes of all
+// levels lie back to back (n float4, the padding between them included).
+__global__ void k_pyr_copy(const float4* src, float4* dst, size_t n, size_t pstride, const unsigned* __restrict__ map)
 {
     const size_t po = pair_off(map, pstride, blockIdx.y);
     src = at(src, po);
     dst = at(dst, po);
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (4 * i >= n) return;
-    if (4 * i + 4 <= n) {
-        reinterpret_cast<float4*>(dst.col)[i] = reinterpret_cast<const float4*>(src.col)[i];
-        reinterpret_cast<float4*>(dst.dep)[i] = reinterpret_cast<const float4*>(src.dep)[i];
-        reinterpret_cast<float4*>(dst.xx)[i] = reinterpret_cast<const float4*>(src.xx)[i];
-        reinterpret_cast<float4*>(dst.yy)[i] = reinterpret_cast<const float4*>(src.yy)[i];
-    } else {
-        for (unsigned k = 4 * i; k < n; ++k) {
-            dst.col[k] = src.col[k];
-            dst.dep[k] = src.dep[k];
-            dst.xx[k] = src.xx[k];
-            dst.yy[k] = src.yy[k];
-        }
-    }
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        dst[i] = src[i];
 }
 
 // Both frames at the solution's total image-plane flow, for the energy.
@@ -830,40 +862,74 @@ __global__ void __launch_bounds__(kEnergyAcc) k_energy_sum(const double* __restr
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-cudaError_t launch_decode_u16(const uint8_t* img, const uint16_t* depth, unsigned W, unsigned H, PyrLevel out,
-                              float fovh, unsigned pairs, size_t pstride, cudaStream_t st, const unsigned* map)
+namespace {
+
+// Up to this many pixels a pyramid is bound by latency: the first pass takes
+// three levels (one launch less for 320x240 frames), 512 threads a tile.  Beyond,
+// by instructions: two levels, so no second-level pixel is computed twice, and
+// 256 threads, so that tiles overlap.  Two pushes on a GB300 (few / many form):
+// one 320x240 frame 34 / 48 us, 8 52 / 64, 64 192 / 154; one 640x480 frame 52 / 61,
+// two 66 / 66, four 82 / 75, 64 605 / 428.
+constexpr size_t kPyrFewPixels = 2 * 640 * 480;
+
+// One pass: count - 1 levels below `src` (and with kWriteFirst src's own planes).
+template <bool kWriteFirst, class Source>
+cudaError_t pyramid_pass(const Source& src, const PyrLevel* levels, unsigned count, bool few, float fovh,
+                         unsigned pairs, size_t pstride, cudaStream_t st, const unsigned* map)
 {
-    dim3 grid((W + 31) / 32, (H + 31) / 32, pairs), block(32, 32);
-    k_decode_u16<<<grid, block, 0, st>>>(img, depth, W, H, out, fovh, pstride, map);
+    const dim3 grid((src.W + kPyrTile - 1) / kPyrTile, (src.H + kPyrTile - 1) / kPyrTile, pairs);
+    const PyrLevel &l1 = levels[1], &l2 = count > 2 ? levels[2] : levels[1];
+    if (few)
+        k_pyramid<Source, kWriteFirst, 512><<<grid, 512, 0, st>>>(src, levels[0], l1, l2, int(count), fovh, pstride, map);
+    else
+        k_pyramid<Source, kWriteFirst, 256><<<grid, 256, 0, st>>>(src, levels[0], l1, l2, int(count), fovh, pstride, map);
     return cudaGetLastError();
 }
 
-cudaError_t launch_decode_rgb8_mm(const uint8_t* rgb, const uint16_t* depth, unsigned W, unsigned H, PyrLevel out,
-                                  float fovh, unsigned pairs, size_t pstride, cudaStream_t st, int rotate180)
+template <class Source>
+cudaError_t pyramid(const Source& src, const PyrLevel* levels, unsigned count, float fovh, unsigned pairs,
+                    size_t pstride, cudaStream_t st, const unsigned* map)
 {
-    dim3 grid((W + 31) / 32, (H + 31) / 32, pairs), block(32, 32);
-    k_decode_rgb8_mm<<<grid, block, 0, st>>>(rgb, depth, W, H, out, fovh, pstride, nullptr, rotate180);
-    return cudaGetLastError();
+    if (count < 2) return cudaErrorInvalidValue;
+    const bool few = size_t(src.W) * src.H * pairs <= kPyrFewPixels;
+    const unsigned first = few ? std::min(count, 3u) : 2u;
+    cudaError_t e = pyramid_pass<true>(src, levels, first, few, fovh, pairs, pstride, st, map);
+    for (unsigned l = first - 1; l + 1 < count && e == cudaSuccess; l += 2) {   // levels l + 1, l + 2 from level l
+        const SourcePlanes up{levels[l].col, levels[l].dep, src.W >> l, src.H >> l};
+        e = pyramid_pass<false>(up, levels + l, std::min(count - l, 3u), few, fovh, pairs, pstride, st, map);
+    }
+    return e;
 }
 
-cudaError_t launch_pyr_level0(const float* I, const float* Z, unsigned R, unsigned C, PyrLevel out, float fovh,
-                              unsigned pairs, size_t pstride, cudaStream_t st, const unsigned* map)
+}  // namespace
+
+cudaError_t launch_pyramid_u16(const uint8_t* img, const uint16_t* depth, unsigned W, unsigned H,
+                               const PyrLevel* levels, unsigned count, float fovh, unsigned pairs, size_t pstride,
+                               cudaStream_t st, const unsigned* map)
 {
-    k_pyr_level0<<<dim3(blocks_for(R * C), pairs), kBlock, 0, st>>>(I, Z, R, C, out, fovh, pstride, map);
-    return cudaGetLastError();
+    return pyramid(SourceU16{img, depth, W, H}, levels, count, fovh, pairs, pstride, st, map);
 }
 
-cudaError_t launch_pyr_down(PyrLevel prev, unsigned R, unsigned C, PyrLevel out, float fovh, unsigned pairs,
-                            size_t pstride, cudaStream_t st, const unsigned* map)
+cudaError_t launch_pyramid_rgb8_mm(const uint8_t* rgb, const uint16_t* depth, unsigned W, unsigned H,
+                                   const PyrLevel* levels, unsigned count, float fovh, unsigned pairs, size_t pstride,
+                                   cudaStream_t st, int rotate180)
 {
-    k_pyr_down<<<dim3(blocks_for(R * C), pairs), kBlock, 0, st>>>(prev, R, C, out, fovh, pstride, map);
-    return cudaGetLastError();
+    return pyramid(SourceRgb{rgb, depth, W, H, rotate180}, levels, count, fovh, pairs, pstride, st, nullptr);
 }
 
-cudaError_t launch_pyr_copy(PyrLevel src, PyrLevel dst, unsigned n, unsigned pairs, size_t pstride,
-                            const unsigned* map, cudaStream_t st)
+cudaError_t launch_pyramid_planes(const float* I, const float* Z, unsigned W, unsigned H, const PyrLevel* levels,
+                                  unsigned count, float fovh, unsigned pairs, size_t pstride, cudaStream_t st)
 {
-    k_pyr_copy<<<dim3(blocks_for((n + 3) / 4), pairs), kBlock, 0, st>>>(src, dst, n, pstride, map);
+    return pyramid(SourcePlanes{I, Z, W, H}, levels, count, fovh, pairs, pstride, st, nullptr);
+}
+
+cudaError_t launch_pyr_copy(const PyrLevel* src, const PyrLevel* dst, unsigned levels, unsigned smallest, unsigned pairs,
+                            size_t pstride, const unsigned* map, cudaStream_t st)
+{
+    const size_t n = (size_t(src[levels - 1].yy - src[0].col) + smallest + 3) / 4;   // whole float4 (planes are padded)
+    const dim3 grid(unsigned(std::min<size_t>((n + kBlock - 1) / kBlock, 1024)), pairs);
+    k_pyr_copy<<<grid, kBlock, 0, st>>>(reinterpret_cast<const float4*>(src[0].col), reinterpret_cast<float4*>(dst[0].col),
+                                       n, pstride, map);
     return cudaGetLastError();
 }
 

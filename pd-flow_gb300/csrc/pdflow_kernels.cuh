@@ -117,22 +117,25 @@ struct Params {
 };
 
 // ---- launchers (each returns the launch error) ----
-// Pyramid launchers: `pairs` frames, pair k's arena buffers k * pstride bytes
-// after pair 0's; the raw inputs of launch_decode_u16 are [pairs][H][W].
-// A non-null `map` ([pairs] arena slots, device) redirects input k to slot map[k].
-cudaError_t launch_decode_u16(const uint8_t* img, const uint16_t* depth, unsigned W, unsigned H, PyrLevel out,
-                              float fovh, unsigned pairs, size_t pstride, cudaStream_t st,
-                              const unsigned* map = nullptr);
+// A frame's pyramid: levels[0 .. count) from its W x H pixels (count >= 2; level
+// l is (W >> l) x (H >> l)), `pairs` frames, pair k's arena buffers k * pstride
+// bytes after pair 0's; camera images are [pairs][H][W].  A non-null `map`
+// ([pairs] arena slots, device) redirects input k to slot map[k].
+cudaError_t launch_pyramid_u16(const uint8_t* img, const uint16_t* depth, unsigned W, unsigned H,
+                               const PyrLevel* levels, unsigned count, float fovh, unsigned pairs, size_t pstride,
+                               cudaStream_t st, const unsigned* map = nullptr);
 // RGB888 [pairs][H][W][3] + millimetre depth [pairs][H][W] (the live application's conversion).
-cudaError_t launch_decode_rgb8_mm(const uint8_t* rgb, const uint16_t* depth, unsigned W, unsigned H, PyrLevel out,
-                                  float fovh, unsigned pairs, size_t pstride, cudaStream_t st, int rotate180);
-cudaError_t launch_pyr_level0(const float* I, const float* Z, unsigned R, unsigned C, PyrLevel out, float fovh,
-                              unsigned pairs, size_t pstride, cudaStream_t st, const unsigned* map = nullptr);
-cudaError_t launch_pyr_down(PyrLevel prev, unsigned R, unsigned C, PyrLevel out, float fovh, unsigned pairs,
-                            size_t pstride, cudaStream_t st, const unsigned* map = nullptr);
-// Copies the planes of `src` over `dst` for the mapped slots (frame t becomes t-1).
-cudaError_t launch_pyr_copy(PyrLevel src, PyrLevel dst, unsigned n, unsigned pairs, size_t pstride,
-                            const unsigned* map, cudaStream_t st);
+cudaError_t launch_pyramid_rgb8_mm(const uint8_t* rgb, const uint16_t* depth, unsigned W, unsigned H,
+                                   const PyrLevel* levels, unsigned count, float fovh, unsigned pairs, size_t pstride,
+                                   cudaStream_t st, int rotate180);
+// Column-major float planes I, Z in every pair's arena slice.
+cudaError_t launch_pyramid_planes(const float* I, const float* Z, unsigned W, unsigned H, const PyrLevel* levels,
+                                  unsigned count, float fovh, unsigned pairs, size_t pstride, cudaStream_t st);
+// Copies the levels' planes of `src` over `dst` for the mapped slots (frame t
+// becomes t-1); the planes of both lie back to back in the same order, the last
+// level's have `smallest` floats.
+cudaError_t launch_pyr_copy(const PyrLevel* src, const PyrLevel* dst, unsigned levels, unsigned smallest, unsigned pairs,
+                            size_t pstride, const unsigned* map, cudaStream_t st);
 // The new frame's weighted image gradients of `count` levels of the same pairs
 // (levels[q]'s geometry and pyramid image), into the aux planes at float aux[q].
 cudaError_t launch_im_gradients(const LevelGeom* levels, const PyrLevel* images, const size_t* aux, unsigned count,

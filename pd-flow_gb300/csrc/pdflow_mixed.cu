@@ -352,19 +352,10 @@ int pdflow_push_frames_mixed(pdflow_solver* s, unsigned n, const unsigned* rows,
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(s->stage_u16, gr.Z, gr.img * 2 * m, cudaMemcpyHostToDevice, s->stream);
         if (e == cudaSuccess)
-            e = launch_decode_u16(s->stage_u8, s->stage_u16, gr.W, gr.H, s->pyr[f][gr.level], s->prm.fovh, m,
-                                  s->pair_stride, s->stream, s->map);
-        if (e == cudaSuccess && gr.level == 0)   // VGA pairs: their 320x240 level
-            e = launch_pyr_down(s->pyr[f][0], 240, 320, s->pyr[f][1], s->prm.fovh, m, s->pair_stride, s->stream,
-                                s->map);
+            e = launch_pyramid_u16(s->stage_u8, s->stage_u16, gr.W, gr.H, s->pyr[f] + gr.level, s->pyr_levels - gr.level,
+                                   s->prm.fovh, m, s->pair_stride, s->stream, s->map);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);   // the map and staging are reused
         if (e != cudaSuccess) return set_error_code(PDFLOW_ERR_CUDA, "mixed push", e);
-    }
-    // levels 2.. for every pair (slots 0..n-1)
-    for (unsigned l = 2; l < s->pyr_levels; ++l) {
-        cudaError_t e = launch_pyr_down(s->pyr[f][l - 1], 480u >> l, 640u >> l, s->pyr[f][l], s->prm.fovh, n,
-                                        s->pair_stride, s->stream);
-        if (e != cudaSuccess) return set_error_code(PDFLOW_ERR_CUDA, "mixed pyramid", e);
     }
     if (s->frames < 2) ++s->frames;
     return PDFLOW_OK;

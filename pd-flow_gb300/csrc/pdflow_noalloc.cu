@@ -170,10 +170,9 @@ int pdflow_solve_pair_noalloc(unsigned rows, unsigned width, unsigned height, co
     const uint16_t* dep[2] = {d_depth1, d_depth2};
     for (int f = 0; f < 2; ++f) {
         s.new_slot ^= 1;
-        e = pdflow::launch_decode_u16(img[f], dep[f], width, height, s.pyr[s.new_slot][0], s.prm.fovh, 1, 0, st);
-        if (e != cudaSuccess) return fail(PDFLOW_ERR_CUDA, "decode launch", e);
-        rc = pdflow::enqueue_pyramid(&s, st, 1);
-        if (rc != PDFLOW_OK) return fail(rc, "pyramid launch");
+        e = pdflow::launch_pyramid_u16(img[f], dep[f], width, height, s.pyr[s.new_slot], s.pyr_levels, s.prm.fovh, 1, 0,
+                                       st);
+        if (e != cudaSuccess) return fail(PDFLOW_ERR_CUDA, "pyramid launch", e);
     }
     s.frames = 2;
     rc = pdflow::enqueue_solve(&s, st, 1);

@@ -153,18 +153,6 @@ void carve_solver(pdflow_solver* s, char* base, size_t* used)
 
 int set_error_code(int code, const char* what, cudaError_t e) { return set_error(code, what, e); }
 
-int enqueue_pyramid(pdflow_solver* s, cudaStream_t st, unsigned pairs, const unsigned* map)
-{
-    const int f = s->new_slot;
-    for (unsigned l = 1; l < s->pyr_levels; ++l) {
-        const unsigned Cl = 640 / (s->cam_mode << l), Rl = 480 / (s->cam_mode << l);
-        CUDA_TRY(launch_pyr_down(s->pyr[f][l - 1], Rl, Cl, s->pyr[f][l], s->prm.fovh, pairs, s->pair_stride, st,
-                                 map),
-                 "pyramid launch");
-    }
-    return PDFLOW_OK;
-}
-
 size_t level_keep_offset(const pdflow_solver* s, unsigned level)
 {
     size_t off = 0;
@@ -502,10 +490,8 @@ int run_graphed(pdflow_solver* s, unsigned pairs, unsigned kind, EnqueueFn fn, c
 // ---------------------------------------------------------------------------
 namespace {
 
-int push_common(pdflow_solver* s, unsigned pairs)
+int push_done(pdflow_solver* s)
 {
-    int rc = enqueue_pyramid(s, s->stream, pairs);
-    if (rc) return rc;
     if (s->frames < 2) ++s->frames;
     return PDFLOW_OK;
 }
@@ -676,10 +662,10 @@ int pdflow_push_frames(pdflow_solver* s, unsigned n, const float* I, const float
              "H2D intensity");
     CUDA_TRY(cudaMemcpy2DAsync(s->stage_Z, s->pair_stride, Z, b, b, n, cudaMemcpyHostToDevice, s->stream),
              "H2D depth");
-    CUDA_TRY(launch_pyr_level0(s->stage_I, s->stage_Z, s->height, s->width, s->pyr[s->new_slot][0], s->prm.fovh, n,
-                               s->pair_stride, s->stream),
-             "level-0 launch");
-    return push_common(s, n);
+    CUDA_TRY(launch_pyramid_planes(s->stage_I, s->stage_Z, s->width, s->height, s->pyr[s->new_slot], s->pyr_levels,
+                                   s->prm.fovh, n, s->pair_stride, s->stream),
+             "pyramid launch");
+    return push_done(s);
 }
 
 int pdflow_push_frame(pdflow_solver* s, const float* I, const float* Z) { return pdflow_push_frames(s, 1, I, Z); }
@@ -692,10 +678,10 @@ int pdflow_push_frames_u16_device(pdflow_solver* s, unsigned n, const uint8_t* d
     if (s->slot_mode) return set_error(PDFLOW_ERR_STATE, "frames were pushed per slot: use the slot calls");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
     s->new_slot ^= 1;
-    CUDA_TRY(launch_decode_u16(d_intensity, d_depth, s->width, s->height, s->pyr[s->new_slot][0], s->prm.fovh, n,
-                               s->pair_stride, s->stream),
-             "decode launch");
-    return push_common(s, n);
+    CUDA_TRY(launch_pyramid_u16(d_intensity, d_depth, s->width, s->height, s->pyr[s->new_slot], s->pyr_levels,
+                                s->prm.fovh, n, s->pair_stride, s->stream),
+             "pyramid launch");
+    return push_done(s);
 }
 
 int pdflow_push_frame_u16_device(pdflow_solver* s, const uint8_t* d_intensity, const uint16_t* d_depth)
@@ -726,10 +712,10 @@ int pdflow_push_frames_rgb8_mm_device(pdflow_solver* s, unsigned n, const uint8_
     if (s->slot_mode) return set_error(PDFLOW_ERR_STATE, "frames were pushed per slot: use the slot calls");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
     s->new_slot ^= 1;
-    CUDA_TRY(launch_decode_rgb8_mm(d_rgb, d_depth_mm, s->width, s->height, s->pyr[s->new_slot][0], s->prm.fovh, n,
-                                   s->pair_stride, s->stream, rotate180 ? 1 : 0),
-             "RGB decode launch");
-    return push_common(s, n);
+    CUDA_TRY(launch_pyramid_rgb8_mm(d_rgb, d_depth_mm, s->width, s->height, s->pyr[s->new_slot], s->pyr_levels,
+                                    s->prm.fovh, n, s->pair_stride, s->stream, rotate180 ? 1 : 0),
+             "RGB pyramid launch");
+    return push_done(s);
 }
 
 int pdflow_push_frames_rgb8_mm(pdflow_solver* s, unsigned n, const uint8_t* rgb, const uint16_t* depth_mm,
@@ -862,15 +848,12 @@ int pdflow_push_frames_slots_u16_device(pdflow_solver* s, unsigned n, const unsi
     // frame t-1 := frame t for these slots, then frame t := the new frame
     const int fn = s->new_slot, fo = fn ^ 1;
     const size_t Nimg = size_t(s->width) * s->height;
-    for (unsigned l = 0; l < s->pyr_levels; ++l)
-        CUDA_TRY(launch_pyr_copy(s->pyr[fn][l], s->pyr[fo][l], unsigned(Nimg >> (2 * l)), n, s->pair_stride, s->map,
-                                 s->stream),
-                 "pyramid copy launch");
-    CUDA_TRY(launch_decode_u16(d_intensity, d_depth, s->width, s->height, s->pyr[fn][0], s->prm.fovh, n,
-                               s->pair_stride, s->stream, s->map),
-             "decode launch");
-    rc = enqueue_pyramid(s, s->stream, n, s->map);
-    if (rc) return rc;
+    CUDA_TRY(launch_pyr_copy(s->pyr[fn], s->pyr[fo], s->pyr_levels, unsigned(Nimg >> (2 * (s->pyr_levels - 1))), n,
+                             s->pair_stride, s->map, s->stream),
+             "pyramid copy launch");
+    CUDA_TRY(launch_pyramid_u16(d_intensity, d_depth, s->width, s->height, s->pyr[fn], s->pyr_levels, s->prm.fovh, n,
+                                s->pair_stride, s->stream, s->map),
+             "pyramid launch");
     for (unsigned k = 0; k < n; ++k)
         if (s->slot_frames[slots[k]] < 2) ++s->slot_frames[slots[k]];
     return PDFLOW_OK;
