@@ -41,6 +41,15 @@ struct pdflow_solver {
     pdflow::LevelSol sol{};
     unsigned* flags = nullptr;           // per-CTA progress counters of the grid-form iteration
     unsigned* status = nullptr;          // device status word (0 = ok)
+    // Pinned host memory the device addresses (null: transfers go to and from the
+    // caller's memory directly): the status word, two frame buffers, a result buffer.
+    unsigned* host_status = nullptr;
+    uint8_t* host_frames[2] = {};
+    size_t host_frame_bytes = 0;
+    cudaEvent_t host_frame_read[2] = {}; // the device has read the frame buffer
+    int host_frame_next = 0;
+    float* host_flow = nullptr;
+    size_t host_flow_bytes = 0;
     int num_sms = 0;
     int iter_form = 10;                  // 10 = streamed strips (levels with a strip per SM; others 9 or 8),
                                          // 9 = deep streamed tiles,
@@ -151,6 +160,17 @@ struct TuneCandidate {
 };
 TuneCandidate tune_candidate(int c);
 int check_status(pdflow_solver* s);
+// The handle's pinned transfer buffers, for results of `flow` bytes and more.
+// check_status in two halves: status_begin before the copies of a result (they
+// may block on the host), status_end after them.
+void create_host_buffers(pdflow_solver* s, size_t flow);
+void destroy_host_buffers(pdflow_solver* s);
+int status_begin(pdflow_solver* s);
+int status_end(pdflow_solver* s);
+// Flow planes (null: not wanted) of `rows`-row pairs to the host: pair k's from
+// `step` bytes after pair k-1's, the first `offset` bytes into the arena; n pairs
+// packed in each of dx, dy, dz.  Ends with the status check.
+int read_planes(pdflow_solver* s, size_t offset, size_t step, unsigned n, size_t floats, float* dx, float* dy, float* dz);
 void set_last_error(const char* text);   // the text pdflow_last_error returns on this thread
 // The iteration form a level (of g.pairs pairs) runs in unless one was chosen
 // for it; `resident`: its iterations may run in one launch (form 9).

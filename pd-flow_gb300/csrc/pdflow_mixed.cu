@@ -296,6 +296,8 @@ int pdflow_create_mixed(unsigned max_pairs, pdflow_solver** out)
     int rc = pdflow_create_batch(480, 640, 480, nullptr, max_pairs, out);
     if (rc) return rc;
     (*out)->mixed = 1;
+    pdflow::destroy_host_buffers(*out);   // sized for 640x480 results: here those of up to 120x160 pass
+    pdflow::create_host_buffers(*out, size_t(60) * 80 * 12);
     (*out)->mixed_rows.assign(max_pairs, 0);
     return PDFLOW_OK;
 }
@@ -426,14 +428,7 @@ int pdflow_read_flow_mixed(pdflow_solver* s, unsigned k, float* dx, float* dy, f
     }
     const unsigned r = s->mixed_rows[k];
     const size_t N = size_t(r) * (r * 4 / 3), po = size_t(k) * s->pair_stride;
-    float* dst[3] = {dx, dy, dz};
-    const float* src[3] = {s->dx, s->dy, s->dz};
-    for (int a = 0; a < 3; ++a)
-        if (dst[a]) {
-            cudaError_t e = cudaMemcpyAsync(dst[a], at(src[a], po), N * 4, cudaMemcpyDeviceToHost, s->stream);
-            if (e != cudaSuccess) return set_error_code(PDFLOW_ERR_CUDA, "D2H flow", e);
-        }
-    return check_status(s);
+    return read_planes(s, po, s->pair_stride, 1, N, dx, dy, dz);
 }
 
 }  // extern "C"

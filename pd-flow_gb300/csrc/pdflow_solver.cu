@@ -8,6 +8,7 @@
 // issues no allocation, no host synchronisation and (in graph mode) one launch.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -82,19 +83,148 @@ namespace pdflow {
 
 void set_last_error(const char* text) { g_last_error = text; }
 
+// The status word comes back through pinned memory, asynchronously: a copy to
+// pageable memory waits for the stream (10 us a call, on top of the result's).
+int status_begin(pdflow_solver* s)
+{
+    if (s->host_status)
+        CUDA_TRY(cudaMemcpyAsync(s->host_status, s->status, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream),
+                 "status read");
+    return PDFLOW_OK;
+}
+
 // Waits for the handle's stream and reports (then clears) a device-side
 // timeout recorded by a bounded wait.
-int check_status(pdflow_solver* s)
+int status_end(pdflow_solver* s)
 {
     unsigned st = 0;
-    CUDA_TRY(cudaMemcpyAsync(&st, s->status, sizeof st, cudaMemcpyDeviceToHost, s->stream), "status read");
+    if (!s->host_status)
+        CUDA_TRY(cudaMemcpyAsync(&st, s->status, sizeof st, cudaMemcpyDeviceToHost, s->stream), "status read");
     CUDA_TRY(cudaStreamSynchronize(s->stream), "synchronize");
+    if (s->host_status) st = *static_cast<volatile unsigned*>(s->host_status);
     if (st != 0) {
         CUDA_TRY(cudaMemsetAsync(s->status, 0, 4 * sizeof st, s->stream), "status reset");   // and the strip counters
         CUDA_TRY(cudaStreamSynchronize(s->stream), "synchronize");
         return set_error(PDFLOW_ERR_TIMEOUT, "a bounded device-side wait gave up (iteration neighbour sync)");
     }
     return PDFLOW_OK;
+}
+
+int check_status(pdflow_solver* s)
+{
+    const int rc = status_begin(s);
+    return rc ? rc : status_end(s);
+}
+
+// Small transfers pass through the handle's pinned buffers, which the kernels
+// address: the pyramid's first pass reads the frame there and k_flow_out writes
+// the planes and the status word there, so that neither side has copies to wait
+// for.  A copy to or from pageable memory costs 10 us and blocks, at any size (and
+// 6 us a MB); what passes through is copied by the host, at about 15 GB/s where the
+// device wrote it.  Two pushes and the wait for them, one 320x240 uint16 frame
+// (230 KB): 89 -> 65 us; as float planes (614 KB): 102 -> 107.  Reading a flow at
+// 60x80 (58 KB): 40 -> 21 us; at 240x320 (922 KB): 48 -> 75.  The limits lie between.
+constexpr size_t kHostFrameLimit = 256u << 10, kHostFlowLimit = 256u << 10;
+
+// For results of `flow` bytes and more; up to 0.1 ms of a handle's creation
+// (pinned pages come 2 MB at a time).  Best effort: without the memory (or
+// where nothing would pass through it) transfers are direct.
+void create_host_buffers(pdflow_solver* s, size_t flow)
+{
+    const size_t frame = size_t(s->width) * s->height * 3 + 256;   // uint8 intensity and uint16 depth
+    const size_t fcap = frame <= kHostFrameLimit ? frame : 0;
+    const size_t ocap = flow <= kHostFlowLimit ? std::min(flow * s->batch, kHostFlowLimit) : 0;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, 256 + 2 * ((fcap + 255) & ~size_t(255)) + ocap, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    s->host_status = static_cast<unsigned*>(p);
+    uint8_t* q = static_cast<uint8_t*>(p) + 256;
+    if (fcap && cudaEventCreateWithFlags(&s->host_frame_read[0], cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&s->host_frame_read[1], cudaEventDisableTiming) == cudaSuccess) {
+        for (int k = 0; k < 2; ++k) s->host_frames[k] = q + k * ((fcap + 255) & ~size_t(255));
+        s->host_frame_bytes = fcap;
+    } else {
+        cudaGetLastError();
+    }
+    s->host_flow = reinterpret_cast<float*>(q + 2 * ((fcap + 255) & ~size_t(255)));
+    s->host_flow_bytes = ocap;
+}
+
+void destroy_host_buffers(pdflow_solver* s)
+{
+    for (cudaEvent_t e : s->host_frame_read)
+        if (e) cudaEventDestroy(e);
+    if (s->host_status) cudaFreeHost(s->host_status);
+    s->host_status = nullptr;
+    for (cudaEvent_t& e : s->host_frame_read) e = nullptr;
+    s->host_frame_bytes = s->host_flow_bytes = 0;
+}
+
+// Ordinary host memory (neither pinned nor managed: work on the stream may still
+// be writing those; nor the device's, which a copy refuses).
+bool pageable(const void* p)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Copies a frame's two images into the next frame buffer; null where it goes
+// directly (size, memory, or a capture, which has to record the caller's address).
+// frame_passed() follows once the kernels that read it are enqueued.
+uint8_t* pass_frame(pdflow_solver* s, const void* a, size_t na, const void* b, size_t nb, size_t* second)
+{
+    *second = (na + 255) & ~size_t(255);
+    if (*second + nb > s->host_frame_bytes) return nullptr;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (!pageable(a) || !pageable(b)) return nullptr;
+    if (cudaEventSynchronize(s->host_frame_read[s->host_frame_next]) != cudaSuccess) return nullptr;
+    uint8_t* dst = s->host_frames[s->host_frame_next];
+    std::memcpy(dst, a, na);
+    std::memcpy(dst + *second, b, nb);
+    return dst;
+}
+
+int frame_passed(pdflow_solver* s, int rc)
+{
+    if (rc != PDFLOW_OK) return rc;
+    CUDA_TRY(cudaEventRecord(s->host_frame_read[s->host_frame_next], s->stream), "frame event");
+    s->host_frame_next ^= 1;
+    return PDFLOW_OK;
+}
+
+int read_planes(pdflow_solver* s, size_t offset, size_t step, unsigned n, size_t floats, float* dx, float* dy, float* dz)
+{
+    float* const dst[3] = {dx, dy, dz};
+    const float* const src[3] = {s->dx, s->dy, s->dz};
+    const size_t b = floats * 4;
+    bool pass = 3 * b * n <= s->host_flow_bytes && n <= 65535;
+    for (float* d : dst) pass = pass && (!d || pageable(d));
+    if (pass) {
+        CUDA_TRY(launch_flow_out(at(s->dx, offset), at(s->dy, offset), at(s->dz, offset), step, n, floats, s->status,
+                                 s->host_flow, s->host_status, s->stream),
+                 "flow read launch");
+        const int rc = status_end(s);
+        for (int a = 0; a < 3; ++a)
+            if (dst[a]) std::memcpy(dst[a], s->host_flow + a * floats * n, b * n);
+        return rc;
+    }
+    int rc = status_begin(s);
+    if (rc) return rc;
+    for (int a = 0; a < 3; ++a)
+        if (dst[a])
+            CUDA_TRY(cudaMemcpy2DAsync(dst[a], b, at(src[a], offset), step, b, n, cudaMemcpyDeviceToHost, s->stream),
+                     "D2H flow");
+    return status_end(s);
 }
 
 // Carves the arena: `batch` identical per-pair slices (pair k's buffers
@@ -613,6 +743,7 @@ int pdflow_create_batch(unsigned rows, unsigned width, unsigned height, const pd
         return set_error(PDFLOW_ERR_CUDA, "stream / arena init", e);
     }
     s->stream = s->own_stream;
+    create_host_buffers(s, size_t(rows) * cols * 12);
     *out = s;
     return PDFLOW_OK;
 }
@@ -634,6 +765,7 @@ int pdflow_destroy(pdflow_solver* s)
     if (s->sol_keep) cudaFree(s->sol_keep);
     if (s->lvl_keep) cudaFree(s->lvl_keep);
     cudaFree(s->arena);
+    destroy_host_buffers(s);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
     delete s;
     return PDFLOW_OK;
@@ -694,6 +826,9 @@ int pdflow_push_frames_u16(pdflow_solver* s, unsigned n, const uint8_t* intensit
     if (!s || !intensity || !depth) return set_error(PDFLOW_ERR_ARG, "null argument");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
     const size_t px = size_t(s->width) * s->height * n;
+    size_t second = 0;
+    if (const uint8_t* f = pass_frame(s, intensity, px, depth, px * 2, &second))
+        return frame_passed(s, pdflow_push_frames_u16_device(s, n, f, reinterpret_cast<const uint16_t*>(f + second)));
     CUDA_TRY(cudaMemcpyAsync(s->stage_u8, intensity, px, cudaMemcpyHostToDevice, s->stream), "H2D intensity");
     CUDA_TRY(cudaMemcpyAsync(s->stage_u16, depth, px * 2, cudaMemcpyHostToDevice, s->stream), "H2D depth");
     return pdflow_push_frames_u16_device(s, n, s->stage_u8, s->stage_u16);
@@ -761,11 +896,7 @@ int pdflow_read_flow_batch(pdflow_solver* s, unsigned n, float* dx, float* dy, f
     if (!s || !dx || !dy || !dz) return set_error(PDFLOW_ERR_ARG, "null argument");
     if (s->mixed) return set_error(PDFLOW_ERR_STATE, "a mixed-resolution handle: use the mixed calls");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
-    const size_t b = size_t(s->rows) * s->cols * 4;
-    CUDA_TRY(cudaMemcpy2DAsync(dx, b, s->dx, s->pair_stride, b, n, cudaMemcpyDeviceToHost, s->stream), "D2H dx");
-    CUDA_TRY(cudaMemcpy2DAsync(dy, b, s->dy, s->pair_stride, b, n, cudaMemcpyDeviceToHost, s->stream), "D2H dy");
-    CUDA_TRY(cudaMemcpy2DAsync(dz, b, s->dz, s->pair_stride, b, n, cudaMemcpyDeviceToHost, s->stream), "D2H dz");
-    return check_status(s);
+    return read_planes(s, 0, s->pair_stride, n, size_t(s->rows) * s->cols, dx, dy, dz);
 }
 
 int pdflow_read_flow(pdflow_solver* s, float* dx, float* dy, float* dz)
@@ -865,6 +996,10 @@ int pdflow_push_frames_slots_u16(pdflow_solver* s, unsigned n, const unsigned* s
     if (!s || !intensity || !depth) return set_error(PDFLOW_ERR_ARG, "null argument");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
     const size_t px = size_t(s->width) * s->height * n;
+    size_t second = 0;
+    if (const uint8_t* f = pass_frame(s, intensity, px, depth, px * 2, &second))
+        return frame_passed(s, pdflow_push_frames_slots_u16_device(s, n, slots, f,
+                                                                   reinterpret_cast<const uint16_t*>(f + second)));
     CUDA_TRY(cudaMemcpyAsync(s->stage_u8, intensity, px, cudaMemcpyHostToDevice, s->stream), "H2D intensity");
     CUDA_TRY(cudaMemcpyAsync(s->stage_u16, depth, px * 2, cudaMemcpyHostToDevice, s->stream), "H2D depth");
     return pdflow_push_frames_slots_u16_device(s, n, slots, s->stage_u8, s->stage_u16);
@@ -888,14 +1023,19 @@ int pdflow_read_flow_slots(pdflow_solver* s, unsigned n, const unsigned* slots, 
     if (!s || !slots || !dx || !dy || !dz) return set_error(PDFLOW_ERR_ARG, "null argument");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
     const size_t N = size_t(s->rows) * s->cols;
-    for (unsigned k = 0; k < n; ++k) {
+    for (unsigned k = 0; k < n; ++k)
         if (slots[k] >= s->batch) return set_error(PDFLOW_ERR_ARG, "slot out of range");
-        const size_t po = slots[k] * s->pair_stride;
-        CUDA_TRY(cudaMemcpyAsync(dx + k * N, at(s->dx, po), N * 4, cudaMemcpyDeviceToHost, s->stream), "D2H dx");
-        CUDA_TRY(cudaMemcpyAsync(dy + k * N, at(s->dy, po), N * 4, cudaMemcpyDeviceToHost, s->stream), "D2H dy");
-        CUDA_TRY(cudaMemcpyAsync(dz + k * N, at(s->dz, po), N * 4, cudaMemcpyDeviceToHost, s->stream), "D2H dz");
+    // runs of consecutive slots, a copy a plane each (every copy to pageable memory
+    // blocks for 10 us or more: six QVGA slots one by one took 314 us)
+    int rc = PDFLOW_OK;
+    for (unsigned k = 0; k < n;) {
+        unsigned m = 1;
+        while (k + m < n && slots[k + m] == slots[k] + m) ++m;
+        const int r = read_planes(s, slots[k] * s->pair_stride, s->pair_stride, m, N, dx + k * N, dy + k * N, dz + k * N);
+        if (rc == PDFLOW_OK) rc = r;
+        k += m;
     }
-    return check_status(s);
+    return rc;
 }
 
 int pdflow_energy_batch(pdflow_solver* s, unsigned n, float* energies)
