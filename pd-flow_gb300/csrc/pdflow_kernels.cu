@@ -449,6 +449,7 @@ __global__ void __launch_bounds__(kBlock) k_level_start(LevelGeom g, int start, 
 __global__ void __launch_bounds__(kBlock) k_level_warp(LevelGeom g, PyrLevel o, PyrLevel n, LevelConsts L, Params p,
                                                        int steps, size_t aux)
 {
+    allow_next_kernel();   // the streamed tiles: their CTAs start as these end, and wait there
     const size_t po = pair_off(g.map, g.pstride, blockIdx.y);
     o = at(o, po);
     n = at(n, po);

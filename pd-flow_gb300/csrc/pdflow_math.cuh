@@ -23,6 +23,15 @@
 
 namespace pdflow {
 
+// Programmatic dependent launch.  A kernel launched with that attribute starts
+// once every CTA of the kernel before it has allowed it (or ended); it touches
+// nothing that kernel reads or writes before after_previous_kernel(), which
+// returns when the kernel before it has ended and its writes are visible.  A CTA
+// allows the next kernel only after its own wait, so no kernel starts while the
+// last but one is running.  Both do nothing in a kernel launched without.
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }

@@ -348,12 +348,15 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
             if constexpr (kStrips) first = strip_at(a, blockIdx.x);
             else first = tile_at(a, blockIdx.x);
             desc = walk_region<kStrips>(a, first);
+            after_previous_kernel();
             if (first.more) issue_region(tm, sm, full, desc);
             else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full) : "memory");
         }
+        after_previous_kernel();
         __syncthreads();   // the mbarriers' initialisation before anyone waits on them
         if (t >= kSThreads) {
             asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSProducerRegs));
+            if (t == kSThreads) allow_next_kernel();
             if (t == kSThreads) produce<kStrips>(a, tm, sm, &desc, full, empty, first);
             return;
         }
@@ -737,11 +740,17 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
         !encode_plane_group(&maps.state, sg[0], 13, ss, g.R, g.C, g.slots, g.pstride, kSR, kSR) ||
         !encode_plane_group(&maps.consts, cg[0], 19, cs, g.R, g.C, g.slots, g.pstride, kSR, kSR))
         return cudaErrorInvalidValue;
-    if (strips)
-        k_iterate_stream<true><<<grid, kSThreads + kSProducer, stream_smem_bytes(), st>>>(a, maps);
-    else
-        k_iterate_stream<false><<<grid, kSThreads + kSProducer, stream_smem_bytes(), st>>>(a, maps);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kSThreads + kSProducer);
+    cfg.dynamicSmemBytes = stream_smem_bytes();
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, strips ? k_iterate_stream<true> : k_iterate_stream<false>, a, maps);
 }
 
 }  // namespace pdflow
