@@ -118,16 +118,17 @@ __device__ __forceinline__ void iterate_resident(const IterArgs& a, float* sm)
         wa = __ldcg(a.acc[0][2] + i);
         d = Duals{__ldcg(a.p_[0][0] + i), __ldcg(a.p_[0][1] + i), __ldcg(a.p_[0][2] + i), __ldcg(a.p_[0][3] + i),
                   __ldcg(a.p_[0][4] + i), __ldcg(a.p_[0][5] + i), __ldcg(a.p_[0][6] + i)};
-        spd = __ldg(L.spd + i); spuvx = __ldg(L.spuvx + i); spuvy = __ldg(L.spuvy + i);
-        spwx = __ldg(L.spwx + i); spwy = __ldg(L.spwy + i); mu = __ldg(L.mu + i); ddt = __ldg(L.ddt + i);
-        ddu = __ldg(L.ddu + i); ddv = __ldg(L.ddv + i); ri = __ldg(L.ri + i); rj = __ldg(L.rj + i);
-        ri_m = fu ? ri : __ldg(L.ri + i - R);
-        rj_m = fv ? rj : __ldg(L.rj + i - 1);
-        dup = __ldg(L.du_prev + i); dvp = __ldg(L.dv_prev + i);
-        dup_u = __ldg(L.du_prev + iu); dvp_u = __ldg(L.dv_prev + iu);
-        dup_v = __ldg(L.du_prev + iv); dvp_v = __ldg(L.dv_prev + iv);
-        tu = __ldg(L.tu + i); tv = __ldg(L.tv + i); tw = __ldg(L.tw + i);
-        dct = __ldg(L.dct + i); dcu = __ldg(L.dcu + i); dcv = __ldg(L.dcv + i);
+        // (plain loads: the set-up may write these planes while this kernel starts)
+        spd = L.spd[i]; spuvx = L.spuvx[i]; spuvy = L.spuvy[i];
+        spwx = L.spwx[i]; spwy = L.spwy[i]; mu = L.mu[i]; ddt = L.ddt[i];
+        ddu = L.ddu[i]; ddv = L.ddv[i]; ri = L.ri[i]; rj = L.rj[i];
+        ri_m = fu ? ri : L.ri[i - R];
+        rj_m = fv ? rj : L.rj[i - 1];
+        dup = L.du_prev[i]; dvp = L.dv_prev[i];
+        dup_u = L.du_prev[iu]; dvp_u = L.dv_prev[iu];
+        dup_v = L.du_prev[iv]; dvp_v = L.dv_prev[iv];
+        tu = L.tu[i]; tv = L.tv[i]; tw = L.tw[i];
+        dct = L.dct[i]; dcu = L.dcu[i]; dcv = L.dcv[i];
     }
     for (unsigned t = 0; t < a.iters; ++t) {
         // ---- dual step ----
@@ -178,6 +179,8 @@ template <int kMode>
 __global__ void __launch_bounds__(kMode == kIterSingle ? kSingleThreads : kIterThreads, 1) k_iterate(IterArgs a)
 {
     extern __shared__ float sm[];
+    after_previous_kernel();
+    allow_next_kernel();
     if (a.g.map || (kMode != kIterGrid && blockIdx.y > 0)) {
         // batch: the pair of grid row y (the grid form solves one pair) of a strided arena
         const size_t po = pair_off(a.g.map, a.g.pstride, kMode == kIterGrid ? 0u : blockIdx.y);
@@ -483,6 +486,11 @@ cudaError_t launch_iterate(const IterPlan& pl, IterArgs a, cudaStream_t st)
         attr[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, k_iterate<kIterCluster>, a);
+    }
+    if (a.g.N <= single) {   // iterate_resident, whose loads may follow the kernel before at once
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 1;
     }
     return cudaLaunchKernelEx(&cfg, k_iterate<kIterSingle>, a);
 }

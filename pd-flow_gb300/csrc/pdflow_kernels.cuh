@@ -5,6 +5,24 @@
 
 namespace pdflow {
 
+// Launches a kernel that may start while the one before it in the stream ends
+// (after_previous_kernel in it waits for that; see pdflow_math.cuh).
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
+}
+
 // One pyramid level of one frame (column-major planes of R*C floats).
 struct PyrLevel {
     float* col;

@@ -740,17 +740,8 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
         !encode_plane_group(&maps.state, sg[0], 13, ss, g.R, g.C, g.slots, g.pstride, kSR, kSR) ||
         !encode_plane_group(&maps.consts, cg[0], 19, cs, g.R, g.C, g.slots, g.pstride, kSR, kSR))
         return cudaErrorInvalidValue;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kSThreads + kSProducer);
-    cfg.dynamicSmemBytes = stream_smem_bytes();
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, strips ? k_iterate_stream<true> : k_iterate_stream<false>, a, maps);
+    return launch_overlapped(strips ? k_iterate_stream<true> : k_iterate_stream<false>, dim3(grid),
+                             dim3(kSThreads + kSProducer), stream_smem_bytes(), st, a, maps);
 }
 
 }  // namespace pdflow

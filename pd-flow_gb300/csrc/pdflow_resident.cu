@@ -93,9 +93,11 @@ __global__ void __launch_bounds__(kLanes* kCols) k_iterate_resident(const __grid
             : "r"(smem_u32(edge)), "r"((unsigned)ov + (unsigned)ou * a.tiles_v));
 
     const float2 zero = make_float2(0.f, 0.f);
-    auto plane = [&](const float* q) {
-        return live ? __ldg(reinterpret_cast<const float2*>(at(q, po) + gi)) : zero;
+    auto plane = [&](const float* q) {   // plain loads: the kernel before may write them while this one starts
+        return live ? *reinterpret_cast<const float2*>(at(q, po) + gi) : zero;
     };
+    after_previous_kernel();
+    allow_next_kernel();
     const PairConsts k{plane(a.consts[0]),  plane(a.consts[1]),  plane(a.consts[2]),  plane(a.consts[3]),
                        plane(a.consts[4]),  plane(a.consts[5]),  plane(a.consts[6]),  plane(a.consts[7]),
                        plane(a.consts[8]),  plane(a.consts[9]),  plane(a.consts[10]), plane(a.consts[11]),
@@ -229,13 +231,15 @@ cudaError_t launch_iterate_resident(LevelGeom g, LevelConsts L, State src, State
     cfg.blockDim = dim3(unsigned(s.threads));
     cfg.dynamicSmemBytes = s.smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = a.tiles;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
     void* args[] = {&a};
     return cudaLaunchKernelExC(&cfg, s.kernel, args);
 }
