@@ -109,6 +109,7 @@ __device__ __forceinline__ void iterate_resident(const IterArgs& a, float* sm)
     float spd = 0.f, spuvx = 0.f, spuvy = 0.f, spwx = 0.f, spwy = 0.f, mu = 0.f, ddt = 0.f, ddu = 0.f, ddv = 0.f;
     float ri = 0.f, rj = 0.f, ri_m = 0.f, rj_m = 0.f, dup = 0.f, dvp = 0.f, dup_u = 0.f, dvp_u = 0.f, dup_v = 0.f,
           dvp_v = 0.f, tu = 0.f, tv = 0.f, tw = 0.f, dct = 0.f, dcu = 0.f, dcv = 0.f;
+    const unsigned iters = a.pair_iters ? __ldg(a.pair_iters + blockIdx.y) : a.iters;
     if (live) {
         du = a.du[i];
         dv = a.dv[i];
@@ -130,7 +131,7 @@ __device__ __forceinline__ void iterate_resident(const IterArgs& a, float* sm)
         tu = L.tu[i]; tv = L.tv[i]; tw = L.tw[i];
         dct = L.dct[i]; dcu = L.dcu[i]; dcv = L.dcv[i];
     }
-    for (unsigned t = 0; t < a.iters; ++t) {
+    for (unsigned t = 0; t < iters; ++t) {
         // ---- dual step ----
         if (live) {
             xa[i] = ua;
@@ -159,16 +160,16 @@ __device__ __forceinline__ void iterate_resident(const IterArgs& a, float* sm)
                                           fv, lv);
             primal_update(du, dv, dw, ua, va, wa, tu, tv, tw, mu, ddu, ddv, d.pd, li, ld, divu, divv, divw, dct, dcu,
                           dcv);
-            if (t + 1 == a.iters) saturate(du, dv, dw, dup, dvp, __ldg(a.depth_old + i));
+            if (t + 1 == iters) saturate(du, dv, dw, dup, dvp, __ldg(a.depth_old + i));
         }
     }
     // final state for the weighted median, the duals to buffer (iters & 1),
-    // as the general loop leaves them
+    // as the general loop leaves them (buffer 0 where the pairs' counts differ)
     if (live) {
         a.du[i] = du;
         a.dv[i] = dv;
         a.dw[i] = dw;
-        const bool fb = a.iters & 1;
+        const bool fb = !a.pair_iters && (iters & 1u);
         const float pn[7] = {d.pd, d.puu, d.puv, d.pvu, d.pvv, d.pwu, d.pwv};
 #pragma unroll
         for (int k = 0; k < 7; ++k) (fb ? a.p_[1][k] : a.p_[0][k])[i] = pn[k];
@@ -460,6 +461,7 @@ cudaError_t launch_wait_probe(unsigned* flags, unsigned* status, unsigned polls,
 
 cudaError_t launch_iterate(const IterPlan& pl, IterArgs a, cudaStream_t st)
 {
+    if (a.pair_iters && (pl.mode != kIterSingle || a.g.N > kSingleThreads)) return cudaErrorInvalidValue;
     a.smem_plane = pl.smem_plane;
     a.smem_state_plane = pl.smem_state_plane;
     cudaLaunchConfig_t cfg = {};

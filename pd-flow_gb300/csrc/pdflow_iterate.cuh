@@ -20,6 +20,8 @@ struct IterArgs {
     Params p;
     const float* depth_old;       // old frame depth at this level (saturation)
     unsigned iters;
+    const unsigned* pair_iters;   // iterations of each pair of a level that fits a CTA, whose duals then end in
+                                  // buffer 0 (null: iters, and duals in buffer iters & 1)
     unsigned* flags;              // per-CTA completed-iteration counters (grid form)
     unsigned* status;             // 0, or kStatusTimeout after a bounded wait gave up
     unsigned smem_plane;          // floats per shared plane of new duals (set by launch_iterate)
@@ -103,7 +105,8 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
 bool resident_eligible(const LevelGeom& g, const LevelConsts& L, const State& src, const State& dst, unsigned sms);
 cudaError_t prepare_resident();
 cudaError_t launch_iterate_resident(LevelGeom g, LevelConsts L, State src, State dst, Params p,
-                                    const float* depth_old, unsigned iters, cudaStream_t st);
+                                    const float* depth_old, unsigned iters, cudaStream_t st,
+                                    const unsigned* pair_iters = nullptr);
 // L2 prefetch distance of the quad tiles in CTAs (0 = off).
 void set_quad_prefetch(unsigned ctas_ahead);
 size_t quads_smem_bytes();

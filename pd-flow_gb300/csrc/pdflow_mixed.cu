@@ -40,8 +40,8 @@ unsigned levels_of(unsigned rows)
 bool is_rows(unsigned r) { return r == 15 || r == 30 || r == 60 || r == 120 || r == 240 || r == 480; }
 
 struct LaunchRec {
-    int kind;            // 0 set-up (init, gradients, warp), 1 tiles, 2 median
-    unsigned step, kk, off, count;
+    int kind;            // 0 set-up (init, gradients, warp), 1 tiles, 2 median, 3 all iterations
+    unsigned step, kk, off, count;   // kind 3: the pairs' iterations follow the slot map
 };
 
 // Iterations per tile launch at step i in form `form` (the autotuned choice,
@@ -56,7 +56,7 @@ unsigned step_kk(const pdflow_solver* s, unsigned i, int form)
 // (forms 7 and 10 need rows % 4 == 0, forms 8 and 9 even rows; the 15x20
 // level runs form 5; by default the strips, form 10, need a strip per SM and
 // rows % 4 == 0, else form 8 runs, or form 9 where the 16x16 tiles fit in one
-// round of CTAs).
+// round of CTAs).  Steps that run whole (step_whole) have no tiles.
 int step_form(const pdflow_solver* s, unsigned i, const LevelGeom& g)
 {
     int f = s->mixed_form[i] >= 3 ? s->mixed_form[i] : (s->iter_form >= 3 ? s->iter_form : 5);
@@ -76,6 +76,29 @@ LevelGeom step_geom(const pdflow_solver* s, unsigned step, unsigned pairs, const
     return g;
 }
 
+// Whether the iterations at step i run as one launch, each pair's own count in
+// it: 9 as resident tiles (where form 9 was chosen, or the handle's forms are the
+// default, and the level fits a cluster), 1 as a CTA per pair (15x20, not tuned),
+// 0 not.  As tiles, pairs of different schedules are a launch per 1-4 iterations, 67
+// launches at the three smallest steps: 16 pairs of rows 60 to 480 solve in 3.99 ms,
+// as whole launches in 3.80.
+int step_whole(const pdflow_solver* s, unsigned i, const LevelGeom& g)
+{
+    const bool chosen = s->mixed_form[i] >= 3;
+    if (chosen ? s->mixed_form[i] != 9 : s->iter_form < 9) return 0;
+    if (g.N <= 300u) return chosen ? 0 : 1;
+    return resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms)) ? 9 : 0;
+}
+
+// The step-size planes the set-up writes at step i.
+int step_planes(const pdflow_solver* s, unsigned i, const LevelGeom& g, bool all_steps)
+{
+    if (all_steps) return kStepsAll;
+    const int whole = step_whole(s, i, g);
+    if (whole == 1) return kStepsRaw;
+    return whole == 9 || step_form(s, i, g) >= 7 ? kStepsQuads : kStepsNone;
+}
+
 // kk iterations of the pairs of `g` in form `form`, state from cur to nxt.
 cudaError_t launch_step_tiles(pdflow_solver* s, const LevelGeom& g, const State& cur, const State& nxt,
                               const Params& p, const PyrLevel& o, unsigned kk, cudaStream_t st, int form)
@@ -85,6 +108,32 @@ cudaError_t launch_step_tiles(pdflow_solver* s, const LevelGeom& g, const State&
                                      stream_layout(form));
     if (form == 7) return launch_iterate_quads(g, s->L, cur, nxt, p, o.dep, kk, false, st, s->status);
     return launch_iterate_tiles2(g, s->L, cur, nxt, p, o.dep, kk, false, st, form - 3, s->status);
+}
+
+// All iterations of the pairs of `g` in one launch: `most` at most, pair k's
+// pair_iters[k].  Resident tiles leave the state in the second buffers, a CTA per
+// pair in the first.
+cudaError_t launch_step_whole(pdflow_solver* s, const LevelGeom& g, const State& alt, const Params& p, const PyrLevel& o,
+                              unsigned most, const unsigned* pair_iters, cudaStream_t st, int whole)
+{
+    if (whole == 9) return launch_iterate_resident(g, s->L, s->S, alt, p, o.dep, most, st, pair_iters);
+    IterArgs a{};
+    a.g = g;
+    a.L = s->L;
+    a.du = s->S.du;
+    a.dv = s->S.dv;
+    a.dw = s->S.dw;
+    float* acc[3] = {s->S.dua, s->S.dva, s->S.dwa};
+    float* duals[7] = {s->S.pd, s->S.puu, s->S.puv, s->S.pvu, s->S.pvv, s->S.pwu, s->S.pwv};
+    for (int k = 0; k < 3; ++k) a.acc[0][k] = a.acc[1][k] = acc[k];
+    for (int k = 0; k < 7; ++k) a.p_[0][k] = a.p_[1][k] = duals[k];
+    a.p = p;
+    a.depth_old = o.dep;
+    a.iters = most;
+    a.pair_iters = pair_iters;
+    a.flags = s->flags;
+    a.status = s->status;
+    return launch_iterate(plan_iterate(g, s->num_sms), a, st);
 }
 
 // The launches of a solve and their slot maps (flags in the high bits).
@@ -103,6 +152,15 @@ void build_plan(const pdflow_solver* s, const std::vector<unsigned>& rows, std::
         table.insert(table.end(), act.begin(), act.end());
         std::vector<unsigned> remaining(act.size()), launches(act.size(), 0);
         for (size_t a = 0; a < act.size(); ++a) remaining[a] = 100u - 15u * (levels_of(rows[act[a]]) - 1u - i);
+        const int whole = step_whole(s, i, step_geom(s, i, unsigned(act.size()), nullptr));
+        if (whole) {
+            plan.push_back({3, i, *std::max_element(remaining.begin(), remaining.end()), unsigned(table.size()),
+                            unsigned(act.size())});
+            table.insert(table.end(), act.begin(), act.end());
+            table.insert(table.end(), remaining.begin(), remaining.end());
+            std::fill(remaining.begin(), remaining.end(), 0u);
+            std::fill(launches.begin(), launches.end(), whole == 9 ? 1u : 0u);
+        }
         const unsigned step_k = step_kk(s, i, step_form(s, i, step_geom(s, i, unsigned(act.size()), nullptr)));
         for (;;) {
             unsigned kk = step_k, live = 0;
@@ -180,17 +238,20 @@ int enqueue_mixed(pdflow_solver* s, cudaStream_t st, const std::vector<LaunchRec
             e = launch_im_gradients(&g, &n, &aux, 1, s->L, st);
             if (e == cudaSuccess)
                 e = launch_level_setup(g, r.step == 0 ? LevelStart::Zeros : LevelStart::Coarse, s->sol, o, n, s->L,
-                                       s->S, p, all_steps ? kStepsAll : (form >= 7 ? kStepsQuads : kStepsNone), aux, st);
+                                       s->S, p, step_planes(s, r.step, g, all_steps), aux, st);
             *count += 3;
             cur = s->S;
             nxt = alt;
+        } else if (r.kind == 3) {
+            e = launch_step_whole(s, g, alt, p, o, r.kk, g.map + r.count, st, step_whole(s, r.step, g));
+            *count += 1;
         } else if (r.kind == 1) {
             e = launch_step_tiles(s, g, cur, nxt, p, o, r.kk, st, form);
             std::swap(cur, nxt);
             *count += 1;
         } else {
             e = launch_median(g, false, o, s->L, s->S, s->sol, s->dx, s->dy, s->dz, p, nullptr, st, &alt,
-                              !all_steps);
+                              steps_hold_ddt_sq(step_planes(s, r.step, g, all_steps)));
             *count += 1;
         }
         if (e != cudaSuccess) return set_error_code(PDFLOW_ERR_CUDA, "mixed batch launch", e);
@@ -250,7 +311,12 @@ int pdflow::mixed_autotune(pdflow_solver* s, unsigned n, unsigned probe_iters, p
                 for (int r = 0; r < 4 && rc == PDFLOW_OK; ++r) {
                     cudaEventRecord(e0, s->stream);
                     State cur = s->S, nxt = alt;
-                    for (unsigned done = 0; done < probe_iters;) {
+                    const bool whole = form == 9 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms));
+                    if (whole) {   // what form 9 then runs
+                        const cudaError_t e = launch_step_whole(s, g, alt, p, o, probe_iters, nullptr, s->stream, 9);
+                        if (e != cudaSuccess) rc = set_error_code(PDFLOW_ERR_CUDA, "mixed autotune launch", e);
+                    }
+                    for (unsigned done = whole ? probe_iters : 0; done < probe_iters;) {
                         const unsigned k = std::min(kk, probe_iters - done);
                         const cudaError_t e = launch_step_tiles(s, g, cur, nxt, p, o, k, s->stream, form);
                         if (e != cudaSuccess) {

@@ -40,6 +40,7 @@ struct ResidentArgs {
     const float* depth_old;
     float lambda_i, lambda_d;
     unsigned iters;
+    const unsigned* pair_iters;   // iterations of each pair (null: iters)
     unsigned tiles_v, tiles;   // tiles per column of tiles, per pair (= the cluster's CTAs)
 };
 
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(kLanes* kCols) k_iterate_resident(const __grid
     auto plane = [&](const float* q) {   // plain loads: the kernel before may write them while this one starts
         return live ? *reinterpret_cast<const float2*>(at(q, po) + gi) : zero;
     };
+    const unsigned iters = a.pair_iters ? __ldg(a.pair_iters + y) : a.iters;   // the same for the whole cluster
     after_previous_kernel();
     allow_next_kernel();
     const PairConsts k{plane(a.consts[0]),  plane(a.consts[1]),  plane(a.consts[2]),  plane(a.consts[3]),
@@ -118,12 +120,12 @@ __global__ void __launch_bounds__(kLanes* kCols) k_iterate_resident(const __grid
     // after the barrier of x + 1, which every CTA reaches after reading x.
     unsigned buffer = 0;
     for (unsigned done = 0;; buffer ^= 1u) {
-        const unsigned kk = min(a.iters - done, (unsigned)kHalo);
+        const unsigned kk = min(iters - done, (unsigned)kHalo);
         for (unsigned j = 0; j < kk; ++j)
             iterate_pair<true, kLanes, false>(s, k, d, X, Y, T::kPlane, me, right, place, a.lambda_i, a.lambda_d,
                                        Hooks{Y + left});
         done += kk;
-        if (done >= a.iters) break;
+        if (done >= iters) break;
         if (ring) {
             const float2 st[13] = {s.du, s.dv, s.dw, s.ua, s.va, s.wa, s.pd, s.puu, s.puv, s.pvu, s.pvv, s.pwu, s.pwv};
 #pragma unroll
@@ -201,7 +203,8 @@ cudaError_t prepare_resident()
 }
 
 cudaError_t launch_iterate_resident(LevelGeom g, LevelConsts L, State src, State dst, Params p,
-                                    const float* depth_old, unsigned iters, cudaStream_t st)
+                                    const float* depth_old, unsigned iters, cudaStream_t st,
+                                    const unsigned* pair_iters)
 {
     if (iters == 0 || reinterpret_cast<uintptr_t>(depth_old) % 8u != 0 || !shape_for(g) ||
         !stream_direct_eligible(g, L, src, dst))
@@ -224,6 +227,7 @@ cudaError_t launch_iterate_resident(LevelGeom g, LevelConsts L, State src, State
     a.lambda_i = p.lambda_i;
     a.lambda_d = p.lambda_d;
     a.iters = iters;
+    a.pair_iters = pair_iters;
     a.tiles_v = (g.R + s.rows - 1) / s.rows;
     a.tiles = shape_tiles(s, g);
     cudaLaunchConfig_t cfg = {};
