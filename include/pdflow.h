@@ -235,7 +235,9 @@ int pdflow_read_flow_mixed(pdflow_solver* s, unsigned k, float* dx, float* dy, f
  * registers while the next region streams into shared memory by TMA (levels
  * with rows % 4 == 0; other even row counts load each pixel pair directly);
  * form 9: the same with 16x16 interiors and a halo of 8,
- * up to 8 iterations per launch, for levels whose launches are latency-bound;
+ * up to 8 iterations per launch, for levels whose launches are latency-bound, or,
+ * at 30x40 and (up to about 20 pairs) 60x80, all the level's iterations in one
+ * launch with a thread-block cluster per pair;
  * form 10: rows of regions walked left to right, each handing the next its
  * last exact column's exchange values, so no left halo is recomputed; levels
  * with rows % 4 == 0).
@@ -245,7 +247,7 @@ int pdflow_read_flow_mixed(pdflow_solver* s, unsigned k, float* dx, float* dy, f
  * handle's solution state is overwritten (the pushed frames are kept).  On a
  * mixed-resolution handle (pdflow_create_mixed) it tunes per coarse-to-fine
  * step (report level i = the 15*2^i x 20*2^i step) over the pairs active at
- * that step, among the tile forms 3..8 (2, 3 or 4 iterations per launch);
+ * that step, among the tile forms 3..10;
  * pdflow_solve_mixed then runs each step in its chosen form. */
 #define PDFLOW_TUNE_CANDIDATES 29     /* form 0, form 1, forms 2..8 x {2, 3, 4}, form 9 x {4, 6, 8}, form 10 x {2, 3, 4} */
 typedef struct pdflow_tune_level {

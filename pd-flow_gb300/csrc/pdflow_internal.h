@@ -51,8 +51,8 @@ struct pdflow_solver {
     float* host_flow = nullptr;
     size_t host_flow_bytes = 0;
     int num_sms = 0;
-    int iter_form = 10;                  // 10 = streamed strips (levels with a strip per SM; others 9 or 8),
-                                         // 9 = deep streamed tiles,
+    int iter_form = 10;                  // 10 = chosen by the level (default_level_form): streamed strips, 8 or 9,
+                                         // 9 = resident tiles (small levels) or deep streamed tiles,
                                          // 8 = streamed register tiles (persistent, one CTA per SM), 7 = quad
                                          // register tiles, 5 / 4 / 3 = paired tiles 24x24 (two CTAs per SM) / 40x34 / 40x40,
                                          // 2 = scalar tiles for large levels,

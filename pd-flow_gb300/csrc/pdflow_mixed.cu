@@ -14,7 +14,8 @@
 // launch choice), uploaded as one table, and the solve is replayed as one CUDA
 // graph.  Each step's iterations run in the tile form and iterations per
 // launch that pdflow_autotune picked for it over the pairs active at that step
-// (mixed_autotune), by default the handle's paired tiles with 4 iterations.
+// (mixed_autotune), by default the handle's form with its halo's iterations; the
+// smallest steps run as one launch with a count per pair (step_whole).
 #include <cuda_runtime.h>
 
 #include <algorithm>
