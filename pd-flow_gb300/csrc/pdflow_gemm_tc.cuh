@@ -54,7 +54,14 @@ cudaError_t launch_conv_dgrad(const void* dy, const void* wt, int P, int H, int 
 unsigned gemm_splits(int K, int k_per_split);
 // Sums the partials of a split GEMM in order into out [M][ldc], or with ldt > 0
 // into its transpose [N][ldt].
+// `bias` (part not null): besides, in the same launch, the channel sums of the
+// partials [nblocks][C] into out[cout].
+struct BiasSum {
+    const float* part = nullptr;
+    int nblocks = 0, C = 0, cout = 0;
+    float* out = nullptr;
+};
 cudaError_t launch_splitk_sum(const float* part, int splits, size_t stride, int M, int N, int ldc, float* out,
-                              cudaStream_t st, int ldt = 0);
+                              cudaStream_t st, int ldt = 0, BiasSum bias = BiasSum());
 
 }  // namespace pdflow

@@ -187,7 +187,7 @@ __global__ void k_pool_grad(const float* __restrict__ dy, int C, int n, int H, i
 // and the column sums of the rounded dY [P][C] (the bias gradient) in the same
 // pass: a thread owns eight channels (one 16-byte piece) of every rows-th row
 // of its block's share, the block adds its threads in a fixed tree and writes
-// one partial sum a channel; k_bias_sum adds the blocks in order.  Bound by
+// one partial sum a channel; k_splitk_sum adds the blocks.  Bound by
 // memory (dA 4 B, A 2 B, dY 2 B a value).  Separate sums, a block per channel
 // striding through dY two bytes at a time, took 2.78 of the 8.3 ms of a
 // 64-input gradient on a GB300; this pass takes over the dY kernel's 0.14 ms.
@@ -234,24 +234,6 @@ __global__ void __launch_bounds__(kSumThreads) k_relu_grad(const float* __restri
         __syncthreads();
     }
     for (int c = threadIdx.x; c < C; c += kSumThreads) part[(size_t)blockIdx.x * C + c] = red[c / 8][c % 8];
-}
-
-// The blocks' partial sums of k_relu_grad, added per channel: 16 warps a
-// channel block of 32 take every 16th partial, then a fixed tree.
-__global__ void __launch_bounds__(512) k_bias_sum(const float* __restrict__ part, int nblocks, int C, int cout,
-                                                  float* __restrict__ out)
-{
-    __shared__ float red[16][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
-    float s = 0.f;
-    if (c < C)
-        for (int b = threadIdx.y; b < nblocks; b += 16) s += part[(size_t)b * C + c];
-    red[threadIdx.y][threadIdx.x] = s;
-    for (int w = 8; w > 0; w >>= 1) {
-        __syncthreads();
-        if ((int)threadIdx.y < w) red[threadIdx.y][threadIdx.x] += red[threadIdx.y + w][threadIdx.x];
-    }
-    if (threadIdx.y == 0 && c < cout) out[c] = red[0][threadIdx.x];
 }
 
 // Masked mean-squared error of the head output [P][16] against labels
@@ -395,7 +377,7 @@ struct pdflow_net {
     float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;   // fp32 [nparams]
     std::vector<__nv_bfloat16*> Wb, WTb;                               // per conv bf16 weights
     __nv_bfloat16 *col = nullptr, *dy = nullptr;
-    float *dcat = nullptr, *head = nullptr, *dhead = nullptr, *part = nullptr;
+    float *dcat = nullptr, *head = nullptr, *dhead = nullptr, *part = nullptr, *bias_part = nullptr;
     float *loss_part = nullptr, *input = nullptr;
     unsigned* count = nullptr;
     unsigned* status = nullptr;
@@ -684,11 +666,8 @@ int backward(pdflow_net* n, int nb)
         const unsigned srows = unsigned(kSumThreads / (c.cout_pad / 8));
         const unsigned nsum = std::min(kSumBlocks, unsigned((P + srows - 1) / srows));
         k_relu_grad<<<nsum, kSumThreads, 0, st>>>(c.relu ? o.g : n->dhead, c.relu ? o.x : nullptr, P, c.cout_pad,
-                                                  n->dy, n->part);
+                                                  n->dy, n->bias_part);
         NET_TRY(cudaGetLastError(), "relu grad launch");
-        k_bias_sum<<<unsigned((c.cout_pad + 31) / 32), dim3(32, 16), 0, st>>>(n->part, int(nsum), c.cout_pad, c.cout,
-                                                                             n->grad + c.boff);
-        NET_TRY(cudaGetLastError(), "bias grad launch");
         // weight gradient: dW^T [K][cout_pad] = im2col^T [K][P] * dY [P][cout_pad], both
         // operands gathered as they lie (no im2col matrix, no transposed copies)
         {
@@ -718,8 +697,8 @@ int backward(pdflow_net* n, int nb)
             if (size_t(splits) * g.split_stride > n->part_elems) return net_fail(PDFLOW_ERR_ARG, "split-K buffer");
             NET_TRY(launch_gemm_tc(g, st), "weight-gradient GEMM launch");
             NET_TRY(launch_splitk_sum(n->part, int(splits), g.split_stride, K, c.cout, c.cout_pad, n->grad + c.woff, st,
-                                      K),
-                    "split-K sum launch");
+                                      K, BiasSum{n->bias_part, int(nsum), c.cout_pad, c.cout, n->grad + c.boff}),
+                    "split-K and bias sum launch");
         }
         if (ci == 0) break;   // no gradient w.r.t. the input
         // input gradient of the concatenated sources
@@ -867,6 +846,7 @@ int pdflow_net_create(unsigned max_batch, unsigned long long seed, pdflow_net** 
     n->dhead = dalloc<float>(n, B * kHW * 16, &e);
     n->part_elems = 300 * maxK;
     n->part = dalloc<float>(n, n->part_elems, &e);
+    n->bias_part = dalloc<float>(n, size_t(kSumBlocks) * 96, &e);
     n->loss_part = dalloc<float>(n, B * kHW / 256 + 2, &e);
     n->input = dalloc<float>(n, B * 4 * kHW, &e);
     n->count = dalloc<unsigned>(n, 4, &e);
