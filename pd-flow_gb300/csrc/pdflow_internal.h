@@ -46,6 +46,7 @@ struct pdflow_solver {
     unsigned* host_status = nullptr;
     uint8_t* host_frames[2] = {};
     size_t host_frame_bytes = 0;
+    bool host_frame_tried = false;
     cudaEvent_t host_frame_read[2] = {}; // the device has read the frame buffer
     int host_frame_next = 0;
     float* host_flow = nullptr;
@@ -164,6 +165,7 @@ int check_status(pdflow_solver* s);
 // check_status in two halves: status_begin before the copies of a result (they
 // may block on the host), status_end after them.
 void create_host_buffers(pdflow_solver* s, size_t flow);
+void create_frame_buffers(pdflow_solver* s);
 void destroy_host_buffers(pdflow_solver* s);
 int status_begin(pdflow_solver* s);
 int status_end(pdflow_solver* s);

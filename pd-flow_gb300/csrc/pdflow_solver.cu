@@ -126,40 +126,55 @@ int check_status(pdflow_solver* s)
 // 60x80 (58 KB): 40 -> 21 us; at 240x320 (922 KB): 48 -> 75.  The limits lie between.
 constexpr size_t kHostFrameLimit = 256u << 10, kHostFlowLimit = 256u << 10;
 
-// For results of `flow` bytes and more; up to 0.1 ms of a handle's creation
-// (pinned pages come 2 MB at a time).  Best effort: without the memory (or
-// where nothing would pass through it) transfers are direct.
+// The status word and a result buffer for flows of `flow` bytes and more, and for
+// a single pair's handle the frame buffers (a batch's on its first push that fits
+// one).  Best effort: without the memory (or where nothing would pass through it)
+// transfers are direct.
 void create_host_buffers(pdflow_solver* s, size_t flow)
 {
-    const size_t frame = size_t(s->width) * s->height * 3 + 256;   // uint8 intensity and uint16 depth
-    const size_t fcap = frame <= kHostFrameLimit ? frame : 0;
-    const size_t ocap = flow <= kHostFlowLimit ? std::min(flow * s->batch, kHostFlowLimit) : 0;
+    const size_t cap = flow <= kHostFlowLimit ? std::min(flow * s->batch, kHostFlowLimit) : 0;
     void* p = nullptr;
-    if (cudaHostAlloc(&p, 256 + 2 * ((fcap + 255) & ~size_t(255)) + ocap, cudaHostAllocDefault) != cudaSuccess) {
+    if (cudaHostAlloc(&p, 256 + cap, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
     s->host_status = static_cast<unsigned*>(p);
-    uint8_t* q = static_cast<uint8_t*>(p) + 256;
-    if (fcap && cudaEventCreateWithFlags(&s->host_frame_read[0], cudaEventDisableTiming) == cudaSuccess &&
-        cudaEventCreateWithFlags(&s->host_frame_read[1], cudaEventDisableTiming) == cudaSuccess) {
-        for (int k = 0; k < 2; ++k) s->host_frames[k] = q + k * ((fcap + 255) & ~size_t(255));
-        s->host_frame_bytes = fcap;
-    } else {
+    s->host_flow = reinterpret_cast<float*>(static_cast<uint8_t*>(p) + 256);
+    s->host_flow_bytes = cap;
+    if (s->batch == 1) create_frame_buffers(s);
+}
+
+void create_frame_buffers(pdflow_solver* s)
+{
+    const size_t frame = size_t(s->width) * s->height * 3 + 256;   // uint8 intensity and uint16 depth
+    if (s->host_frame_tried || frame > kHostFrameLimit) return;
+    s->host_frame_tried = true;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, 2 * kHostFrameLimit, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
+        return;
     }
-    s->host_flow = reinterpret_cast<float*>(q + 2 * ((fcap + 255) & ~size_t(255)));
-    s->host_flow_bytes = ocap;
+    s->host_frames[0] = static_cast<uint8_t*>(p);
+    s->host_frames[1] = s->host_frames[0] + kHostFrameLimit;
+    if (cudaEventCreateWithFlags(&s->host_frame_read[0], cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&s->host_frame_read[1], cudaEventDisableTiming) == cudaSuccess)
+        s->host_frame_bytes = frame;
+    else
+        cudaGetLastError();
 }
 
 void destroy_host_buffers(pdflow_solver* s)
 {
-    for (cudaEvent_t e : s->host_frame_read)
+    for (cudaEvent_t& e : s->host_frame_read) {
         if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+    if (s->host_frames[0]) cudaFreeHost(s->host_frames[0]);
     if (s->host_status) cudaFreeHost(s->host_status);
+    s->host_frames[0] = s->host_frames[1] = nullptr;
     s->host_status = nullptr;
-    for (cudaEvent_t& e : s->host_frame_read) e = nullptr;
     s->host_frame_bytes = s->host_flow_bytes = 0;
+    s->host_frame_tried = false;
 }
 
 // Ordinary host memory (neither pinned nor managed: work on the stream may still
@@ -174,19 +189,32 @@ bool pageable(const void* p)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
+// Another thread's capture in global mode forbids this thread the waits and
+// allocations that a capture of its own would record wrongly; these are none.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
 // Copies a frame's two images into the next frame buffer; null where it goes
 // directly (size, memory, or a capture, which has to record the caller's address).
 // frame_passed() follows once the kernels that read it are enqueued.
 uint8_t* pass_frame(pdflow_solver* s, const void* a, size_t na, const void* b, size_t nb, size_t* second)
 {
     *second = (na + 255) & ~size_t(255);
-    if (*second + nb > s->host_frame_bytes) return nullptr;
+    if (*second + nb > (s->host_frame_tried ? s->host_frame_bytes : kHostFrameLimit)) return nullptr;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return nullptr;
     }
     if (!pageable(a) || !pageable(b)) return nullptr;
+    const RelaxedCapture relaxed;
+    create_frame_buffers(s);
+    if (*second + nb > s->host_frame_bytes) return nullptr;
     if (cudaEventSynchronize(s->host_frame_read[s->host_frame_next]) != cudaSuccess) return nullptr;
     uint8_t* dst = s->host_frames[s->host_frame_next];
     std::memcpy(dst, a, na);
