@@ -95,9 +95,10 @@ inline StreamLayout stream_layout(int form)
 }
 cudaError_t prepare_stream_tiles();
 size_t stream_smem_bytes();
+// follows: the kernel before in the stream is a launch of the same level's tiles.
 cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State dst, Params p, const float* depth_old,
                                   unsigned kk, bool last, cudaStream_t st, unsigned* status, unsigned ctas,
-                                  StreamLayout layout);
+                                  StreamLayout layout, bool follows = false);
 // Resident tiles (pdflow_resident.cu): every iteration of a small level in one
 // launch, a cluster per pair with a tile per CTA (the deep tiles' form, 9,
 // where the level fits a cluster); same preconditions as the streamed tiles

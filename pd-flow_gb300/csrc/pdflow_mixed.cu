@@ -102,11 +102,12 @@ int step_planes(const pdflow_solver* s, unsigned i, const LevelGeom& g, bool all
 
 // kk iterations of the pairs of `g` in form `form`, state from cur to nxt.
 cudaError_t launch_step_tiles(pdflow_solver* s, const LevelGeom& g, const State& cur, const State& nxt,
-                              const Params& p, const PyrLevel& o, unsigned kk, cudaStream_t st, int form)
+                              const Params& p, const PyrLevel& o, unsigned kk, cudaStream_t st, int form,
+                              bool follows = false)
 {
     if (form >= 8)
         return launch_iterate_stream(g, s->L, cur, nxt, p, o.dep, kk, false, st, s->status, s->num_sms,
-                                     stream_layout(form));
+                                     stream_layout(form), follows);
     if (form == 7) return launch_iterate_quads(g, s->L, cur, nxt, p, o.dep, kk, false, st, s->status);
     return launch_iterate_tiles2(g, s->L, cur, nxt, p, o.dep, kk, false, st, form - 3, s->status);
 }
@@ -247,7 +248,7 @@ int enqueue_mixed(pdflow_solver* s, cudaStream_t st, const std::vector<LaunchRec
             e = launch_step_whole(s, g, alt, p, o, r.kk, g.map + r.count, st, step_whole(s, r.step, g));
             *count += 1;
         } else if (r.kind == 1) {
-            e = launch_step_tiles(s, g, cur, nxt, p, o, r.kk, st, form);
+            e = launch_step_tiles(s, g, cur, nxt, p, o, r.kk, st, form, plan[q - 1].kind == 1);
             std::swap(cur, nxt);
             *count += 1;
         } else {

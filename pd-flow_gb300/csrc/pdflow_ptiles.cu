@@ -60,7 +60,10 @@
 // starts as one of the launch before leaves its SM, prepares its barriers and its
 // first region's descriptor, and waits for that launch's end before its first
 // copy (one VGA pair, 25 launches of about 19 us at 480x640 and 22 of 7 at
-// 240x320: 1237 -> 1191 us with its transfers).
+// 240x320: 1237 -> 1191 us with its transfers), or, from a level's second launch
+// on, before its first copy of state: the constants are final, so their 19 planes
+// arrive while the launch before ends (one VGA solve 962 -> 928 us, one 320x240
+// 500 -> 486, five VGA pairs 3007 -> 2932).
 #include <cuda.h>
 
 #include <algorithm>
@@ -112,6 +115,7 @@ struct StreamArgs {
     Params p;
     unsigned kk;
     bool last;
+    bool follows;              // the kernel before in the stream is a launch of this level: the constants are final
     int tile, halo;            // interior rows and columns, halo width (tile + 2 halo = kSR)
     unsigned tiles_v;          // tiles per column of tiles
     unsigned tiles;            // tiles per pair
@@ -259,22 +263,26 @@ __device__ __forceinline__ Tile continue_unit(const StreamArgs& a, Tile t)
 
 // The tensor copies of a region into the staging planes, completing on `bar`
 // (every consumer warp has read staging).
-__device__ __forceinline__ void issue_region(const StreamMaps& tm, float* sm, uint32_t bar, const Region& r)
+__device__ __forceinline__ void expect_region(uint32_t bar)
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier generic reads before async writes
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                  "r"((uint32_t)N_STAGE * (uint32_t)kSPlane * 4u)
                  : "memory");
+}
+__device__ __forceinline__ void copy_group(const CUtensorMap& map, float* to, uint32_t bar, const Region& r)
+{
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(sm + S_DU * kSPlane)),
-        "l"(reinterpret_cast<uint64_t>(&tm.state)), "r"(r.rv0), "r"(r.ru0), "r"(0), "r"((int)r.slot), "r"(bar)
+        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(to)),
+        "l"(reinterpret_cast<uint64_t>(&map)), "r"(r.rv0), "r"(r.ru0), "r"(0), "r"((int)r.slot), "r"(bar)
         : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(sm + K_RI * kSPlane)),
-        "l"(reinterpret_cast<uint64_t>(&tm.consts)), "r"(r.rv0), "r"(r.ru0), "r"(0), "r"((int)r.slot), "r"(bar)
-        : "memory");
+}
+__device__ __forceinline__ void issue_region(const StreamMaps& tm, float* sm, uint32_t bar, const Region& r)
+{
+    expect_region(bar);
+    copy_group(tm.state, sm + S_DU * kSPlane, bar, r);
+    copy_group(tm.consts, sm + K_RI * kSPlane, bar, r);
 }
 
 // The producer lane: the CTA's walk (tiles blockIdx.x, + gridDim.x, ...; or,
@@ -355,9 +363,18 @@ __global__ void __launch_bounds__(kTma ? kSThreads + kSProducer : kSThreads, 1)
             if constexpr (kStrips) first = strip_at(a, blockIdx.x);
             else first = tile_at(a, blockIdx.x);
             desc = walk_region<kStrips>(a, first);
+            // the first region: its constants before the wait where they are final
+            if (first.more) {
+                expect_region(full);
+                if (a.follows) copy_group(tm.consts, sm + K_RI * kSPlane, full, desc);
+            }
             after_previous_kernel();
-            if (first.more) issue_region(tm, sm, full, desc);
-            else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full) : "memory");
+            if (first.more) {
+                copy_group(tm.state, sm + S_DU * kSPlane, full, desc);
+                if (!a.follows) copy_group(tm.consts, sm + K_RI * kSPlane, full, desc);
+            } else {
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full) : "memory");
+            }
         }
         after_previous_kernel();
         __syncthreads();   // the mbarriers' initialisation before anyone waits on them
@@ -694,7 +711,7 @@ cudaError_t prepare_stream_tiles()
 
 cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State dst, Params p, const float* depth_old,
                                   unsigned kk, bool last, cudaStream_t st, unsigned* status, unsigned ctas,
-                                  StreamLayout layout)
+                                  StreamLayout layout, bool follows)
 {
     // the region stays 32 x 32; rows of region origins stay multiples of 4
     // (16-byte tensor-copy coordinates): halo 4 (interior 24) or 8 (interior 16)
@@ -716,6 +733,7 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
     a.p = p;
     a.kk = kk;
     a.last = last;
+    a.follows = follows;
     a.status = status;
     a.tile = kST;
     a.halo = kSH;

@@ -454,7 +454,7 @@ static int enqueue_iterations(pdflow_solver* s, cudaStream_t st, const LevelGeom
             const unsigned kk = (iters - done < h) ? iters - done : h;
             if (quads && form >= 8)
                 CUDA_TRY(launch_iterate_stream(g, s->L, cur, nxt, p, o.dep, kk, done + kk == iters, st, s->status,
-                                               unsigned(s->num_sms), stream_layout(form)),
+                                               unsigned(s->num_sms), stream_layout(form), done > 0),
                          "streamed tile iteration launch");
             else if (quads)
                 CUDA_TRY(launch_iterate_quads(g, s->L, cur, nxt, p, o.dep, kk, done + kk == iters, st, s->status),
