@@ -60,6 +60,10 @@ int pdflow_set_iteration_form(pdflow_solver* s, int form);
  * (graph replays count the kernels of the captured solve). */
 int pdflow_last_solve_launches(const pdflow_solver* s, unsigned* count);
 
+/* How often calls of this handle have waited for its stream so far (each
+ * reading or synchronising call: once). */
+int pdflow_wait_count(const pdflow_solver* s, unsigned long long* count);
+
 /* Runs `iters` iterations of coarse-to-fine level `level` (0 = coarsest) for
  * pairs [0, n) in the launch form pdflow_solve uses, on the handle's stream,
  * after a solve has left that level's constants in place, and returns the

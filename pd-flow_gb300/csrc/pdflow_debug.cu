@@ -220,6 +220,13 @@ int pdflow_last_solve_launches(const pdflow_solver* s, unsigned* count)
     return PDFLOW_OK;
 }
 
+int pdflow_wait_count(const pdflow_solver* s, unsigned long long* count)
+{
+    if (!s || !count) return fail(PDFLOW_ERR_ARG, "null argument");
+    *count = s->waits;
+    return PDFLOW_OK;
+}
+
 int pdflow_time_level_iterations(pdflow_solver* s, unsigned n, unsigned level, unsigned iters, float* ms)
 {
     if (!s || !ms || n == 0 || n > s->batch || level >= s->ctf_levels || iters == 0)

@@ -51,6 +51,7 @@ struct pdflow_solver {
     int host_frame_next = 0;
     float* host_flow = nullptr;
     size_t host_flow_bytes = 0;
+    unsigned long long waits = 0;        // times a call waited for the stream (status_end)
     int num_sms = 0;
     int iter_form = 10;                  // 10 = chosen by the level (default_level_form): streamed strips, 8 or 9,
                                          // 9 = resident tiles (small levels) or deep streamed tiles,
@@ -169,10 +170,12 @@ void create_frame_buffers(pdflow_solver* s);
 void destroy_host_buffers(pdflow_solver* s);
 int status_begin(pdflow_solver* s);
 int status_end(pdflow_solver* s);
-// Flow planes (null: not wanted) of `rows`-row pairs to the host: pair k's from
-// `step` bytes after pair k-1's, the first `offset` bytes into the arena; n pairs
-// packed in each of dx, dy, dz.  Ends with the status check.
-int read_planes(pdflow_solver* s, size_t offset, size_t step, unsigned n, size_t floats, float* dx, float* dy, float* dz);
+// Flow planes (null: not wanted) of pairs of `floats` pixels to the host, the runs'
+// pairs packed one after another in each of dx, dy, dz; ends with the status check.
+struct FlowRun {
+    unsigned slot, pairs;                // arena slots [slot, slot + pairs)
+};
+int read_planes(pdflow_solver* s, const FlowRun* runs, unsigned count, size_t floats, float* dx, float* dy, float* dz);
 void set_last_error(const char* text);   // the text pdflow_last_error returns on this thread
 // The iteration form a level (of g.pairs pairs) runs in unless one was chosen
 // for it; `resident`: its iterations may run in one launch (form 9).

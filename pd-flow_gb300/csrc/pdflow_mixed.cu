@@ -495,8 +495,8 @@ int pdflow_read_flow_mixed(pdflow_solver* s, unsigned k, float* dx, float* dy, f
         return PDFLOW_ERR_ARG;
     }
     const unsigned r = s->mixed_rows[k];
-    const size_t N = size_t(r) * (r * 4 / 3), po = size_t(k) * s->pair_stride;
-    return read_planes(s, po, s->pair_stride, 1, N, dx, dy, dz);
+    const FlowRun run{k, 1};
+    return read_planes(s, &run, 1, size_t(r) * (r * 4 / 3), dx, dy, dz);
 }
 
 }  // extern "C"

@@ -100,6 +100,7 @@ int status_end(pdflow_solver* s)
     unsigned st = 0;
     if (!s->host_status)
         CUDA_TRY(cudaMemcpyAsync(&st, s->status, sizeof st, cudaMemcpyDeviceToHost, s->stream), "status read");
+    ++s->waits;
     CUDA_TRY(cudaStreamSynchronize(s->stream), "synchronize");
     if (s->host_status) st = *static_cast<volatile unsigned*>(s->host_status);
     if (st != 0) {
@@ -230,29 +231,56 @@ int frame_passed(pdflow_solver* s, int rc)
     return PDFLOW_OK;
 }
 
-int read_planes(pdflow_solver* s, size_t offset, size_t step, unsigned n, size_t floats, float* dx, float* dy, float* dz)
+// Runs go through the pinned buffer as many at a time as it holds, with a wait each
+// time; those it does not hold, and all of them where the caller's memory is not
+// pageable, as copies with one wait.  Six scattered 320x240 slots on a GB300: flows
+// at 60x80 into pageable memory 61 us (two waits; a wait a run 94, as copies 166),
+// into pinned memory 46 (a wait a run 87); at 240x320 into pinned memory 73 (114).
+int read_planes(pdflow_solver* s, const FlowRun* runs, unsigned count, size_t floats, float* dx, float* dy, float* dz)
 {
     float* const dst[3] = {dx, dy, dz};
     const float* const src[3] = {s->dx, s->dy, s->dz};
-    const size_t b = floats * 4;
-    bool pass = 3 * b * n <= s->host_flow_bytes && n <= 65535;
+    const size_t b = floats * 4, step = s->pair_stride;
+    bool pass = true, copied = false;
     for (float* d : dst) pass = pass && (!d || pageable(d));
-    if (pass) {
-        CUDA_TRY(launch_flow_out(at(s->dx, offset), at(s->dy, offset), at(s->dz, offset), step, n, floats, s->status,
-                                 s->host_flow, s->host_status, s->stream),
-                 "flow read launch");
-        const int rc = status_end(s);
-        for (int a = 0; a < 3; ++a)
-            if (dst[a]) std::memcpy(dst[a], s->host_flow + a * floats * n, b * n);
-        return rc;
+    const size_t most = pass ? std::min<size_t>(s->host_flow_bytes / (3 * b), 65535) : 0;   // pairs that pass at once
+    int rc = PDFLOW_OK;
+    size_t k = 0;   // pairs before run r
+    for (unsigned r = 0; r < count;) {
+        unsigned end = r;
+        size_t n = 0;
+        while (end < count && n + runs[end].pairs <= most) n += runs[end++].pairs;
+        if (end == r) {
+            if (!copied)
+                if (const int e = status_begin(s)) return e;
+            for (int a = 0; a < 3; ++a)
+                if (dst[a])
+                    CUDA_TRY(cudaMemcpy2DAsync(dst[a] + floats * k, b, at(src[a], runs[r].slot * step), step, b,
+                                               runs[r].pairs, cudaMemcpyDeviceToHost, s->stream),
+                             "D2H flow");
+            copied = true;
+            k += runs[r++].pairs;
+            continue;
+        }
+        size_t at_k = 0;
+        for (unsigned q = r; q < end; at_k += runs[q++].pairs) {
+            const size_t o = runs[q].slot * step;
+            CUDA_TRY(launch_flow_out(at(s->dx, o), at(s->dy, o), at(s->dz, o), step, runs[q].pairs, floats, s->status,
+                                     s->host_flow + 3 * floats * at_k, s->host_status, s->stream),
+                     "flow read launch");
+        }
+        const int waited = status_end(s);
+        if (rc == PDFLOW_OK) rc = waited;
+        const float* from = s->host_flow;
+        for (; r < end; k += runs[r++].pairs)
+            for (int a = 0; a < 3; ++a, from += floats * runs[r].pairs)
+                if (dst[a]) std::memcpy(dst[a] + floats * k, from, b * runs[r].pairs);
     }
-    int rc = status_begin(s);
-    if (rc) return rc;
-    for (int a = 0; a < 3; ++a)
-        if (dst[a])
-            CUDA_TRY(cudaMemcpy2DAsync(dst[a], b, at(src[a], offset), step, b, n, cudaMemcpyDeviceToHost, s->stream),
-                     "D2H flow");
-    return status_end(s);
+    if (copied) {
+        const int waited = status_end(s);
+        if (rc == PDFLOW_OK) rc = waited;
+    }
+    return rc;
 }
 
 // Carves the arena: `batch` identical per-pair slices (pair k's buffers
@@ -924,7 +952,8 @@ int pdflow_read_flow_batch(pdflow_solver* s, unsigned n, float* dx, float* dy, f
     if (!s || !dx || !dy || !dz) return set_error(PDFLOW_ERR_ARG, "null argument");
     if (s->mixed) return set_error(PDFLOW_ERR_STATE, "a mixed-resolution handle: use the mixed calls");
     if (bad_count(s, n)) return set_error(PDFLOW_ERR_ARG, "pair count out of range");
-    return read_planes(s, 0, s->pair_stride, n, size_t(s->rows) * s->cols, dx, dy, dz);
+    const FlowRun all{0, n};
+    return read_planes(s, &all, 1, size_t(s->rows) * s->cols, dx, dy, dz);
 }
 
 int pdflow_read_flow(pdflow_solver* s, float* dx, float* dy, float* dz)
@@ -1055,15 +1084,12 @@ int pdflow_read_flow_slots(pdflow_solver* s, unsigned n, const unsigned* slots, 
         if (slots[k] >= s->batch) return set_error(PDFLOW_ERR_ARG, "slot out of range");
     // runs of consecutive slots, a copy a plane each (every copy to pageable memory
     // blocks for 10 us or more: six QVGA slots one by one took 314 us)
-    int rc = PDFLOW_OK;
-    for (unsigned k = 0; k < n;) {
-        unsigned m = 1;
-        while (k + m < n && slots[k + m] == slots[k] + m) ++m;
-        const int r = read_planes(s, slots[k] * s->pair_stride, s->pair_stride, m, N, dx + k * N, dy + k * N, dz + k * N);
-        if (rc == PDFLOW_OK) rc = r;
-        k += m;
+    std::vector<FlowRun> runs;
+    for (unsigned k = 0; k < n; ++k) {
+        if (!runs.empty() && slots[k] == runs.back().slot + runs.back().pairs) ++runs.back().pairs;
+        else runs.push_back(FlowRun{slots[k], 1});
     }
-    return rc;
+    return read_planes(s, runs.data(), unsigned(runs.size()), N, dx, dy, dz);
 }
 
 int pdflow_energy_batch(pdflow_solver* s, unsigned n, float* energies)
