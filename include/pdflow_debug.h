@@ -64,6 +64,10 @@ int pdflow_last_solve_launches(const pdflow_solver* s, unsigned* count);
  * reading or synchronising call: once). */
 int pdflow_wait_count(const pdflow_solver* s, unsigned long long* count);
 
+/* Host memory this handle has pinned so far for its transfers (taken by the
+ * first call that has a use for it). */
+int pdflow_pinned_bytes(const pdflow_solver* s, size_t* bytes);
+
 /* Runs `iters` iterations of coarse-to-fine level `level` (0 = coarsest) for
  * pairs [0, n) in the launch form pdflow_solve uses, on the handle's stream,
  * after a solve has left that level's constants in place, and returns the

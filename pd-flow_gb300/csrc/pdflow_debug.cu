@@ -227,6 +227,13 @@ int pdflow_wait_count(const pdflow_solver* s, unsigned long long* count)
     return PDFLOW_OK;
 }
 
+int pdflow_pinned_bytes(const pdflow_solver* s, size_t* bytes)
+{
+    if (!s || !bytes) return fail(PDFLOW_ERR_ARG, "null argument");
+    *bytes = s->host_pinned_bytes;
+    return PDFLOW_OK;
+}
+
 int pdflow_time_level_iterations(pdflow_solver* s, unsigned n, unsigned level, unsigned iters, float* ms)
 {
     if (!s || !ms || n == 0 || n > s->batch || level >= s->ctf_levels || iters == 0)

@@ -41,8 +41,11 @@ struct pdflow_solver {
     pdflow::LevelSol sol{};
     unsigned* flags = nullptr;           // per-CTA progress counters of the grid-form iteration
     unsigned* status = nullptr;          // device status word (0 = ok)
-    // Pinned host memory the device addresses (null: transfers go to and from the
-    // caller's memory directly): the status word, two frame buffers, a result buffer.
+    // Pinned host memory the device addresses, taken on first use (null: transfers go
+    // to and from the caller's memory directly): the status word, a result buffer, two
+    // frame buffers.
+    size_t host_pinned_bytes = 0;
+    bool host_result_tried = false;
     unsigned* host_status = nullptr;
     uint8_t* host_frames[2] = {};
     size_t host_frame_bytes = 0;
@@ -162,10 +165,10 @@ struct TuneCandidate {
 };
 TuneCandidate tune_candidate(int c);
 int check_status(pdflow_solver* s);
-// The handle's pinned transfer buffers, for results of `flow` bytes and more.
 // check_status in two halves: status_begin before the copies of a result (they
 // may block on the host), status_end after them.
-void create_host_buffers(pdflow_solver* s, size_t flow);
+// The handle's pinned transfer buffers, on first use.
+void create_result_buffer(pdflow_solver* s);
 void create_frame_buffers(pdflow_solver* s);
 void destroy_host_buffers(pdflow_solver* s);
 int status_begin(pdflow_solver* s);

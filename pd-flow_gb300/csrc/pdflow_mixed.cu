@@ -364,8 +364,6 @@ int pdflow_create_mixed(unsigned max_pairs, pdflow_solver** out)
     int rc = pdflow_create_batch(480, 640, 480, nullptr, max_pairs, out);
     if (rc) return rc;
     (*out)->mixed = 1;
-    pdflow::destroy_host_buffers(*out);   // sized for 640x480 results: here those of up to 120x160 pass
-    pdflow::create_host_buffers(*out, size_t(60) * 80 * 12);
     (*out)->mixed_rows.assign(max_pairs, 0);
     return PDFLOW_OK;
 }

@@ -87,6 +87,7 @@ void set_last_error(const char* text) { g_last_error = text; }
 // pageable memory waits for the stream (10 us a call, on top of the result's).
 int status_begin(pdflow_solver* s)
 {
+    create_result_buffer(s);
     if (s->host_status)
         CUDA_TRY(cudaMemcpyAsync(s->host_status, s->status, sizeof(unsigned), cudaMemcpyDeviceToHost, s->stream),
                  "status read");
@@ -127,22 +128,39 @@ int check_status(pdflow_solver* s)
 // 60x80 (58 KB): 40 -> 21 us; at 240x320 (922 KB): 48 -> 75.  The limits lie between.
 constexpr size_t kHostFrameLimit = 256u << 10, kHostFlowLimit = 256u << 10;
 
-// The status word and a result buffer for flows of `flow` bytes and more, and for
-// a single pair's handle the frame buffers (a batch's on its first push that fits
-// one).  Best effort: without the memory (or where nothing would pass through it)
-// transfers are direct.
-void create_host_buffers(pdflow_solver* s, size_t flow)
+// Another thread's capture in global mode forbids this thread the waits and
+// allocations that a capture of its own would record wrongly; these are none.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
+// Pinned memory is taken by the first call that has a use for it (a caller with
+// frames and flows on the device has none): the status word and a result buffer by
+// the first that waits, the frame buffers by the first push that fits one.  Best
+// effort: without the memory (or where nothing would pass through it) transfers are
+// direct.  Taken at creation, a handle for one 320x240 pair took 250 us to create,
+// without 100; the first push and read take that time instead.
+void create_result_buffer(pdflow_solver* s)
 {
+    if (s->host_result_tried) return;
+    s->host_result_tried = true;
+    const RelaxedCapture relaxed;
+    // of a mixed batch, flows of up to 60x80 pass (of five pairs and more, up to 120x160)
+    const size_t flow = (s->mixed ? size_t(60) * 80 : size_t(s->rows) * s->cols) * 12;
     const size_t cap = flow <= kHostFlowLimit ? std::min(flow * s->batch, kHostFlowLimit) : 0;
     void* p = nullptr;
     if (cudaHostAlloc(&p, 256 + cap, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
+    s->host_pinned_bytes += 256 + cap;
     s->host_status = static_cast<unsigned*>(p);
     s->host_flow = reinterpret_cast<float*>(static_cast<uint8_t*>(p) + 256);
     s->host_flow_bytes = cap;
-    if (s->batch == 1) create_frame_buffers(s);
 }
 
 void create_frame_buffers(pdflow_solver* s)
@@ -155,6 +173,7 @@ void create_frame_buffers(pdflow_solver* s)
         cudaGetLastError();
         return;
     }
+    s->host_pinned_bytes += 2 * kHostFrameLimit;
     s->host_frames[0] = static_cast<uint8_t*>(p);
     s->host_frames[1] = s->host_frames[0] + kHostFrameLimit;
     if (cudaEventCreateWithFlags(&s->host_frame_read[0], cudaEventDisableTiming) == cudaSuccess &&
@@ -166,16 +185,10 @@ void create_frame_buffers(pdflow_solver* s)
 
 void destroy_host_buffers(pdflow_solver* s)
 {
-    for (cudaEvent_t& e : s->host_frame_read) {
+    for (cudaEvent_t e : s->host_frame_read)
         if (e) cudaEventDestroy(e);
-        e = nullptr;
-    }
     if (s->host_frames[0]) cudaFreeHost(s->host_frames[0]);
     if (s->host_status) cudaFreeHost(s->host_status);
-    s->host_frames[0] = s->host_frames[1] = nullptr;
-    s->host_status = nullptr;
-    s->host_frame_bytes = s->host_flow_bytes = 0;
-    s->host_frame_tried = false;
 }
 
 // Ordinary host memory (neither pinned nor managed: work on the stream may still
@@ -189,16 +202,6 @@ bool pageable(const void* p)
     }
     return a.type == cudaMemoryTypeUnregistered;
 }
-
-// Another thread's capture in global mode forbids this thread the waits and
-// allocations that a capture of its own would record wrongly; these are none.
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    RelaxedCapture(const RelaxedCapture&) = delete;
-    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
-};
 
 // Copies a frame's two images into the next frame buffer; null where it goes
 // directly (size, memory, or a capture, which has to record the caller's address).
@@ -241,6 +244,7 @@ int read_planes(pdflow_solver* s, const FlowRun* runs, unsigned count, size_t fl
     float* const dst[3] = {dx, dy, dz};
     const float* const src[3] = {s->dx, s->dy, s->dz};
     const size_t b = floats * 4, step = s->pair_stride;
+    create_result_buffer(s);
     bool pass = true, copied = false;
     for (float* d : dst) pass = pass && (!d || pageable(d));
     const size_t most = pass ? std::min<size_t>(s->host_flow_bytes / (3 * b), 65535) : 0;   // pairs that pass at once
@@ -799,7 +803,6 @@ int pdflow_create_batch(unsigned rows, unsigned width, unsigned height, const pd
         return set_error(PDFLOW_ERR_CUDA, "stream / arena init", e);
     }
     s->stream = s->own_stream;
-    create_host_buffers(s, size_t(rows) * cols * 12);
     *out = s;
     return PDFLOW_OK;
 }

@@ -194,7 +194,8 @@ _SIGNATURES = {
     "pdflow_set_tile_copy_mode": (ctypes.c_int, [ctypes.c_int, ctypes.c_int]),
     "pdflow_set_quad_prefetch": (ctypes.c_int, [ctypes.c_uint]),
     "pdflow_measure_copy_gbs": (ctypes.c_int, [ctypes.c_size_t, u32, vp, ctypes.POINTER(ctypes.c_float)]),
-    "pdflow_wait_count": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_ulonglong)]),
+    "pdflow_wait_count": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_ulonglong)]),
+    "pdflow_pinned_bytes": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_size_t)]),
     "pdflow_check_div_rcp": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_ulonglong, ctypes.POINTER(ctypes.c_ulonglong)]),
     "pdflow_check_disc_factor": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_ulonglong,
                                                 ctypes.POINTER(ctypes.c_ulonglong)]),
