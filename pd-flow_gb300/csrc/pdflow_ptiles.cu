@@ -67,6 +67,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "pdflow_iterate.cuh"
@@ -685,9 +686,20 @@ bool stream_direct_eligible(const LevelGeom& g, const LevelConsts& L, const Stat
     return true;
 }
 
+// Whether the kernels that stream their regions have the registers their split
+// counts on (prepare_stream_tiles): with another count the consumers' setmaxnreg
+// would wait for what the launch did not bring, so they do not run and levels take
+// the tiles on direct loads.  The build refuses such a compiler's output.
+static std::atomic<bool> streamed_copies{false};
+
+static bool copies_eligible(const LevelGeom& g, const LevelConsts& L, const State& src, const State& dst)
+{
+    return streamed_copies && quads_eligible(g, L, src, dst);
+}
+
 bool stream_eligible(const LevelGeom& g, const LevelConsts& L, const State& src, const State& dst, int form)
 {
-    if (quads_eligible(g, L, src, dst)) return true;
+    if (form == 7 ? quads_eligible(g, L, src, dst) : copies_eligible(g, L, src, dst)) return true;
     return (form == 8 || form == 9) && stream_direct_eligible(g, L, src, dst);
 }
 
@@ -700,12 +712,13 @@ cudaError_t prepare_stream_tiles()
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem_bytes());
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     }
-    // the consumers' setmaxnreg would wait for registers the launch did not bring
+    bool exact = e == cudaSuccess;
     for (const void* k : {(const void*)k_iterate_stream<false>, (const void*)k_iterate_stream<true>}) {
         cudaFuncAttributes fa{};
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k);
-        if (e == cudaSuccess && fa.numRegs != kSLaunchRegs) e = cudaErrorInvalidConfiguration;
+        exact = exact && fa.numRegs == kSLaunchRegs;
     }
+    if (e == cudaSuccess) streamed_copies = exact;
     return e;
 }
 
@@ -720,7 +733,7 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
     // the tensor copies need the quad tiles' preconditions (16-byte aligned
     // planes at one spacing, rows % 4 == 0); the tiles also run on direct loads
     // where the rows are even
-    const bool tma = quads_eligible(g, L, src, dst);
+    const bool tma = copies_eligible(g, L, src, dst);
     if (kk == 0 || kk > (unsigned)kSH || !status || ctas == 0 || reinterpret_cast<uintptr_t>(depth_old) % 8u != 0 ||
         !(tma || (!strips && stream_direct_eligible(g, L, src, dst))))
         return cudaErrorInvalidValue;

@@ -13,6 +13,7 @@ from __future__ import annotations
 import concurrent.futures as cf
 import glob
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -69,6 +70,23 @@ def _compile(src: str):
     return obj, r.stderr
 
 
+# Kernels whose register split needs the launch to bring an exact count: the
+# consumers' setmaxnreg waits for what is missing (pdflow_ptiles.cu).
+EXACT_REGISTERS = {r"k_iterate_streamILb[01]ELb1E": 96}
+
+
+def check_registers(report: str) -> None:
+    """Raises where the compiler's report gives a kernel of EXACT_REGISTERS another count, or none."""
+    used = re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", report, re.S)
+    for pattern, want in EXACT_REGISTERS.items():
+        counts = {name: int(n) for name, n in used if re.search(pattern, name)}
+        if not counts:
+            raise RuntimeError(f"no kernel {pattern} in the compiler's report")
+        for name, n in counts.items():
+            if n != want:
+                raise RuntimeError(f"{name} uses {n} registers a thread; its register split needs exactly {want}")
+
+
 def build(verbose: bool = False) -> str:
     """Compiles csrc/ into lib/libpdflow_gb300.so (incremental) and returns its path."""
     os.makedirs(OBJDIR, exist_ok=True)
@@ -79,6 +97,7 @@ def build(verbose: bool = False) -> str:
     logs = "".join(l for _, l in results)     # every translation unit's report, fresh or kept
     with open(os.path.join(LIBDIR, "ptxas.log"), "w") as f:
         f.write(logs)
+    check_registers(logs)
     if _stale(LIB_PATH, objs):
         cuda_lib = os.path.join(_cuda_home(), "lib64")
         cmd = [_nvcc(), *ARCH, "-shared", "-cudart", "shared", "-o", LIB_PATH, *objs,
