@@ -138,6 +138,10 @@ int pdflow_check_disc_factor(unsigned long long pairs, unsigned long long seed, 
 int pdflow_strip_units(unsigned bands, unsigned cols, unsigned iters_per_launch, unsigned ctas, unsigned* whole,
                        unsigned* tier_n, unsigned* tier_p);
 
+/* How many strip plans (pdflow_strip_units and the strips' launches) the calling
+ * thread has searched for so far; a few are kept per thread and found again. */
+int pdflow_strip_plan_count(unsigned long long* count);
+
 /* Copy bandwidth of this GPU for a working set of `bytes` per buffer (the
  * roofline denominators; no counterpart in the reference): allocates two
  * buffers of `bytes` and copies them into each other `reps` times within one

@@ -379,6 +379,13 @@ int pdflow_check_disc_factor(unsigned long long pairs, unsigned long long seed, 
     return count_mismatches(k_disc_check, pairs, seed, mismatches);
 }
 
+int pdflow_strip_plan_count(unsigned long long* count)
+{
+    if (!count) return fail(PDFLOW_ERR_ARG, "null argument");
+    *count = pdflow::strip_plans();
+    return PDFLOW_OK;
+}
+
 int pdflow_strip_units(unsigned bands, unsigned cols, unsigned iters_per_launch, unsigned ctas, unsigned* whole,
                        unsigned* tier_n, unsigned* tier_p)
 {

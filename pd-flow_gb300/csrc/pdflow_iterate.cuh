@@ -86,6 +86,8 @@ struct StripUnits {
     unsigned whole, tier_n[3], tier_p[3];
 };
 StripUnits strip_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid);
+// How many of the calling thread's calls have searched for a plan (the others found it kept).
+unsigned long long strip_plans();
 // When a launch of the level's strips ends on `ctas` CTAs at 4 iterations per
 // launch, in regions a CTA (the 24x24 tiles' end is their rounds of CTAs).
 float strips_end(const LevelGeom& g, unsigned ctas);

@@ -634,6 +634,9 @@ StripUnits plan_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid)
 
 }  // namespace
 
+static thread_local unsigned long long plans = 0;
+unsigned long long strip_plans() { return plans; }
+
 // Strip units.  Each piece of a strip recomputes a left halo, so many strips
 // (over four a CTA) stay whole but for a short tail: on 64-pair VGA solves (1
 // 280 strips of 23 regions at 480x640, 640 of 12 at 240x320) the last grid /
@@ -643,20 +646,22 @@ StripUnits plan_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid)
 // regions, the work is 18.9), so the cuts are chosen by when the queue ends:
 // there 200 strips in 3 pieces and 40 in 4 end after 19.8 (85 iterations 2.76 ->
 // 2.26 ms on a GB300; 13 pairs at 480x640 5.10 -> 4.56, 20 pairs 7.47 -> 6.78).
-// The choice is a function of its arguments; the last few are kept.
+// The choice is a function of its arguments; the last 64 are kept (a search takes
+// up to 0.5 ms of host time).
 StripUnits strip_units(unsigned strips_n, unsigned C, unsigned kk, unsigned grid)
 {
     struct Kept {
         unsigned key[4];
         StripUnits units;
     };
-    thread_local Kept kept[16] = {};
+    thread_local Kept kept[64] = {};
     thread_local unsigned next = 0;
     const unsigned key[4] = {strips_n, C, kk, grid};
     for (const Kept& k : kept)
         if (std::equal(key, key + 4, k.key)) return k.units;
+    ++plans;
     const StripUnits su = plan_units(strips_n, C, kk, grid);
-    Kept& k = kept[next++ % 16u];
+    Kept& k = kept[next++ % 64u];
     std::copy(key, key + 4, k.key);
     k.units = su;
     return su;
@@ -754,7 +759,7 @@ cudaError_t launch_iterate_stream(LevelGeom g, LevelConsts L, State src, State d
     a.tiles = a.tiles_v * ((g.C + kST - 1) / kST);
     a.total = a.tiles * g.pairs;
     const unsigned grid = ctas < a.total ? ctas : a.total;
-    const StripUnits su = strip_units(g.pairs * a.tiles_v, g.C, kk, grid);
+    const StripUnits su = strips ? strip_units(g.pairs * a.tiles_v, g.C, kk, grid) : StripUnits{};
     a.whole = su.whole;
     for (int i = 0; i < 3; ++i) {
         a.tier_n[i] = su.tier_n[i];

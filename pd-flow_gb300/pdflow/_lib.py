@@ -199,6 +199,7 @@ _SIGNATURES = {
     "pdflow_check_div_rcp": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_ulonglong, ctypes.POINTER(ctypes.c_ulonglong)]),
     "pdflow_check_disc_factor": (ctypes.c_int, [ctypes.c_ulonglong, ctypes.c_ulonglong,
                                                 ctypes.POINTER(ctypes.c_ulonglong)]),
+    "pdflow_strip_plan_count": (ctypes.c_int, [ctypes.POINTER(ctypes.c_ulonglong)]),
     "pdflow_strip_units": (ctypes.c_int, [u32, u32, u32, u32, ctypes.POINTER(u32), ctypes.POINTER(u32),
                                           ctypes.POINTER(u32)]),
     "pdflow_debug_wait_timeout": (ctypes.c_int, [vp, u32]),
