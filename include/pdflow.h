@@ -237,7 +237,9 @@ int pdflow_read_flow_mixed(pdflow_solver* s, unsigned k, float* dx, float* dy, f
  * form 9: the same with 16x16 interiors and a halo of 8,
  * up to 8 iterations per launch, for levels whose launches are latency-bound, or,
  * at 30x40 and (up to about 20 pairs) 60x80, all the level's iterations in one
- * launch with a thread-block cluster per pair;
+ * launch with a thread-block cluster per pair (there the iterations per launch
+ * have no meaning: any value runs the same launch, and the autotuner times one of
+ * the form's candidates and reports its time for all three);
  * form 10: rows of regions walked left to right, each handing the next its
  * last exact column's exchange values, so no left halo is recomputed; levels
  * with rows % 4 == 0).

@@ -309,11 +309,15 @@ int pdflow::mixed_autotune(pdflow_solver* s, unsigned n, unsigned probe_iters, p
                 const unsigned kk = tune_candidate(idx).kk;
                 if (form < 3) continue;                   // mixed steps run tile forms only
                 if (form >= 7 && !stream_eligible(g, s->L, s->S, s->S, form)) continue;
+                const bool whole = form == 9 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms));
+                if (whole && tune_candidate(idx - 1).form == 9) {   // one launch at any iterations per launch
+                    rep.level[i].ms_per_iter[idx] = rep.level[i].ms_per_iter[idx - 1];
+                    continue;
+                }
                 float t = INFINITY;
                 for (int r = 0; r < 4 && rc == PDFLOW_OK; ++r) {
                     cudaEventRecord(e0, s->stream);
                     State cur = s->S, nxt = alt;
-                    const bool whole = form == 9 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms));
                     if (whole) {   // what form 9 then runs
                         const cudaError_t e = launch_step_whole(s, g, alt, p, o, probe_iters, nullptr, s->stream, 9);
                         if (e != cudaSuccess) rc = set_error_code(PDFLOW_ERR_CUDA, "mixed autotune launch", e);

@@ -90,6 +90,13 @@ int pdflow_autotune(pdflow_solver* s, unsigned n, unsigned probe_iters, pdflow_t
             rep.level[i].ms_per_iter[c] = NAN;
             if (kCandidates[c].form == 1 && !one_ok) continue;
             if (kCandidates[c].form >= 7 && !stream_eligible(g, s->L, s->S, s->S, kCandidates[c].form)) continue;
+            // resident tiles are one launch at any iterations per launch: one candidate
+            const bool again = c > 0 && kCandidates[c].form == 9 && kCandidates[c - 1].form == 9 &&
+                               resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms));
+            if (again) {
+                rep.level[i].ms_per_iter[c] = rep.level[i].ms_per_iter[c - 1];
+                continue;
+            }
             s->level_form[i] = kCandidates[c].form;
             s->level_kk[i] = kCandidates[c].kk;
             float t = INFINITY;
