@@ -29,9 +29,12 @@ int pdflow_debug_solve(pdflow_solver* s, pdflow_dump_fn fn, void* ctx);
  * column pieces of them; taken from a device counter as CTAs finish) left to
  * right and hands each region's last exact column's exchange values to the
  * next one, so that only a right halo is recomputed (28 of 32 columns exact
- * at 4 iterations per launch); levels with fewer bands than SMs run 8
- * instead, or 9 where all of the level's 16x16 tiles fit in one round of
- * CTAs (a single pair's 60x80 and 120x160 levels); 9 = as 8 with 16x16
+ * at 4 iterations per launch); levels whose tiles end earlier on the SMs
+ * run 8 instead, or 9 where all of the level's 16x16 tiles fit in one round of
+ * CTAs (a single pair's 120x160 level) or the level runs resident; 15x20 runs as
+ * one launch with a CTA per pair; 9 = all iterations of 30x40 and (up to about 20
+ * pairs) 60x80 in one launch with a thread-block cluster per pair ("resident"),
+ * the other levels as 8 with 16x16
  * interiors and a halo of 8 (up to 8 iterations per launch); 8 = every
  * level of a batch (more than one pair), and a single pair's levels above 300
  * pixels, as temporally blocked 24x24 tiles (halo 4, up to 4 iterations per
@@ -39,7 +42,7 @@ int pdflow_debug_solve(pdflow_solver* s, pdflow_dump_fn fn, void* ctx);
  * constants in registers (one pixel pair per thread, packed FP32x2) while
  * the next tile's region streams into shared memory by two 4D TMA tensor
  * copies; levels whose row count is even but not a multiple of 4 (30x40)
- * load each pixel pair directly instead, and 15x20 runs form 5 there;
+ * load each pixel pair directly instead, and a batch's 15x20 runs form 5 there;
  * 7 = the same tiles as one CTA per tile, four rows per
  * thread with the state in registers and the constants in shared memory;
  * 5 = every level of a batch, and a single pair's levels above

@@ -78,16 +78,16 @@ LevelGeom step_geom(const pdflow_solver* s, unsigned step, unsigned pairs, const
 }
 
 // Whether the iterations at step i run as one launch, each pair's own count in
-// it: 9 as resident tiles (where form 9 was chosen, or the handle's forms are the
-// default, and the level fits a cluster), 1 as a CTA per pair (15x20, not tuned),
-// 0 not.  As tiles, pairs of different schedules are a launch per 1-4 iterations, 67
+// it: 9 as resident tiles (where form 9 was chosen for the step or the handle, or the
+// form is the default, and the level fits a cluster), 1 as a CTA per pair (15x20 by
+// default), 0 not.  As tiles, pairs of different schedules are a launch per 1-4 iterations, 67
 // launches at the three smallest steps: 16 pairs of rows 60 to 480 solve in 3.99 ms,
 // as whole launches in 3.80.
 int step_whole(const pdflow_solver* s, unsigned i, const LevelGeom& g)
 {
     const bool chosen = s->mixed_form[i] >= 3;
     if (chosen ? s->mixed_form[i] != 9 : s->iter_form < 9) return 0;
-    if (g.N <= 300u) return chosen ? 0 : 1;
+    if (g.N <= 300u) return !chosen && s->iter_form == 10 ? 1 : 0;
     return resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms)) ? 9 : 0;
 }
 

@@ -384,16 +384,17 @@ LevelGeom level_geom(const pdflow_solver* s, unsigned i, unsigned* level_image, 
 // run as one launch (k_iterate: one CTA, one cluster, or, for a single pair,
 // the cooperative full grid) or, for a batch of pairs at a level that needs
 // the full grid, as two batched kernels per iteration.
-// Whether level `level`'s iterations run as tiles.  The 15x20 level runs as one
-// launch with a CTA per pair (register-resident, one pixel a thread) instead:
+// Whether level `level`'s iterations run as tiles.  By default the 15x20 level runs
+// as one launch with a CTA per pair (register-resident, one pixel a thread) instead:
 // per VGA solve 0.034 ms for any batch up to an SM per pair, against 0.085 ms of
 // paired tiles (64 pairs).  Everything larger runs tiles (per iteration at
-// 30x40 .. 120x160 about half the time of the one-launch form).
+// 30x40 .. 120x160 about half the time of the one-launch form).  A tile form chosen
+// for the handle runs tiles at 15x20 too, of a batch.
 static bool level_runs_tiles(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned level)
 {
     const int forced = level < 8 ? s->level_form[level] : -1;
     if (forced >= 0) return forced >= 2 && iters > 0;
-    return s->iter_form >= 2 && iters > 0 && g.N > 300u;
+    return s->iter_form >= 2 && iters > 0 && (g.N > 300u || (g.pairs > 1 && s->iter_form != 10));
 }
 
 }  // namespace pdflow
@@ -432,8 +433,7 @@ static int level_form(const pdflow_solver* s, const LevelGeom& g, unsigned level
 // streamed tiles and strips, forms 8-10): chosen for the level and possible at its size
 // (rows % 4 == 0, or even rows for the streamed tiles; other levels of such a
 // solve run the paired 24x24 tiles, form 5).
-static bool level_runs_quads(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned pairs,
-                             unsigned level)
+static bool level_runs_quads(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned level)
 {
     if (!level_runs_tiles(s, g, iters, level)) return false;
     const int form = level_form(s, g, level);
@@ -441,12 +441,11 @@ static bool level_runs_quads(const pdflow_solver* s, const LevelGeom& g, unsigne
 }
 
 // The step-size planes the level's set-up writes for its iteration form.
-static int level_steps(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned pairs, unsigned level,
-                       bool all_steps)
+static int level_steps(const pdflow_solver* s, const LevelGeom& g, unsigned iters, unsigned level, bool all_steps)
 {
     if (all_steps) return kStepsAll;
     if (!level_runs_tiles(s, g, iters, level)) return kStepsRaw;
-    return level_runs_quads(s, g, iters, pairs, level) ? kStepsQuads : kStepsNone;
+    return level_runs_quads(s, g, iters, level) ? kStepsQuads : kStepsNone;
 }
 
 // Enqueues `iters` iterations of level i for pairs [0, pairs) in the
@@ -464,7 +463,7 @@ static int enqueue_iterations(pdflow_solver* s, cudaStream_t st, const LevelGeom
     const int form = level_form(s, g, level);
     const bool one_launch = forced >= 0 ? (forced == 1 && iters > 0 && one_launch_ok)
                                         : (s->iter_form >= 1 && iters > 0 && !tiles && one_launch_ok);
-    const bool quads = tiles && level_runs_quads(s, g, iters, pairs, level);
+    const bool quads = tiles && level_runs_quads(s, g, iters, level);
     const bool paired = tiles && form >= 3;
     const int shape = form >= 7 ? 2 : form - 3;   // 40x40, 40x34, 24x24 or 24x28 tiles (forms 7-10 elsewhere: 24x24)
     if (quads && form == 9 && resident_eligible(g, s->L, s->S, s->S, unsigned(s->num_sms))) {
@@ -606,7 +605,7 @@ int enqueue_solve(pdflow_solver* s, cudaStream_t st, unsigned pairs, const Solve
         cudaEvent_t* tr = plan.trace ? plan.trace + 3 * (i - plan.first) : nullptr;
         if (tr) CUDA_TRY(cudaEventRecord(tr[0], st), "trace event");
         const unsigned iters = scaled_iters(s->prm.num_max_iter[i], plan.iter_scale);
-        const int steps = level_steps(s, g, iters, pairs, i, plan.all_steps);
+        const int steps = level_steps(s, g, iters, i, plan.all_steps);
         const LevelStart start = seed ? LevelStart::Seed : (i == 0 ? LevelStart::Zeros : LevelStart::Coarse);
         CUDA_TRY(launch_level_setup(g, start, s->sol, o, n, s->L, s->S, p, steps, aux_offset(s, i), st, seed),
                  "level set-up launch");
