@@ -381,7 +381,7 @@ struct pdflow_net {
     float *loss_part = nullptr, *input = nullptr;
     unsigned* count = nullptr;
     unsigned* status = nullptr;
-    size_t col_elems = 0, part_elems = 0;
+    size_t part_elems = 0;
     int step = 0;
     size_t device_bytes = 0;
     std::vector<void*> allocs;
@@ -820,7 +820,8 @@ int pdflow_net_create(unsigned max_batch, unsigned long long seed, pdflow_net** 
     n->max_batch = max_batch;
     build_graph(n);
     cudaError_t e = cudaSuccess;
-    const size_t B = max_batch;
+    // im2col matrices: only the batches below kImplicitConvMinBatch have them
+    const size_t B = max_batch, Bcol = std::min<size_t>(B, kImplicitConvMinBatch - 1);
     n->w = dalloc<float>(n, n->nparams, &e);
     n->m = dalloc<float>(n, n->nparams, &e);
     n->v = dalloc<float>(n, n->nparams, &e);
@@ -829,16 +830,15 @@ int pdflow_net_create(unsigned max_batch, unsigned long long seed, pdflow_net** 
     for (auto& c : n->conv) {
         n->Wb.push_back(dalloc<__nv_bfloat16>(n, size_t(c.cout_pad) * c.K(), &e));
         n->WTb.push_back(dalloc<__nv_bfloat16>(n, size_t(c.K()) * c.cout_pad, &e));
-        const size_t P = B * c.H * c.W, Pp = (P + 7) / 8 * 8;
+        const size_t P = B * c.H * c.W;
         maxK = std::max(maxK, size_t(c.K()) * c.cout_pad);
-        maxPK = std::max(maxPK, Pp * c.K());
+        maxPK = std::max(maxPK, Bcol * c.H * c.W * c.K());
         maxPcin = std::max(maxPcin, P * (c.c1 + c.c2));
     }
     for (auto& a : n->act) {
         a.x = dalloc<__nv_bfloat16>(n, B * a.H * a.W * a.C, &e);
         a.g = dalloc<float>(n, B * a.H * a.W * a.C, &e);
     }
-    n->col_elems = maxPK;
     n->col = dalloc<__nv_bfloat16>(n, maxPK, &e);
     n->dcat = dalloc<float>(n, maxPcin, &e);
     n->dy = dalloc<__nv_bfloat16>(n, B * kHW * 96, &e);
