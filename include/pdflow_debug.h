@@ -121,7 +121,8 @@ int pdflow_set_quad_prefetch(unsigned ctas_ahead);
  * rounded reciprocal and two FMA corrections (Markstein's theorem) instead
  * of an IEEE division; this compares that quotient with the IEEE one
  * (__fdiv_rn) bit for bit on `pairs` random pairs of the range the kernels
- * use it in and returns how many differ (0 expected). */
+ * use it in (numerators up to 2^90 and quotients at the shrinkage's threshold
+ * among them) and returns how many differ (0 expected). */
 int pdflow_check_div_rcp(unsigned long long pairs, unsigned long long seed, unsigned long long* mismatches);
 
 /* Check of the disc projection's factor (no counterpart in the reference):

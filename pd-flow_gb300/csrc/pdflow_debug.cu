@@ -261,9 +261,13 @@ int pdflow_time_level_iterations(pdflow_solver* s, unsigned n, unsigned level, u
 
 namespace {
 
-// div_rcp against the IEEE division on random pairs of its range: a = +-2^[-60, 59]
-// x mantissa (one in 1024 a signed zero), b = 2^[-40, 59] x mantissa (one in 256
-// just above the shrinkage's 1e-10 floor); counts the pairs whose bits differ.
+// div_rcp against the IEEE division on random pairs of its range; counts the pairs
+// whose bits differ.  Half: a = +-2^[-60, 59] x mantissa (one in 1024 a signed zero),
+// b = 2^[-40, 59] x mantissa (one in 256 just above the shrinkage's 1e-10 floor).  A
+// quarter: a = +-2^[60, 89] x mantissa, b's exponent at most 30 below a's.  A
+// quarter as the shrinkage forms them next to its threshold: th = 2^[-30, 59] x
+// mantissa, b = th + 1e-10, a = a1 of with |a1| = 2^[-30, 29] x mantissa and |of| up to
+// 7 ulp below th.
 __device__ __forceinline__ unsigned mix64(unsigned long long x)
 {
     x ^= x >> 33;
@@ -284,10 +288,21 @@ __global__ void k_div_rcp_check(unsigned long long n, unsigned long long seed, u
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         const unsigned r1 = mix64(seed + 2 * i), r2 = mix64(seed + 2 * i + 1);
-        float a = rand_mag(r1, -60, 59);
-        if ((r2 & 1023u) == 0) a = (r2 & 1024u) ? -0.f : 0.f;
-        float b = rand_mag(r2 & 0x7fffffffu, -40, 59);
-        if ((r1 & 255u) == 3) b = __fadd_rn(__uint_as_float((mix64(r1) & 0x007fffffu) | 0x2e000000u), 1e-10f);
+        float a, b;
+        if (i % 4 == 0) {
+            a = rand_mag(r1, 60, 89);
+            b = rand_mag(r2 & 0x7fffffffu, int((__float_as_uint(a) >> 23) & 255u) - 127 - 30, 59);
+        } else if (i % 4 == 1) {
+            const float th = rand_mag(r2 & 0x7fffffffu, -30, 59);
+            const float of = __uint_as_float(max(__float_as_uint(th) - (mix64(r2) & 7u), 0x30800000u));   // not below 2^-30
+            a = __fmul_rn(rand_mag(r1, -30, 29), of);
+            b = __fadd_rn(th, 1e-10f);
+        } else {
+            a = rand_mag(r1, -60, 59);
+            if ((r2 & 1023u) == 0) a = (r2 & 1024u) ? -0.f : 0.f;
+            b = rand_mag(r2 & 0x7fffffffu, -40, 59);
+            if ((r1 & 255u) == 3) b = __fadd_rn(__uint_as_float((mix64(r1) & 0x007fffffu) | 0x2e000000u), 1e-10f);
+        }
         if (__float_as_uint(div_rcp(-a, b, -__frcp_rn(b))) != __float_as_uint(__fdiv_rn(a, b))) ++mine;
     }
     if (mine) atomicAdd(bad, mine);

@@ -344,7 +344,8 @@ __device__ __forceinline__ void primal_update(float& du, float& dv, float& dw, f
 // na and ny save the negations.  Valid for a == 0 or 2^-60 <= |a| < 2^60 and
 // 2^-40 <= b < 2^60, and up to |a| < 2^90 where |a / b| < 2^31 (no
 // intermediate leaves the normal range).  Checked bit for bit against
-// __fdiv_rn on 1.7e10 random pairs of that range.
+// __fdiv_rn on 1.7e10 random pairs of that range, a quarter of them with |a| above
+// 2^60 and a quarter with the quotient at the shrinkage's threshold.
 __device__ __forceinline__ float div_rcp(float na, float b, float ny)
 {
     const float q0 = mul(na, ny);
