@@ -261,7 +261,7 @@ struct GradLevels {
 __global__ void k_im_gradients(const __grid_constant__ GradLevels lv, LevelConsts L, size_t pstride,
                                const unsigned* __restrict__ map)
 {
-    allow_next_kernel();
+    allow_next_kernel();   // no wait before it: an ordinary launch, all before it has ended
     unsigned q = 0;
     while (q + 1 < lv.count && blockIdx.x >= lv.first_block[q + 1]) ++q;
     const size_t po = pair_off(map, pstride, blockIdx.y);
@@ -698,7 +698,9 @@ __global__ void __launch_bounds__(kMedRows * kMedCols) k_median(LevelGeom g, boo
     dz = at(dz, po);
     const int R = (int)g.R, C = (int)g.C;
     const int v0 = (int)blockIdx.x * kMedRows, u0 = (int)blockIdx.y * kMedCols;
-    allow_next_kernel();   // the next level's start, as these CTAs end
+    // the next level's start, as these CTAs end (no wait before it: this is an ordinary
+    // launch, all before it has ended)
+    allow_next_kernel();
     // the tile and its halo: rows v0-1 .. v0+kMedRows, columns u0-1 .. u0+kMedCols
     for (int e = threadIdx.y * kMedRows + threadIdx.x; e < kMedHR * kMedHC; e += kMedRows * kMedCols) {
         const int hr = e % kMedHR, hc = e / kMedHR, gv = v0 - 1 + hr, gu = u0 - 1 + hc;

@@ -149,13 +149,13 @@ cudaError_t launch_pyramid_rgb8_mm(const uint8_t* rgb, const uint16_t* depth, un
 // Column-major float planes I, Z in every pair's arena slice.
 cudaError_t launch_pyramid_planes(const float* I, const float* Z, unsigned W, unsigned H, const PyrLevel* levels,
                                   unsigned count, float fovh, unsigned pairs, size_t pstride, cudaStream_t st);
-// Copies the levels' planes of `src` over `dst` for the mapped slots (frame t
-// becomes t-1); the planes of both lie back to back in the same order, the last
-// level's have `smallest` floats.
 // Flow planes of n pairs (`step` bytes apart, `floats` each, a multiple of 4) and
 // the status word to device-addressable host memory: out[plane][pair][floats].
 cudaError_t launch_flow_out(const float* dx, const float* dy, const float* dz, size_t step, unsigned n, size_t floats,
                             const unsigned* status, float* out, unsigned* out_status, cudaStream_t st);
+// Copies the levels' planes of `src` over `dst` for the mapped slots (frame t
+// becomes t-1); the planes of both lie back to back in the same order, the last
+// level's have `smallest` floats.
 cudaError_t launch_pyr_copy(const PyrLevel* src, const PyrLevel* dst, unsigned levels, unsigned smallest, unsigned pairs,
                             size_t pstride, const unsigned* map, cudaStream_t st);
 // The new frame's weighted image gradients of `count` levels of the same pairs

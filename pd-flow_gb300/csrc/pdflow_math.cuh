@@ -28,7 +28,8 @@ namespace pdflow {
 // nothing that kernel reads or writes before after_previous_kernel(), which
 // returns when the kernel before it has ended and its writes are visible.  A CTA
 // allows the next kernel only after its own wait, so no kernel starts while the
-// last but one is running.  Both do nothing in a kernel launched without.
+// last but one is running; one without a wait may allow it at once only if it is
+// an ordinary launch.  Both do nothing in a kernel launched without.
 __device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

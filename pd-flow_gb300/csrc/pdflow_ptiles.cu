@@ -23,9 +23,10 @@
 // the region is updated in every iteration; the stale ring at non-border
 // region edges is never read by an exact pixel and only the interior is
 // stored.  Needs rows % 4 == 0 (16-byte aligned tensor-copy rows); levels
-// with an even row count otherwise (a VGA solve's 30x40) run the tiles with
-// each thread loading its pixel pair's 32 values directly (8-byte loads, no
-// staging: such levels have about one region per CTA, nothing to stream).
+// with an even row count otherwise (30x40, where form 8 was chosen: by default it
+// runs resident, pdflow_resident.cu) run the tiles with each thread loading its
+// pixel pair's 32 values directly (8-byte loads, no staging: such levels have
+// about one region per CTA, nothing to stream).
 //
 // Strips (iteration form 10).  Of an iteration's column neighbours only the
 // primal step's backward difference looks left (ri * the dual's u-component
@@ -51,7 +52,7 @@
 // mbarrier they arrive on), so the walk's index arithmetic, the unit counter's
 // latency and the copies' issue are off the arithmetic's path, and a region
 // has no block barrier but the iterations' two.  Bound: instruction issue and
-// latency (16 warps an SM, the registers' limit; 51.5 % issue active, 6.73 warp
+// latency (16 warps an SM, the registers' limit; 51.3 % issue active, 6.63 warp
 // instructions a pixel-iteration).  When
 // thread 0 of the consumers did the walk behind a block barrier a region, 64
 // VGA pairs took 35.74 ms and five 3.68 ms; with the producer 32.43 and 3.48.
