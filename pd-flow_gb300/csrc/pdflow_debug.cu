@@ -230,7 +230,7 @@ int pdflow_wait_count(const pdflow_solver* s, unsigned long long* count)
 int pdflow_pinned_bytes(const pdflow_solver* s, size_t* bytes)
 {
     if (!s || !bytes) return fail(PDFLOW_ERR_ARG, "null argument");
-    *bytes = s->host_pinned_bytes;
+    *bytes = s->host_result_block + s->host_frame_block;
     return PDFLOW_OK;
 }
 

@@ -44,7 +44,7 @@ struct pdflow_solver {
     // Pinned host memory the device addresses, taken on first use (null: transfers go
     // to and from the caller's memory directly): the status word, a result buffer, two
     // frame buffers.
-    size_t host_pinned_bytes = 0;
+    size_t host_result_block = 0, host_frame_block = 0;   // their blocks' bytes
     bool host_result_tried = false;
     unsigned* host_status = nullptr;
     uint8_t* host_frames[2] = {};

@@ -138,6 +138,71 @@ struct RelaxedCapture {
     RelaxedCapture& operator=(const RelaxedCapture&) = delete;
 };
 
+// Pinned blocks of destroyed handles, kept for the next ones (4 MB at most) while any
+// handle lives and given back with the last.  A program that replaces a handle frees
+// the old one's blocks before the new one's first use: pinning and unpinning took
+// 0.4 ms a replacement.  A block is given after the work on it has ended.
+class PinnedBlocks {
+public:
+    void enter()
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        ++handles_;
+    }
+    void leave()
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (--handles_ > 0) return;
+        for (; used_ > 0; --used_) cudaFreeHost(kept_[used_ - 1].p);
+        bytes_ = 0;
+    }
+    // At least *bytes, which becomes the block's size; null without the memory.
+    void* take(size_t* bytes)
+    {
+        *bytes = (*bytes + kUnit - 1) / kUnit * kUnit;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            for (int i = 0; i < used_; ++i)
+                if (kept_[i].bytes == *bytes) {
+                    void* p = kept_[i].p;
+                    kept_[i] = kept_[--used_];
+                    bytes_ -= *bytes;
+                    return p;
+                }
+        }
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, *bytes, cudaHostAllocDefault) == cudaSuccess) return p;
+        cudaGetLastError();
+        return nullptr;
+    }
+    void give(void* p, size_t bytes)
+    {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (used_ < kMost && bytes_ + bytes <= kMostBytes) {
+                kept_[used_++] = {p, bytes};
+                bytes_ += bytes;
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+
+private:
+    static constexpr size_t kUnit = 64u << 10, kMostBytes = 4u << 20;
+    static constexpr int kMost = 64;
+    struct Block {
+        void* p;
+        size_t bytes;
+    };
+    std::mutex mu_;
+    Block kept_[kMost];
+    int used_ = 0;
+    size_t bytes_ = 0;
+    unsigned handles_ = 0;
+};
+static PinnedBlocks g_pinned;
+
 // Pinned memory is taken by the first call that has a use for it (a caller with
 // frames and flows on the device has none): the status word and a result buffer by
 // the first that waits, the frame buffers by the first push that fits one.  Best
@@ -152,12 +217,10 @@ void create_result_buffer(pdflow_solver* s)
     // of a mixed batch, flows of up to 60x80 pass (of five pairs and more, up to 120x160)
     const size_t flow = (s->mixed ? size_t(60) * 80 : size_t(s->rows) * s->cols) * 12;
     const size_t cap = flow <= kHostFlowLimit ? std::min(flow * s->batch, kHostFlowLimit) : 0;
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, 256 + cap, cudaHostAllocDefault) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    s->host_pinned_bytes += 256 + cap;
+    size_t bytes = 256 + cap;
+    void* p = g_pinned.take(&bytes);
+    if (!p) return;
+    s->host_result_block = bytes;
     s->host_status = static_cast<unsigned*>(p);
     s->host_flow = reinterpret_cast<float*>(static_cast<uint8_t*>(p) + 256);
     s->host_flow_bytes = cap;
@@ -168,12 +231,10 @@ void create_frame_buffers(pdflow_solver* s)
     const size_t frame = size_t(s->width) * s->height * 3 + 256;   // uint8 intensity and uint16 depth
     if (s->host_frame_tried || frame > kHostFrameLimit) return;
     s->host_frame_tried = true;
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, 2 * kHostFrameLimit, cudaHostAllocDefault) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    s->host_pinned_bytes += 2 * kHostFrameLimit;
+    size_t bytes = 2 * kHostFrameLimit;
+    void* p = g_pinned.take(&bytes);
+    if (!p) return;
+    s->host_frame_block = bytes;
     s->host_frames[0] = static_cast<uint8_t*>(p);
     s->host_frames[1] = s->host_frames[0] + kHostFrameLimit;
     if (cudaEventCreateWithFlags(&s->host_frame_read[0], cudaEventDisableTiming) == cudaSuccess &&
@@ -187,8 +248,9 @@ void destroy_host_buffers(pdflow_solver* s)
 {
     for (cudaEvent_t e : s->host_frame_read)
         if (e) cudaEventDestroy(e);
-    if (s->host_frames[0]) cudaFreeHost(s->host_frames[0]);
-    if (s->host_status) cudaFreeHost(s->host_status);
+    if (s->host_frames[0]) g_pinned.give(s->host_frames[0], s->host_frame_block);
+    if (s->host_status) g_pinned.give(s->host_status, s->host_result_block);
+    g_pinned.leave();
 }
 
 // Ordinary host memory (neither pinned nor managed: work on the stream may still
@@ -802,6 +864,7 @@ int pdflow_create_batch(unsigned rows, unsigned width, unsigned height, const pd
         return set_error(PDFLOW_ERR_CUDA, "stream / arena init", e);
     }
     s->stream = s->own_stream;
+    g_pinned.enter();
     *out = s;
     return PDFLOW_OK;
 }

@@ -76,3 +76,49 @@ def test_a_mixed_handle_pins_at_its_first_read(built_lib):
     # its passing results are those of rows up to 120, not the whole arena's
     assert 60 * 80 * 12 <= _pinned(m) <= (256 << 10) + 4096
     m.close()
+
+
+def test_handles_replaced_in_several_threads(built_lib):
+    """Blocks of destroyed handles serve new ones: four threads that each replace
+    handles of different sizes, the old one destroyed before or after the new one's
+    first use, get every pair's own flow."""
+    import threading
+    kinds = [(60, 1), (15, 3), (60, 6), (30, 1)]
+    pairs = [scenes.make_pair(30 + k) for k in range(6)]
+
+    def solve(rows, n, shift, old=None):
+        b = BatchSolver(rows, 320, 240, n)
+        order = [pairs[(shift + k) % 6] for k in range(n)]
+        for f in (0, 1):
+            b.push_raw(np.stack([p[2 * f] for p in order]), np.stack([p[2 * f + 1] for p in order]))
+        if old is not None:
+            old.close()
+        b.solve(n)
+        return b, np.stack(b.read_flow(n)).view(np.uint32).copy()
+
+    want = {}
+    for rows, n in kinds:
+        for shift in range(3):
+            b, want[rows, n, shift] = solve(rows, n, shift)
+            b.close()
+    bad = []
+
+    def work(t):
+        old = None
+        for rep in range(12):
+            rows, n = kinds[(t + rep) % 4]
+            if old is not None and rep % 2:
+                old.close()
+                old = None
+            old, got = solve(rows, n, rep % 3, old)
+            if not np.array_equal(got, want[rows, n, rep % 3]):
+                bad.append((t, rep))
+        old.close()
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    assert all(w.any() for w in want.values())
