@@ -307,9 +307,10 @@ int read_planes(pdflow_solver* s, const FlowRun* runs, unsigned count, size_t fl
     const float* const src[3] = {s->dx, s->dy, s->dz};
     const size_t b = floats * 4, step = s->pair_stride;
     create_result_buffer(s);
-    bool pass = true, copied = false;
-    for (float* d : dst) pass = pass && (!d || pageable(d));
-    const size_t most = pass ? std::min<size_t>(s->host_flow_bytes / (3 * b), 65535) : 0;   // pairs that pass at once
+    size_t most = std::min<size_t>(s->host_flow_bytes / (3 * b), 65535);   // pairs that pass at once
+    for (float* d : dst)
+        if (most > 0 && d && !pageable(d)) most = 0;
+    bool copied = false;
     int rc = PDFLOW_OK;
     size_t k = 0;   // pairs before run r
     for (unsigned r = 0; r < count;) {
